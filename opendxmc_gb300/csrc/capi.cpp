@@ -124,9 +124,9 @@ struct dxmcg_world {
     DeviceBuffer<uint8_t> mat;
     DeviceBuffer<uint32_t> vox;
     DeviceBuffer<Tally> tally;
-    DeviceBuffer<float> tot;
+    DeviceBuffer<float2> tot;
     DeviceBuffer<float4> xs;
-    DeviceBuffer<float> maj;
+    DeviceBuffer<float2> maj;
     DeviceBuffer<DevMaterial> mats;
     DeviceBuffer<float> ctab; // Compton angle quantiles per material and energy
     DeviceBuffer<float> rtab; // Rayleigh angle quantiles per material and energy
@@ -145,7 +145,7 @@ struct dxmcg_world {
     // two-region Woodcock: box of the voxels whose material is neither 0 nor
     // transparent (lo x, y, z, hi x, y, z), and material 0's majorant
     DeviceBuffer<int> boxBuf;
-    DeviceBuffer<float> majOut;
+    DeviceBuffer<float2> majOut;
     // dose readback staging when the caller's arrays are not pinned host memory
     DeviceBuffer<double> readDose, readVar;
     DeviceBuffer<unsigned long long> readCount;
@@ -883,9 +883,11 @@ DXMCG_API int dxmcg_world_build(dxmcg_world* w)
     DXMCG_CUDA(w->mats.alloc(M));
     DXMCG_CUDA(w->counters.alloc(1));
     DXMCG_CUDA(w->tally.alloc(w->N));
-    DXMCG_CUDA(cudaMemcpyAsync(w->tot.p, tot.data(), tot.size() * sizeof(float), cudaMemcpyHostToDevice, w->stream));
+    const std::vector<float2> totPairs = tablePairs(tot), majPairs = tablePairs(majf);
+    DXMCG_CUDA(cudaMemcpyAsync(w->tot.p, totPairs.data(), totPairs.size() * sizeof(float2), cudaMemcpyHostToDevice,
+        w->stream));
     DXMCG_CUDA(cudaMemcpyAsync(w->xs.p, xs.data(), xs.size() * sizeof(float4), cudaMemcpyHostToDevice, w->stream));
-    DXMCG_CUDA(cudaMemcpyAsync(w->maj.p, majf.data(), kNE * sizeof(float), cudaMemcpyHostToDevice, w->stream));
+    DXMCG_CUDA(cudaMemcpyAsync(w->maj.p, majPairs.data(), kNE * sizeof(float2), cudaMemcpyHostToDevice, w->stream));
     DXMCG_CUDA(cudaMemcpyAsync(w->mats.p, dm.data(), M * sizeof(DevMaterial), cudaMemcpyHostToDevice, w->stream));
     std::vector<float> ctab(static_cast<size_t>(M) * kNE * kCTabK);
     buildComptonAngleTables(w->materials.data(), M, w->correction, ctab.data());
@@ -922,9 +924,11 @@ DXMCG_API int dxmcg_world_build(dxmcg_world* w)
         std::vector<float> mo(kNE);
         buildBackgroundMajorant(tot.data(), w->rhoMax[0], mo.data());
         DXMCG_CUDA(w->majOut.alloc(kNE));
-        DXMCG_CUDA(cudaMemcpyAsync(w->majOut.p, mo.data(), kNE * sizeof(float), cudaMemcpyHostToDevice, w->stream));
+        const std::vector<float2> moPairs = tablePairs(mo);
+        DXMCG_CUDA(cudaMemcpyAsync(w->majOut.p, moPairs.data(), kNE * sizeof(float2), cudaMemcpyHostToDevice,
+            w->stream));
+        DXMCG_CUDA(cudaStreamSynchronize(w->stream)); // the staging above must outlive the copies
     }
-    DXMCG_CUDA(cudaStreamSynchronize(w->stream));
     w->hasBox = twoRegionBox(w->box, w->dims);
     w->historiesScored = 0.0;
     w->built = true;
@@ -1043,7 +1047,7 @@ DXMCG_API int dxmcg_world_tables(dxmcg_world* w, int material, float* xs4, float
         DXMCG_CUDA(cudaMemcpy(xs4, w->xs.p + static_cast<size_t>(material) * kNE, kNE * sizeof(float4),
             cudaMemcpyDeviceToHost));
     if (majorant)
-        DXMCG_CUDA(cudaMemcpy(majorant, w->maj.p, kNE * sizeof(float), cudaMemcpyDeviceToHost));
+        std::copy(w->hostMaj.begin(), w->hostMaj.end(), majorant);
     return DXMCG_OK;
 }
 

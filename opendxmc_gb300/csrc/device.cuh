@@ -85,11 +85,11 @@ namespace dev {
         f = x - static_cast<float>(k);
     }
 
-    __device__ __forceinline__ float lerp1(const float* t, int i, float f)
+    // t[i] holds the table's values at i and i + 1: one 8-byte load
+    __device__ __forceinline__ float lerp1(const float2* t, int i, float f)
     {
-        const float a = __ldg(t + i);
-        const float b = __ldg(t + i + 1);
-        return fmaf(f, b - a, a);
+        const float2 ab = __ldg(t + i);
+        return fmaf(f, ab.y - ab.x, ab.x);
     }
 
     // ---------------------------------------------------------------- samplers
@@ -172,6 +172,13 @@ namespace dev {
         return fmaf(fe, hi - lo, lo);
     }
 
+    // E / E_C of the Compton line at 1 - cos theta = omu, product and sum rounded
+    // separately: histories must not depend on where the compiler fuses them
+    __device__ __forceinline__ float comptonRatio(float E, float omu)
+    {
+        return __fadd_rn(1.0f, __fmul_rn(E * (1.0f / kMeKeV), omu));
+    }
+
     // Compton scattering: the angle from the Klein-Nishina x S table, E' from the
     // Compton relation (correction 0 and 1), or Doppler-broadened by a bound electron's
     // momentum (correction 2, which may send the draw back for a new angle).
@@ -179,18 +186,17 @@ namespace dev {
     __device__ float sampleCompton(float E, const DevMaterial* __restrict__ M, const float* __restrict__ ctab,
         int ie, float fe, int correction, U& r, float& cost, unsigned& err)
     {
-        const float k = E * (1.0f / kMeKeV);
         for (int guard = 0; guard < kMaxRejections; ++guard) {
             const float omu = oneMinusCos(ctab, ie, fe, r.u());
-            const float xm1 = k * omu;
+            const float ratio = comptonRatio(E, omu);
             cost = 1.0f - omu;
             if (correction >= 2) {
                 float Ep;
-                if (!dopplerEnergy(E, 1.0f + xm1, omu, M, r, Ep))
+                if (!dopplerEnergy(E, ratio, omu, M, r, Ep))
                     continue;
                 return Ep;
             }
-            return E * __frcp_rn(1.0f + xm1);
+            return E * __frcp_rn(ratio);
         }
         err |= kErrRejectLimit;
         cost = 1.0f;

@@ -6,9 +6,9 @@
 //                      material index (one 4-byte gather per voxel visit;
 //                      density keeps 16 significant bits, |rel. rounding| <= 2^-16)
 //   tally  Tally[N]    {energy, energy^2, events} in one 32-byte sector
-//   tot    float[M][NE]        total mass attenuation per material (cm^2/g)
+//   tot    float2[M][NE]       total mass attenuation per material (cm^2/g) at i, i + 1
 //   xs     float4[M][NE]       (photo, incoherent, coherent, total)
-//   maj    float[NE]           majorant mu_max(E) over the grid (1/cm)
+//   maj    float2[NE]          majorant mu_max(E) over the grid (1/cm) at i, i + 1
 //   mats   DevMaterial[M]      per-element sampling data
 #pragma once
 
@@ -106,9 +106,9 @@ struct DevJob {
     float isp[3];
     float L[3];
     float Lin[3]; // largest float strictly below L
-    const float* tot;
+    const float2* tot;
     const float4* xs;
-    const float* maj;
+    const float2* maj;
     const DevMaterial* mats;
     const float* rtab; // [n_mats][kTableNE][kCTabK] Rayleigh 1 - cos theta quantiles
     const float* ctab; // [n_mats][kTableNE][kCTabK] Compton 1 - cos theta quantiles
@@ -146,7 +146,7 @@ struct DevJob {
     int b0[3];
     unsigned bn[3];
     float blo[3], bhi[3];
-    const float* majOut;
+    const float2* majOut;
 };
 
 constexpr int kCellShift = 3; // gather-skip cells of 8 x 8 x 8 voxels

@@ -293,6 +293,14 @@ void buildBackgroundMajorant(const float* tot0, double rho0, float* out)
         out[i] = static_cast<float>(std::max(static_cast<double>(tot0[i]) * rho0 * kMajorantSafety, 1e-30));
 }
 
+std::vector<float2> tablePairs(const std::vector<float>& t)
+{
+    std::vector<float2> p(t.size());
+    for (size_t i = 0; i < t.size(); ++i)
+        p[i] = { t[i], t[(i + 1) % kNE == 0 ? i : i + 1] };
+    return p;
+}
+
 bool twoRegionBox(const int box[6], const int32_t dims[3])
 {
     return box[3] >= 0
@@ -317,7 +325,7 @@ bool twoRegionFor(const dxmcg_run_options& o, double boxFrac)
     return o.two_region > 0 || boxFrac < 0.5;
 }
 
-void setTwoRegion(DevJob& J, const int box[6], const double spacing[3], const float* majOut)
+void setTwoRegion(DevJob& J, const int box[6], const double spacing[3], const float2* majOut)
 {
     J.boxOn = 1;
     J.majOut = majOut;

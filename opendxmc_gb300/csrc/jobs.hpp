@@ -37,6 +37,8 @@ void materialTables(const dxmcg_material& m, int correction, double* photo, doub
 // majorant of material 0 alone: rho0 x its total attenuation, with the same safety
 // factor and floor as the grid's majorant
 void buildBackgroundMajorant(const float* tot0, double rho0, float* out);
+// tables of kNE values as (value i, value i + 1) pairs, as the kernels read them
+std::vector<float2> tablePairs(const std::vector<float>& t);
 // Compton and Rayleigh angle quantiles out[m][i][j] (kCTabK per row; see kCTabK),
 // kept per (composition, correction) for the life of the physics tables
 void buildComptonAngleTables(const dxmcg_material* mats, int M, int correction, float* out);
@@ -52,7 +54,7 @@ double boxFraction(const int box[6], const int32_t dims[3]);
 // torso, +13 %) and 0.36 (512x512x400 torso, +23 %); off at 0.53-0.62 (the batch
 // workload's ellipsoids, -12 %) and 0.94 (the DX cylinder, -11 %).
 bool twoRegionFor(const dxmcg_run_options& o, double boxFrac);
-void setTwoRegion(DevJob& J, const int box[6], const double spacing[3], const float* majOut);
+void setTwoRegion(DevJob& J, const int box[6], const double spacing[3], const float2* majOut);
 void buildDeviceTables(const dxmcg_material* mats, int M, int correction, const double* rhoMax, float* tot,
     float4* xs, float* maj, DevMaterial* dm);
 

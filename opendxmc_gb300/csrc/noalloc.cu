@@ -57,14 +57,14 @@ namespace {
     constexpr size_t kOffBowtie = alignUp(kOffSpec + 2 * sizeof(DevSpectrum));
     constexpr size_t kOffMats = alignUp(kOffBowtie + sizeof(DevBowtie));
     constexpr size_t kOffMaj = alignUp(kOffMats + kMaxMaterials * sizeof(DevMaterial));
-    constexpr size_t kOffTot = alignUp(kOffMaj + kTableNE * sizeof(float));
-    constexpr size_t kOffXs = alignUp(kOffTot + kMaxMaterials * kTableNE * sizeof(float));
+    constexpr size_t kOffTot = alignUp(kOffMaj + kTableNE * sizeof(float2));
+    constexpr size_t kOffXs = alignUp(kOffTot + kMaxMaterials * kTableNE * sizeof(float2));
     constexpr size_t kOffExps = alignUp(kOffXs + kMaxMaterials * kTableNE * sizeof(float4));
     constexpr size_t kOffCTab = alignUp(kOffExps + kMaxExposures * sizeof(DevExposure));
     constexpr size_t kOffRTab = alignUp(kOffCTab + kMaxMaterials * kTableNE * kCTabK * sizeof(float));
     constexpr size_t kOffBox = alignUp(kOffRTab + kMaxMaterials * kTableNE * kCTabK * sizeof(float)); // 6 ints
     constexpr size_t kOffMajOut = alignUp(kOffBox + 6 * sizeof(int));
-    constexpr size_t kUsed = kOffMajOut + kTableNE * sizeof(float);
+    constexpr size_t kUsed = kOffMajOut + kTableNE * sizeof(float2);
     static_assert(kUsed <= kScratchBytes, "scratch layout exceeds the static array");
     static_assert(sizeof(dxmcg_tally_record) == sizeof(Tally), "tally record layout");
 
@@ -240,7 +240,9 @@ extern "C" DXMCG_API int dxmcg_transport_run_noalloc(const int32_t dims[3], cons
     std::vector<float> maj(kTableNE);
     std::vector<DevMaterial> dm(n_materials);
     buildDeviceTables(materials, n_materials, correction, rhoMax, tot.data(), xs.data(), maj.data(), dm.data());
-    NOALLOC_CUDA(cudaMemcpyAsync(base + kOffTot, tot.data(), tot.size() * sizeof(float), cudaMemcpyHostToDevice, s));
+    const std::vector<float2> totPairs = tablePairs(tot), majPairs = tablePairs(maj);
+    NOALLOC_CUDA(cudaMemcpyAsync(base + kOffTot, totPairs.data(), totPairs.size() * sizeof(float2),
+        cudaMemcpyHostToDevice, s));
     NOALLOC_CUDA(cudaMemcpyAsync(base + kOffXs, xs.data(), xs.size() * sizeof(float4), cudaMemcpyHostToDevice, s));
     std::vector<float> ctab(static_cast<size_t>(n_materials) * kTableNE * kCTabK);
     buildComptonAngleTables(materials, n_materials, correction, ctab.data());
@@ -248,12 +250,14 @@ extern "C" DXMCG_API int dxmcg_transport_run_noalloc(const int32_t dims[3], cons
     std::vector<float> rtab(static_cast<size_t>(n_materials) * kTableNE * kCTabK);
     buildRayleighAngleTables(materials, n_materials, rtab.data());
     NOALLOC_CUDA(cudaMemcpyAsync(base + kOffRTab, rtab.data(), rtab.size() * sizeof(float), cudaMemcpyHostToDevice, s));
-    NOALLOC_CUDA(cudaMemcpyAsync(base + kOffMaj, maj.data(), maj.size() * sizeof(float), cudaMemcpyHostToDevice, s));
+    NOALLOC_CUDA(cudaMemcpyAsync(base + kOffMaj, majPairs.data(), majPairs.size() * sizeof(float2), cudaMemcpyHostToDevice, s));
     const bool twoRegion = woodcock && twoRegionBox(hostBox, dims) && twoRegionFor(o, boxFraction(hostBox, dims));
     std::vector<float> majOut(kTableNE);
+    std::vector<float2> majOutPairs;
     if (twoRegion) {
         buildBackgroundMajorant(tot.data(), rhoMax[0], majOut.data());
-        NOALLOC_CUDA(cudaMemcpyAsync(base + kOffMajOut, majOut.data(), majOut.size() * sizeof(float),
+        majOutPairs = tablePairs(majOut);
+        NOALLOC_CUDA(cudaMemcpyAsync(base + kOffMajOut, majOutPairs.data(), majOutPairs.size() * sizeof(float2),
             cudaMemcpyHostToDevice, s));
     }
     NOALLOC_CUDA(cudaMemcpyAsync(base + kOffMats, dm.data(), dm.size() * sizeof(DevMaterial), cudaMemcpyHostToDevice, s));
@@ -275,18 +279,18 @@ extern "C" DXMCG_API int dxmcg_transport_run_noalloc(const int32_t dims[3], cons
     J.vox = nullptr;
     J.dens = device_density;
     J.mat = device_material;
-    J.tot = reinterpret_cast<const float*>(base + kOffTot);
+    J.tot = reinterpret_cast<const float2*>(base + kOffTot);
     J.xs = reinterpret_cast<const float4*>(base + kOffXs);
     J.ctab = reinterpret_cast<const float*>(base + kOffCTab);
     J.rtab = reinterpret_cast<const float*>(base + kOffRTab);
-    J.maj = reinterpret_cast<const float*>(base + kOffMaj);
+    J.maj = reinterpret_cast<const float2*>(base + kOffMaj);
     J.mats = reinterpret_cast<const DevMaterial*>(base + kOffMats);
     J.tally = reinterpret_cast<Tally*>(device_tally);
     J.exps = reinterpret_cast<const DevExposure*>(base + kOffExps);
     J.spec = reinterpret_cast<const DevSpectrum*>(base + kOffSpec);
     J.bowtie = hj.hasBowtie ? reinterpret_cast<const DevBowtie*>(base + kOffBowtie) : nullptr;
     if (twoRegion)
-        setTwoRegion(J, hostBox, spacing_cm, reinterpret_cast<const float*>(base + kOffMajOut));
+        setTwoRegion(J, hostBox, spacing_cm, reinterpret_cast<const float2*>(base + kOffMajOut));
 
     LaunchShape shape;
     shape.block = o.block_size > 0 ? std::max(32, std::min(256, o.block_size / 32 * 32)) : 256;

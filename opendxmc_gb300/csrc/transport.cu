@@ -1,4 +1,5 @@
-// transport.cu -- the persistent photon-transport kernel (sm_103a).
+// transport.cu -- exact Siddon flights and macro-cell delta tracking (sm_103a), and the
+// launchers of every transport kernel (the default Woodcock tracking: woodcock.cu).
 //
 // Every lane owns one photon and is in one of five states: stepping, waiting for
 // a Compton interaction, waiting for a Rayleigh interaction, waiting for the
@@ -10,18 +11,13 @@
 //             pool of history indices that the warp takes from a global work-queue
 //             head in chunks of kChunk (one atomic per chunk);
 //   interact  lanes waiting for an interaction run it together once at least
-//             `interactBatch` lanes wait (Compton: the angle from the material's
-//             Klein-Nishina x S(x)/Z quantile table, and at level 2 the Doppler
-//             energy of a bound electron; Rayleigh: element choice from the
-//             material's share table and analytic inversion of F^2, rejection on
-//             (1 + cos^2)/2; fluorescence: K-shell vacancy and yield);
-//   step      stepping lanes take up to `woodcockSteps` Woodcock steps against the
-//             majorant mu_max(E), stopping at a real collision or an escape (or, in
-//             the regular-tracking variant, one free flight with exact Siddon path
-//             lengths; with macro cells, one flight against the cell majorants); a
-//             real collision picks its type at once: photoelectric absorption is
-//             scored on the spot below level 2, the other events park the lane
-//             until the next interact phase.
+//             `interactBatch` lanes wait (Compton and Rayleigh: the angle from the
+//             material's quantile tables, at level 2 the Doppler energy of a bound
+//             electron; fluorescence: K-shell vacancy and yield);
+//   step      stepping lanes take one free flight with exact Siddon path lengths, or one
+//             flight against the macro cells' majorants; a real collision picks its type
+//             at once: photoelectric absorption is scored on the spot below level 2, the
+//             other events park the lane until the next interact phase.
 //
 // Parking interactions and batching refills regroups the expensive, divergent
 // work so that it runs with many lanes active instead of one or two.  A history
@@ -32,43 +28,12 @@
 #include <cmath>
 #include <cstdint>
 
-#include "device.cuh"
+#include "transport_common.cuh"
 
 namespace dxmcg {
 namespace {
-    using namespace dev;
-
-    constexpr int kChunk = 256; // histories a warp takes from the queue at once
-
     // kPhoto: a photoelectric absorption waiting for its fluorescence (correction level 2)
     enum LaneState : int { kDead = 0, kStepping = 1, kCompton = 2, kRayleigh = 3, kPhoto = 4 };
-    enum BlockCount : int {
-        cHist,
-        cMissed,
-        cPhoto,
-        cCompton,
-        cRayleigh,
-        cCutoff,
-        cErrors,
-        cInteracted,
-        cFluorescence,
-        cNum
-    };
-
-    __device__ __forceinline__ unsigned long long warpSum(unsigned long long v)
-    {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            v += __shfl_xor_sync(kFull, v, o);
-        return v;
-    }
-    __device__ __forceinline__ double warpSum(double v)
-    {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            v += __shfl_xor_sync(kFull, v, o);
-        return v;
-    }
 
     // Kahan-compensated FP32 sum; value() returns it in FP64 once, at the end.
     struct KahanSum {
@@ -82,268 +47,6 @@ namespace {
         }
         __device__ __forceinline__ double value() const { return static_cast<double>(s) - static_cast<double>(c); }
     };
-
-    // Per-thread sums of the source, escaped and deposited energy (K = 0, 1, 2), and
-    // the warp's pool of history indices [next, end) with its exhausted flag, in
-    // registers (LaneTotals<false>) or in shared memory (LaneTotals<true>; sums: value
-    // sEnergy[2K][thread], compensation [2K + 1]).  They change a few times per history
-    // or once per refill phase, so shared memory costs little where registers are short.
-    constexpr int kSumSource = 0, kSumEscaped = 1, kSumDeposited = 2;
-    __shared__ float sEnergy[6][256];
-    __shared__ unsigned long long sPool[256 / 32][2];
-    __shared__ int sExhausted[256 / 32];
-
-    template <bool SHARED>
-    struct LaneTotals;
-
-    template <>
-    struct LaneTotals<false> {
-        KahanSum sum[3];
-        unsigned long long next = 0, end = 0;
-        bool done = false;
-        __device__ __forceinline__ void init() { }
-        template <int K>
-        __device__ __forceinline__ void add(float x)
-        {
-            sum[K].add(x);
-        }
-        template <int K>
-        __device__ __forceinline__ double value() const
-        {
-            return sum[K].value();
-        }
-        __device__ __forceinline__ bool exhausted() const { return done; }
-        __device__ __forceinline__ void markExhausted() { done = true; }
-        __device__ __forceinline__ void loadPool(unsigned long long& n, unsigned long long& e) const
-        {
-            n = next;
-            e = end;
-        }
-        __device__ __forceinline__ void storePool(unsigned long long n, unsigned long long e)
-        {
-            next = n;
-            end = e;
-        }
-    };
-
-    template <>
-    struct LaneTotals<true> {
-        __device__ __forceinline__ void init()
-        {
-#pragma unroll
-            for (int k = 0; k < 6; ++k)
-                sEnergy[k][threadIdx.x] = 0.0f;
-            if ((threadIdx.x & 31u) == 0) {
-                sPool[threadIdx.x >> 5][0] = sPool[threadIdx.x >> 5][1] = 0ull;
-                sExhausted[threadIdx.x >> 5] = 0;
-            }
-            __syncwarp();
-        }
-        template <int K>
-        __device__ __forceinline__ void add(float x)
-        {
-            const float c = sEnergy[2 * K + 1][threadIdx.x], s0 = sEnergy[2 * K][threadIdx.x];
-            const float y = x - c;
-            const float t = s0 + y;
-            sEnergy[2 * K + 1][threadIdx.x] = (t - s0) - y;
-            sEnergy[2 * K][threadIdx.x] = t;
-        }
-        template <int K>
-        __device__ __forceinline__ double value() const
-        {
-            return static_cast<double>(sEnergy[2 * K][threadIdx.x])
-                - static_cast<double>(sEnergy[2 * K + 1][threadIdx.x]);
-        }
-        __device__ __forceinline__ bool exhausted() const { return sExhausted[threadIdx.x >> 5] != 0; }
-        // warp-uniform: every lane calls it; one writes, the barrier publishes
-        __device__ __forceinline__ void markExhausted()
-        {
-            __syncwarp();
-            if ((threadIdx.x & 31u) == 0)
-                sExhausted[threadIdx.x >> 5] = 1;
-            __syncwarp();
-        }
-        __device__ __forceinline__ void loadPool(unsigned long long& n, unsigned long long& e) const
-        {
-            n = sPool[threadIdx.x >> 5][0];
-            e = sPool[threadIdx.x >> 5][1];
-        }
-        __device__ __forceinline__ void storePool(unsigned long long n, unsigned long long e)
-        {
-            __syncwarp();
-            if ((threadIdx.x & 31u) == 0) {
-                sPool[threadIdx.x >> 5][0] = n;
-                sPool[threadIdx.x >> 5][1] = e;
-            }
-            __syncwarp();
-        }
-    };
-
-    // The photon's energy-grid position and the majorant its next flight steps
-    // against.  A negative invMmax marks a flight outside the two-region box, against
-    // majOut(E) = mmax = -1 / invMmax (no extra loop-carried register).
-    struct EnergyCache {
-        int ie;
-        float fe, mmax, invMmax;
-        __device__ __forceinline__ void set(const DevJob& J, float E)
-        {
-            gridPos(E, ie, fe);
-            toInner(J);
-        }
-        __device__ __forceinline__ void toInner(const DevJob& J)
-        {
-            mmax = lerp1(J.maj, ie, fe);
-            invMmax = 1.0f / mmax;
-        }
-        __device__ __forceinline__ void toOuter(const DevJob& J)
-        {
-            mmax = lerp1(J.majOut, ie, fe);
-            invMmax = -1.0f / mmax;
-        }
-    };
-
-    // Per-thread count of tentative collisions outside the two-region box (they read
-    // their voxel without the cell bound); about one per history, so kept in shared
-    // memory rather than in a register across the transport loop.
-    __shared__ unsigned sOuterVisits[256];
-
-    // Voxel (ix, iy, iz) lies outside the two-region box.
-    __device__ __forceinline__ bool outsideBox(const DevJob& J, int ix, int iy, int iz)
-    {
-        return (static_cast<unsigned>(ix - J.b0[0]) >= J.bn[0]) | (static_cast<unsigned>(iy - J.b0[1]) >= J.bn[1])
-            | (static_cast<unsigned>(iz - J.b0[2]) >= J.bn[2]);
-    }
-
-    // Distance along the flight to the widened box (FLT_MAX if the line misses it, 0
-    // from inside it).  Approximate reciprocals: the margin of the box absorbs their
-    // error, so the entry is never found late.
-    __device__ __forceinline__ float boxEntry(const DevJob& J, const Photon& ph)
-    {
-        const float p[3] = { ph.px, ph.py, ph.pz };
-        const float d[3] = { ph.dx, ph.dy, ph.dz };
-        float tn = 0.0f, tf = FLT_MAX;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const float inv = __fdividef(1.0f, d[a]);
-            const float t1 = (J.blo[a] - p[a]) * inv, t2 = (J.bhi[a] - p[a]) * inv;
-            tn = fmaxf(tn, fminf(t1, t2));
-            tf = fminf(tf, fmaxf(t1, t2));
-        }
-        return tn <= tf ? tn : FLT_MAX;
-    }
-
-    // Density and material of voxel v: one 4-byte word in the packed layout, or two
-    // loads from caller-owned arrays in the unpacked layout.
-    template <bool PACKED>
-    __device__ __forceinline__ float voxelAt(const DevJob& J, uint32_t v, int& m)
-    {
-        if (PACKED) {
-            const uint32_t word = __ldg(J.vox + v);
-            m = static_cast<int>(word & 0xffu);
-            return __uint_as_float(word & 0xffffff00u);
-        }
-        m = static_cast<int>(__ldg(J.mat + v));
-        return __ldg(J.dens + v);
-    }
-
-    // Woodcock step; returns true on a real collision in voxel v / material m.
-    //
-    // Gather skip (J.cbound set): the tentative collision is real when u mu_max(E) <
-    // rho mu_m(E).  The cell's bound b_c satisfies rho mu_m(E) <= b_c mu_max(E) for each
-    // of its voxels, with a margin larger than the FP32 roundings of both sides, so
-    // u mu_max >= b_c mu_max settles the step as virtual without reading the voxel.
-    // Otherwise the voxel is read and the usual test decides, on the same uniform: the
-    // decisions, and so the histories, are those of the plain step.  Cells holding a
-    // transparent voxel (b_c = +inf) take the plain step, which draws the uniform only
-    // for a voxel that is not transparent.
-    //
-    // BOX (the two-region instance, for jobs with J.boxOn): a flight outside the box
-    // steps against majOut; if the box comes first, the photon moves to it and steps
-    // on against maj (the flight is memoryless), drawing no acceptance uniform.  A
-    // flight against maj that ends outside the box decides its tentative collision as
-    // usual (maj bounds every voxel); the flights after it step against majOut.  Every
-    // decision keeps the tentative-collision rate at or above rho mu(E) on the path, so
-    // the transport is that of plain Woodcock with fewer tentative collisions.  Outside
-    // the box the cell bounds (relative to maj) are not used.
-    template <bool PACKED, bool BOX>
-    __device__ __forceinline__ bool woodcockStep(const DevJob& J, Photon& ph, Rng& rng, EnergyCache& ec,
-        bool& escaped, uint32_t& v, int& m, unsigned& visits, unsigned& skipped)
-    {
-        const bool outer = BOX && ec.invMmax < 0.0f;
-        // hardware log2: |error| <= 2^-21.4 near u = 1, where the step is < 1e-6 mean free paths
-        const float s = fmaxf(-__logf(rng.u()), 0.0f) * (BOX ? fabsf(ec.invMmax) : ec.invMmax);
-        if (BOX && outer) {
-            const float te = boxEntry(J, ph);
-            if (te < s) {
-                ph.px = fmaf(te, ph.dx, ph.px);
-                ph.py = fmaf(te, ph.dy, ph.py);
-                ph.pz = fmaf(te, ph.dz, ph.pz);
-                ec.toInner(J);
-                return false;
-            }
-        }
-        ph.px = fmaf(s, ph.dx, ph.px);
-        ph.py = fmaf(s, ph.dy, ph.py);
-        ph.pz = fmaf(s, ph.dz, ph.pz);
-        // voxel indices by rounding down; outside the grid one of them is negative
-        // (huge as unsigned) or >= its dimension (conversions saturate far away)
-        const int ix = __float2int_rd(ph.px * J.isp[0]);
-        const int iy = __float2int_rd(ph.py * J.isp[1]);
-        const int iz = __float2int_rd(ph.pz * J.isp[2]);
-        if ((static_cast<unsigned>(ix) >= static_cast<unsigned>(J.nx))
-            | (static_cast<unsigned>(iy) >= static_cast<unsigned>(J.ny))
-            | (static_cast<unsigned>(iz) >= static_cast<unsigned>(J.nz))) {
-            escaped = true;
-            return false;
-        }
-        ++visits;
-        v = static_cast<uint32_t>(ix + J.nx * (iy + J.ny * iz));
-        if (!BOX) {
-            if (J.cbound) {
-                const float b = __ldg(J.cbound
-                    + ((ix >> kCellShift) + J.cb[0] * ((iy >> kCellShift) + J.cb[1] * (iz >> kCellShift))));
-                if (b <= FLT_MAX) {
-                    const float t = rng.u() * ec.mmax;
-                    if (t >= b * ec.mmax) {
-                        ++skipped;
-                        return false;
-                    }
-                    const float rho = voxelAt<PACKED>(J, v, m);
-                    return t < rho * lerp1(J.tot + m * kTableNE, ec.ie, ec.fe);
-                }
-            }
-            const float rho = voxelAt<PACKED>(J, v, m);
-            if (m == DXMCG_TRANSPARENT_MATERIAL)
-                return false;
-            const float mu = rho * lerp1(J.tot + m * kTableNE, ec.ie, ec.fe);
-            return rng.u() * ec.mmax < mu;
-        }
-        if (outer)
-            ++sOuterVisits[threadIdx.x];
-        bool real = false, decided = false;
-        if (J.cbound && !outer) {
-            const float b = __ldg(J.cbound
-                + ((ix >> kCellShift) + J.cb[0] * ((iy >> kCellShift) + J.cb[1] * (iz >> kCellShift))));
-            if (b <= FLT_MAX) {
-                decided = true;
-                const float t = rng.u() * ec.mmax;
-                if (t >= b * ec.mmax) {
-                    ++skipped;
-                } else {
-                    const float rho = voxelAt<PACKED>(J, v, m);
-                    real = t < rho * lerp1(J.tot + m * kTableNE, ec.ie, ec.fe);
-                }
-            }
-        }
-        if (!decided) {
-            const float rho = voxelAt<PACKED>(J, v, m);
-            if (m != DXMCG_TRANSPARENT_MATERIAL)
-                real = rng.u() * ec.mmax < rho * lerp1(J.tot + m * kTableNE, ec.ie, ec.fe);
-        }
-        if (J.boxOn && !outer && outsideBox(J, ix, iy, iz))
-            ec.toOuter(J);
-        return real;
-    }
 
     // One free flight with exact voxel path lengths; true on a collision.
     template <bool PACKED>
@@ -482,10 +185,8 @@ namespace {
     template <int TRACKING, bool PACKED, bool MULTI>
     __global__ void __launch_bounds__(256) transportKernel(const DevJob J0, const DevJob* __restrict__ jobs,
         const unsigned long long* __restrict__ offsets, int nJobs, unsigned long long h_end,
-        DevCounters* __restrict__ ctr, int refillBatch, int interactBatch, int woodcockSteps)
+        DevCounters* __restrict__ ctr, int refillBatch, int interactBatch, int)
     {
-        constexpr bool BOX = TRACKING == kTrackWoodcockBox;
-        constexpr bool WOODCOCK = TRACKING == DXMCG_TRACK_WOODCOCK || BOX;
         int jid = 0;
         // event counters per warp (no block-wide barrier: warps finish independently)
         __shared__ unsigned long long sCountAll[256 / 32][cNum];
@@ -496,23 +197,18 @@ namespace {
         __syncwarp();
 
         const unsigned ltMask = (1u << lane) - 1u;
-        // energy sums (FP32, compensated) and the warp's history pool: in shared memory
-        // for the two-region instance, whose step would spill otherwise; in registers
-        // for the others, where shared memory measured slower (4 % on the 256x256x200
-        // torso, 5 % on the 64-job batch, whose instance spills a little instead)
-        LaneTotals<BOX> ls;
-        ls.init();
+        KahanSum sum[3];                      // kSumSource, kSumEscaped, kSumDeposited
+        unsigned long long poolNext = 0, poolEnd = 0; // the warp's pool of history indices
+        bool exhausted = false;
         int st = kDead;
         Photon ph;
         Rng rng;
         EnergyCache ec { 0, 0.0f, 1.0f, 1.0f };
         uint32_t pv = 0; // voxel of the parked interaction
         int pm = 0;      // its material
-        unsigned steps = 0, visits = 0, crossings = 0, err = 0, skipped = 0;
+        unsigned steps = 0, visits = 0, crossings = 0, err = 0;
         int cx = 0, cy = 0, cz = 0; // macro cell of the photon (MACRO tracking)
         bool fresh = false;
-        if (BOX)
-            sOuterVisits[threadIdx.x] = 0u;
 
         for (;;) {
             const unsigned stepping = __ballot_sync(kFull, st == kStepping);
@@ -521,16 +217,14 @@ namespace {
             const int nStep = __popc(stepping);
 
             // ---- refill
-            if (dead && !ls.exhausted() && (__popc(dead) >= refillBatch || nStep == 0)) {
-                unsigned long long poolNext, poolEnd;
-                ls.loadPool(poolNext, poolEnd);
+            if (dead && !exhausted && (__popc(dead) >= refillBatch || nStep == 0)) {
                 if (poolNext >= poolEnd) {
                     unsigned long long base = 0;
                     if (lane == 0)
                         base = atomicAdd(&ctr->next, static_cast<unsigned long long>(kChunk));
                     base = __shfl_sync(kFull, base, 0);
                     if (base >= h_end) {
-                        ls.markExhausted();
+                        exhausted = true;
                         poolNext = poolEnd = 0;
                     } else {
                         poolNext = base;
@@ -558,7 +252,7 @@ namespace {
                     const DevJob& Jr = MULTI ? jobs[jid] : J0;
                     rng.init(Jr.key, h);
                     sampleSource(Jr, h, ph, rng);
-                    ls.template add<kSumSource>(ph.w * ph.E);
+                    sum[kSumSource].add(ph.w * ph.E);
                     entered = enterGrid(Jr, ph);
                     if (entered) {
                         st = kStepping;
@@ -568,21 +262,16 @@ namespace {
                             gridPos(ph.E, ec.ie, ec.fe);
                         else
                             ec.set(Jr, ph.E);
-                        if (BOX && Jr.boxOn
-                            && outsideBox(Jr, __float2int_rd(ph.px * Jr.isp[0]), __float2int_rd(ph.py * Jr.isp[1]),
-                                __float2int_rd(ph.pz * Jr.isp[2])))
-                            ec.toOuter(Jr);
                         if (TRACKING == DXMCG_TRACK_MACRO) {
                             cx = min(static_cast<int>(ph.px / Jr.cellL[0]), Jr.mc[0] - 1);
                             cy = min(static_cast<int>(ph.py / Jr.cellL[1]), Jr.mc[1] - 1);
                             cz = min(static_cast<int>(ph.pz / Jr.cellL[2]), Jr.mc[2] - 1);
                         }
                     } else {
-                        ls.template add<kSumEscaped>(ph.w * ph.E);
+                        sum[kSumEscaped].add(ph.w * ph.E);
                     }
                 }
                 poolNext += min(static_cast<unsigned long long>(__popc(dead)), avail);
-                ls.storePool(poolNext, poolEnd);
                 const unsigned mStart = __ballot_sync(kFull, start);
                 const unsigned mIn = __ballot_sync(kFull, entered);
                 if (lane == 0 && mStart) {
@@ -612,12 +301,12 @@ namespace {
                 if (compton) {
                     const float e = ph.w * (ph.E - Ep);
                     deposit(J.tally, pv, e);
-                    ls.template add<kSumDeposited>(e);
+                    sum[kSumDeposited].add(e);
                     ph.E = Ep;
                     if (Ep < 1.0f) {
                         const float r = ph.w * Ep;
                         deposit(J.tally, pv, r);
-                        ls.template add<kSumDeposited>(r);
+                        sum[kSumDeposited].add(r);
                         st = kDead;
                         cut = true;
                     } else {
@@ -635,7 +324,7 @@ namespace {
                     const float Ef = samplePhotoFluorescence(ph.E, J.mats + pm, rng);
                     const float e = ph.w * (ph.E - Ef);
                     deposit(J.tally, pv, e);
-                    ls.template add<kSumDeposited>(e);
+                    sum[kSumDeposited].add(e);
                     if (Ef > 0.0f) {
                         const float u1 = rng.u();
                         isotropicDirection(ph.dx, ph.dy, ph.dz, u1, rng.u());
@@ -667,7 +356,7 @@ namespace {
             }
 
             if (__ballot_sync(kFull, st != kDead) == 0u) {
-                if (ls.exhausted())
+                if (exhausted)
                     break;
                 continue;
             }
@@ -679,21 +368,12 @@ namespace {
                 uint32_t v = 0;
                 int m = 0;
                 bool real = false;
-                if (WOODCOCK) {
-                    // several steps per phase: most are virtual, and each phase boundary
-                    // costs the warp its votes; a lane stops at a real collision or escape
-                    for (int k = 0;;) {
-                        real = woodcockStep<PACKED, BOX>(J, ph, rng, ec, escaped, v, m, visits, skipped);
-                        if (real || escaped || ++k >= woodcockSteps)
-                            break;
-                        ++steps;
-                    }
-                } else if (TRACKING == DXMCG_TRACK_SIDDON)
+                if (TRACKING == DXMCG_TRACK_SIDDON)
                     real = siddonFlight<PACKED>(J, ph, rng, ec, escaped, v, m, visits);
                 else
                     real = macroFlight<PACKED>(J, ph, rng, ec, cx, cy, cz, escaped, v, m, visits, crossings, err);
                 if (escaped) {
-                    ls.template add<kSumEscaped>(ph.w * ph.E);
+                    sum[kSumEscaped].add(ph.w * ph.E);
                     st = kDead;
                 } else if (real) {
                     first = fresh;
@@ -713,7 +393,7 @@ namespace {
                         } else {
                             const float e = ph.w * ph.E;
                             deposit(J.tally, v, e);
-                            ls.template add<kSumDeposited>(e);
+                            sum[kSumDeposited].add(e);
                             st = kDead;
                         }
                     } else {
@@ -744,11 +424,9 @@ namespace {
         // ---- flush: per-lane sums by warp, block counters by one thread
         const unsigned long long vi = warpSum(static_cast<unsigned long long>(visits));
         const unsigned long long cr = warpSum(static_cast<unsigned long long>(crossings));
-        const unsigned long long sk = warpSum(static_cast<unsigned long long>(skipped));
-        const unsigned long long ov = BOX ? warpSum(static_cast<unsigned long long>(sOuterVisits[threadIdx.x])) : 0ull;
-        const double es = warpSum(ls.template value<kSumSource>());
-        const double ee = warpSum(ls.template value<kSumEscaped>());
-        const double ed = warpSum(ls.template value<kSumDeposited>());
+        const double es = warpSum(sum[kSumSource].value());
+        const double ee = warpSum(sum[kSumEscaped].value());
+        const double ed = warpSum(sum[kSumDeposited].value());
         unsigned errAll = err;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
@@ -758,81 +436,63 @@ namespace {
             atomicAdd(&ctr->visits, vi);
             if (cr)
                 atomicAdd(&ctr->crossings, cr);
-            if (sk)
-                atomicAdd(&ctr->skipped, sk);
-            if (ov)
-                atomicAdd(&ctr->outer, ov);
             atomicAdd(&ctr->e_source, es);
             atomicAdd(&ctr->e_escaped, ee);
             atomicAdd(&ctr->e_deposited, ed);
             if (errAll)
                 atomicOr(&ctr->error_flags, errAll);
-            atomicAdd(&ctr->histories, sCount[cHist]);
-            atomicAdd(&ctr->missed, sCount[cMissed]);
-            atomicAdd(&ctr->photo, sCount[cPhoto]);
-            atomicAdd(&ctr->compton, sCount[cCompton]);
-            atomicAdd(&ctr->rayleigh, sCount[cRayleigh]);
-            atomicAdd(&ctr->cutoff, sCount[cCutoff]);
-            atomicAdd(&ctr->errors, sCount[cErrors]);
-            atomicAdd(&ctr->interacted, sCount[cInteracted]);
-            if (sCount[cFluorescence])
-                atomicAdd(&ctr->fluorescence, sCount[cFluorescence]);
+            flushCounts(ctr, sCount);
         }
     }
 
 } // namespace
 
 namespace {
-    using TransportFn = void (*)(const DevJob, const DevJob*, const unsigned long long*, int, unsigned long long,
-        DevCounters*, int, int, int);
-
     // kernel instance for a tracking mode on the packed (world) or unpacked
-    // (caller-owned arrays) voxel layout, single job or a batch of jobs;
-    // nullptr where no instance exists
-    TransportFn kernelFor(int tracking, bool packed, bool multi = false)
+    // (caller-owned arrays) voxel layout, single job or a batch of jobs, with n_mats
+    // materials; nullptr where no instance exists
+    TransportFn kernelFor(int tracking, bool packed, bool multi, int n_mats)
     {
-        if (multi) {
-            switch (tracking) {
-            case DXMCG_TRACK_WOODCOCK: return transportKernel<DXMCG_TRACK_WOODCOCK, true, true>;
-            case kTrackWoodcockBox: return transportKernel<kTrackWoodcockBox, true, true>;
-            case DXMCG_TRACK_SIDDON: return transportKernel<DXMCG_TRACK_SIDDON, true, true>;
-            case DXMCG_TRACK_MACRO: return transportKernel<DXMCG_TRACK_MACRO, true, true>;
-            default: return nullptr;
-            }
-        }
-        if (packed) {
-            switch (tracking) {
-            case DXMCG_TRACK_WOODCOCK: return transportKernel<DXMCG_TRACK_WOODCOCK, true, false>;
-            case kTrackWoodcockBox: return transportKernel<kTrackWoodcockBox, true, false>;
-            case DXMCG_TRACK_SIDDON: return transportKernel<DXMCG_TRACK_SIDDON, true, false>;
-            case DXMCG_TRACK_MACRO: return transportKernel<DXMCG_TRACK_MACRO, true, false>;
-            default: return nullptr;
-            }
-        }
-        switch (tracking) {
-        case DXMCG_TRACK_WOODCOCK: return transportKernel<DXMCG_TRACK_WOODCOCK, false, false>;
-        case kTrackWoodcockBox: return transportKernel<kTrackWoodcockBox, false, false>;
-        case DXMCG_TRACK_SIDDON: return transportKernel<DXMCG_TRACK_SIDDON, false, false>;
-        default: return nullptr;
-        }
+        if (tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox)
+            return woodcockKernelFor(packed, tracking == kTrackWoodcockBox, multi, n_mats);
+        const bool siddon = tracking == DXMCG_TRACK_SIDDON;
+        if (!siddon && (tracking != DXMCG_TRACK_MACRO || !packed))
+            return nullptr;
+        if (multi)
+            return siddon ? transportKernel<DXMCG_TRACK_SIDDON, true, true>
+                          : transportKernel<DXMCG_TRACK_MACRO, true, true>;
+        if (!packed)
+            return transportKernel<DXMCG_TRACK_SIDDON, false, false>;
+        return siddon ? transportKernel<DXMCG_TRACK_SIDDON, true, false>
+                      : transportKernel<DXMCG_TRACK_MACRO, true, false>;
     }
 
-    cudaError_t launchWith(TransportFn fn, const DevJob& job, const DevJob* jobs, const unsigned long long* offsets,
-        int nJobs, unsigned long long h_end, DevCounters* ctr, LaunchShape shape, cudaStream_t s)
+    cudaError_t launchWith(int tracking, bool packed, const DevJob& job, const DevJob* jobs,
+        const unsigned long long* offsets, int nJobs, unsigned long long h_end, DevCounters* ctr, LaunchShape shape,
+        cudaStream_t s)
     {
+        const bool multi = jobs != nullptr;
+        const bool woodcock = tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox;
+        const TransportFn fn = kernelFor(tracking, packed, multi, job.n_mats);
         if (!fn)
             return cudaErrorInvalidValue;
-        const int refill = shape.refill_batch > 0 ? shape.refill_batch : 8;
-        const int interact = shape.interact_batch > 0 ? shape.interact_batch : 8;
+        const int refill = shape.refill_batch > 0 ? shape.refill_batch : (woodcock ? kWoodcockRefillBatch : 8);
+        const int interact
+            = shape.interact_batch > 0 ? shape.interact_batch : (woodcock ? kWoodcockInteractBatch : 8);
         const int wsteps = shape.woodcock_steps > 0 ? shape.woodcock_steps : 8;
-        fn<<<shape.grid, shape.block, 0, s>>>(job, jobs, offsets, nJobs, h_end, ctr, refill, interact, wsteps);
+        const size_t smem = woodcock ? woodcockSharedBytes(shape.block, multi, job.n_mats) : 0;
+        fn<<<shape.grid, shape.block, smem, s>>>(job, jobs, offsets, nJobs, h_end, ctr, refill, interact, wsteps);
         return cudaGetLastError();
     }
 
-    int residentBlocks(TransportFn fn, int block)
+    // resident blocks per SM of the instance that needs most shared memory
+    int residentBlocks(int tracking, bool packed, bool multi, int block)
     {
         int n = 0;
-        if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, 0) != cudaSuccess)
+        const bool woodcock = tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox;
+        const TransportFn fn = kernelFor(tracking, packed, multi, kSharedTableMaterials);
+        const size_t smem = woodcock ? woodcockSharedBytes(block, multi, kSharedTableMaterials) : 0;
+        if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) != cudaSuccess)
             return 1;
         return n > 0 ? n : 1;
     }
@@ -841,13 +501,13 @@ namespace {
 cudaError_t launchTransport(const DevJob& job, unsigned long long h_end, DevCounters* ctr, LaunchShape shape,
     cudaStream_t s)
 {
-    return launchWith(kernelFor(kernelTracking(job), true), job, nullptr, nullptr, 1, h_end, ctr, shape, s);
+    return launchWith(kernelTracking(job), true, job, nullptr, nullptr, 1, h_end, ctr, shape, s);
 }
 
 cudaError_t launchTransportUnpacked(const DevJob& job, unsigned long long h_end, DevCounters* ctr,
     LaunchShape shape, cudaStream_t s)
 {
-    return launchWith(kernelFor(kernelTracking(job), false), job, nullptr, nullptr, 1, h_end, ctr, shape, s);
+    return launchWith(kernelTracking(job), false, job, nullptr, nullptr, 1, h_end, ctr, shape, s);
 }
 
 cudaError_t launchTransportBatch(int tracking, const DevJob* jobs, const unsigned long long* offsets, int nJobs,
@@ -856,19 +516,19 @@ cudaError_t launchTransportBatch(int tracking, const DevJob* jobs, const unsigne
     if (!jobs || !offsets || nJobs < 1)
         return cudaErrorInvalidValue;
     const DevJob unused {};
-    return launchWith(kernelFor(tracking, true, true), unused, jobs, offsets, nJobs, h_end, ctr, shape, s);
+    return launchWith(tracking, true, unused, jobs, offsets, nJobs, h_end, ctr, shape, s);
 }
 
-int transportMaxBlocksPerSMBatch(int block, int tracking) { return residentBlocks(kernelFor(tracking, true, true), block); }
+int transportMaxBlocksPerSMBatch(int block, int tracking) { return residentBlocks(tracking, true, true, block); }
 
-int transportMaxBlocksPerSMUnpacked(int block, int tracking) { return residentBlocks(kernelFor(tracking, false), block); }
+int transportMaxBlocksPerSMUnpacked(int block, int tracking) { return residentBlocks(tracking, false, false, block); }
 
-int transportMaxBlocksPerSM(int block, int tracking) { return residentBlocks(kernelFor(tracking, true), block); }
+int transportMaxBlocksPerSM(int block, int tracking) { return residentBlocks(tracking, true, false, block); }
 
 int transportRegistersPerThread(int tracking)
 {
     cudaFuncAttributes a {};
-    const TransportFn fn = kernelFor(tracking, true);
+    const TransportFn fn = kernelFor(tracking, true, false, kSharedTableMaterials);
     return fn && cudaFuncGetAttributes(&a, fn) == cudaSuccess ? a.numRegs : -1;
 }
 
