@@ -179,23 +179,72 @@ namespace {
         }
     }
 
+    // factors[k] = toDose / (1 + k / 2^15), correctly rounded
+    __global__ void doseFactorKernel(double toDose, double* __restrict__ factors)
+    {
+        const int k = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+        if (k < kDoseFactors)
+            factors[k] = toDose / (1.0 + static_cast<double>(k) * (1.0 / kDoseFactors));
+    }
+
+    // a / b for an integer-valued b, given y = 1 / b correctly rounded: each step adds the
+    // exact residual's share; after the first the quotient is faithful, and the second
+    // then rounds it correctly (Markstein, IBM J. Res. Dev. 34, 111, 1990).
+    __device__ __forceinline__ double quotient(double a, double b, double y)
+    {
+        double q = a * y;
+        q = fma(fma(-b, q, a), y, q);
+        return fma(fma(-b, q, a), y, q);
+    }
+
+    // Dose, variance and event count of each voxel.  The pass moves 32 bytes of tally in
+    // and 24 bytes out a voxel; its FP64 arithmetic bound it (0.068 us per thousand voxels
+    // on the device, with two divisions each).  So a voxel without events, whose results
+    // are zeros, does none and does not read its word, and the divisions are a table
+    // entry and two corrected products with a reciprocal, the same doubles.  VEC: two
+    // voxels a thread, 16-byte stores.  Eight worlds of 0.7-1.4 million voxels into device
+    // memory: 594 -> 168 us in all; 105 million voxels: 7.2 -> 1.53 ms (0.94 at the
+    // copy rate).  Into pinned host memory the link bounds it, 193 GB/s, as a copy measures.
+    template <bool VEC>
     __global__ void finalizeKernel(const Tally* __restrict__ t, const uint32_t* __restrict__ vox, size_t n,
-        double toDose, double nh, double* __restrict__ dose, double* __restrict__ var,
+        DoseScale scale, double nh, double invNh, double* __restrict__ dose, double* __restrict__ var,
         unsigned long long* __restrict__ cnt)
     {
-        for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
-             i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-            const Tally r = t[i];
-            const float rho = __uint_as_float(vox[i] & 0xffffff00u);
-            const double s = rho > 0.0f ? toDose / rho : 0.0;
+        constexpr int V = VEC ? 2 : 1;
+        const size_t i = V * (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x);
+        if (i >= n)
+            return;
+        double d[V], v[V];
+        unsigned long long c[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            d[k] = v[k] = 0.0;
+            c[k] = 0ull;
+            if (VEC && i + k >= n)
+                continue;
+            const double2 e = *reinterpret_cast<const double2*>(&t[i + k].e);
+            c[k] = t[i + k].n;
+            if (c[k] == 0ull)
+                continue;
+            const double s = doseFactor(scale, vox[i + k]);
+            d[k] = e.x * s;
+            const double x = nh > 0 ? e.y - quotient(e.x * e.x, nh, invNh) : 0.0;
+            v[k] = (x > 0.0 ? x : 0.0) * s * s;
+        }
+        if (VEC && i + 1 < n) {
             if (dose)
-                dose[i] = r.e * s;
-            if (var) {
-                const double v = nh > 0 ? (r.e2 - r.e * r.e / nh) : 0.0;
-                var[i] = (v > 0.0 ? v : 0.0) * s * s;
-            }
+                *reinterpret_cast<double2*>(dose + i) = make_double2(d[0], d[V - 1]);
+            if (var)
+                *reinterpret_cast<double2*>(var + i) = make_double2(v[0], v[V - 1]);
             if (cnt)
-                cnt[i] = r.n;
+                *reinterpret_cast<ulonglong2*>(cnt + i) = make_ulonglong2(c[0], c[V - 1]);
+        } else {
+            if (dose)
+                dose[i] = d[0];
+            if (var)
+                var[i] = v[0];
+            if (cnt)
+                cnt[i] = c[0];
         }
     }
 
@@ -366,10 +415,26 @@ cudaError_t launchMaterialBox(const uint8_t* mat, int nx, int ny, int nz, int* b
     return cudaGetLastError();
 }
 
-cudaError_t launchFinalize(const Tally* tally, const uint32_t* vox, size_t n, double energy_to_dose,
-    double n_histories, double* dose, double* var, unsigned long long* count, cudaStream_t s)
+cudaError_t launchDoseFactors(double toDose, double* factors, cudaStream_t s)
 {
-    finalizeKernel<<<gridFor(n, 256), 256, 0, s>>>(tally, vox, n, energy_to_dose, n_histories, dose, var, count);
+    doseFactorKernel<<<kDoseFactors / 256, 256, 0, s>>>(toDose, factors);
+    return cudaGetLastError();
+}
+
+cudaError_t launchFinalize(const Tally* tally, const uint32_t* vox, size_t n, DoseScale scale, double n_histories,
+    double* dose, double* var, unsigned long long* count, cudaStream_t s)
+{
+    const double inv = n_histories > 0 ? 1.0 / n_histories : 0.0;
+    const bool vec = ((reinterpret_cast<uintptr_t>(dose) | reinterpret_cast<uintptr_t>(var)
+                          | reinterpret_cast<uintptr_t>(count))
+                         & 15u)
+        == 0u;
+    if (vec)
+        finalizeKernel<true><<<gridFor((n + 1) / 2, 256), 256, 0, s>>>(tally, vox, n, scale, n_histories, inv, dose,
+            var, count);
+    else
+        finalizeKernel<false><<<gridFor(n, 256), 256, 0, s>>>(tally, vox, n, scale, n_histories, inv, dose, var,
+            count);
     return cudaGetLastError();
 }
 

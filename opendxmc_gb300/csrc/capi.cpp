@@ -158,6 +158,9 @@ struct dxmcg_world {
     std::vector<double> rhoMax;
     double historiesScored = 0.0;
     double voxelVolume = 0.0;
+    DeviceBuffer<double> doseFactors; // of the voxel volume, filled by the first build
+
+    DoseScale doseScale() const { return { kKeVToMilliGrayGram / voxelVolume, doseFactors.p }; }
 };
 
 namespace {
@@ -898,6 +901,14 @@ DXMCG_API int dxmcg_world_build(dxmcg_world* w)
     DXMCG_CUDA(w->rtab.alloc(rtab.size()));
     DXMCG_CUDA(cudaMemcpyAsync(w->rtab.p, rtab.data(), rtab.size() * sizeof(float), cudaMemcpyHostToDevice, w->stream));
     DXMCG_CUDA(cudaMemsetAsync(w->tally.p, 0, w->N * sizeof(Tally), w->stream));
+    // every factor, for any density, a normal double
+    const double toDose = kKeVToMilliGrayGram / w->voxelVolume;
+    if (!w->doseFactors.p && toDose > 1e-200 && toDose < 1e200) {
+        DXMCG_CUDA(w->doseFactors.alloc(kDoseFactors));
+        e = launchDoseFactors(toDose, w->doseFactors.p, w->stream);
+        if (e != cudaSuccess)
+            return cudaFail(e, "dose-factor kernel");
+    }
     // gather-skip bounds of the Woodcock step
     {
         const std::vector<float> ratio = majorantRatios(w);
@@ -1022,8 +1033,8 @@ DXMCG_API int dxmcg_world_read_dose(dxmcg_world* w, double* dose, double* varian
         DXMCG_CUDA(w->readCount.alloc(w->N));
         dc = w->readCount.p;
     }
-    cudaError_t e = launchFinalize(w->tally.p, w->vox.p, w->N, kKeVToMilliGrayGram / w->voxelVolume,
-        w->historiesScored, dd, dv, dc, w->stream);
+    cudaError_t e
+        = launchFinalize(w->tally.p, w->vox.p, w->N, w->doseScale(), w->historiesScored, dd, dv, dc, w->stream);
     if (e != cudaSuccess)
         return cudaFail(e, "finalize kernel");
     if (dose && dd == w->readDose.p)
@@ -1646,7 +1657,7 @@ DXMCG_API int dxmcg_world_read_dose_postprocessed(dxmcg_world* w, int delete_air
         DXMCG_CUDA(c.alloc(w->N));
     DXMCG_CUDA(mx.alloc(1));
     DXMCG_CUDA(micro.alloc(1));
-    const cudaError_t e = launchDosePostprocess(w->tally.p, w->vox.p, w->N, kKeVToMilliGrayGram / w->voxelVolume,
+    const cudaError_t e = launchDosePostprocess(w->tally.p, w->vox.p, w->N, w->doseScale(),
         w->historiesScored, delete_air_dose ? 1 : 0, mx.p, dose ? d.p : nullptr, variance ? v.p : nullptr,
         count ? c.p : nullptr, micro.p, w->stream);
     if (e != cudaSuccess)
@@ -1675,7 +1686,7 @@ DXMCG_API int dxmcg_world_denoise(dxmcg_world* w, dxmcg_denoiser* d, double scal
     DXMCG_CUDA(cudaSetDevice(w->device));
     DXMCG_CUDA(cudaStreamSynchronize(w->stream));
     return nn::denoiseWorld(d, w->device, w->tally.p, w->vox.p, w->dims[0], w->dims[1], w->dims[2],
-        kKeVToMilliGrayGram / w->voxelVolume, scale, dose_out, scale_used, w->stream);
+        w->doseScale(), scale, dose_out, scale_used, w->stream);
 }
 
 DXMCG_API dxmcg_progress* dxmcg_progress_create(void) { return new dxmcg_progress(); }

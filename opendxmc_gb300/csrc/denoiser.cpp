@@ -462,7 +462,7 @@ namespace dxmcg {
 namespace nn {
     // the world path (capi.cpp): input from a tally, forward, dose = pred * scale
     int denoiseWorld(dxmcg_denoiser* d, int device, const Tally* tally, const uint32_t* vox, int nx, int ny, int nz,
-        double toDose, double scale, double* hostOut, double* scaleUsed, cudaStream_t s)
+        DoseScale toDose, double scale, double* hostOut, double* scaleUsed, cudaStream_t s)
     {
         int rc = checkNet(d);
         if (rc != DXMCG_OK)
@@ -477,7 +477,7 @@ namespace nn {
             NN_CUDA(d->meanCount.reserve(1));
             NN_CUDA(cudaMemsetAsync(d->meanSum.p, 0, sizeof(double), s));
             NN_CUDA(cudaMemsetAsync(d->meanCount.p, 0, sizeof(unsigned long long), s));
-            NN_CUDA(launchDoseMean(tally, vox, toDose, n, 0.2f, d->meanSum.p, d->meanCount.p, s));
+            NN_CUDA(launchDoseMean(tally, vox, toDose.toDose, n, 0.2f, d->meanSum.p, d->meanCount.p, s));
             double hs = 0;
             unsigned long long hc = 0;
             NN_CUDA(cudaMemcpyAsync(&hs, d->meanSum.p, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -828,7 +828,7 @@ DXMCG_API int dxmcg_denoiser_prepare_input(const float* dose, const float* densi
         return DXMCG_OK;
     if (!dose || !density || !material || !input || !(scale > 0.0))
         return fail(DXMCG_ERR_ARGUMENT, "denoiser_prepare_input: null array or scale <= 0");
-    NN_CUDA(nn::launchPrepareInput(dose, density, material, nullptr, nullptr, 0.0, n, static_cast<float>(1.0 / scale),
+    NN_CUDA(nn::launchPrepareInput(dose, density, material, nullptr, nullptr, DoseScale {}, n, static_cast<float>(1.0 / scale),
         static_cast<bf16*>(input), static_cast<cudaStream_t>(cuda_stream)));
     return DXMCG_OK;
 }

@@ -132,7 +132,7 @@ struct BrickMarks {
 // (dose, dens, mat) or from a world (tally, vox, toDose); with a world, optionally
 // the brick marks above (fewer than 2^32 voxels)
 cudaError_t launchPrepareInput(const float* dose, const float* dens, const uint8_t* mat, const Tally* tally,
-    const uint32_t* vox, double toDose, size_t n, float invScale, __nv_bfloat16* out, cudaStream_t s,
+    const uint32_t* vox, DoseScale toDose, size_t n, float invScale, __nv_bfloat16* out, cudaStream_t s,
     const BrickMarks* marks = nullptr);
 // patches outside their volume (or of a volume index out of range) are written as zeros
 cudaError_t launchGatherPatches(const __nv_bfloat16* const* inputs, const float* const* targets, const int* dims,
@@ -142,7 +142,7 @@ cudaError_t launchDoseMean(const Tally* tally, const uint32_t* vox, double toDos
 
 // a world's dose through the network (denoiser.cpp); dims nx, ny, nz (x fastest)
 int denoiseWorld(dxmcg_denoiser* d, int device, const Tally* tally, const uint32_t* vox, int nx, int ny, int nz,
-    double toDose, double scale, double* hostOut, double* scaleUsed, cudaStream_t s);
+    DoseScale toDose, double scale, double* hostOut, double* scaleUsed, cudaStream_t s);
 
 } // namespace nn
 } // namespace dxmcg

@@ -19,6 +19,7 @@
 #include <cuda_bf16.h>
 
 #include "denoiser.hpp"
+#include "device.cuh"
 
 namespace dxmcg {
 namespace nn {
@@ -590,7 +591,7 @@ namespace {
     // the bricks holding a non-air voxel are marked too when marks.active is set.
     __global__ void prepareInputKernel(const float* __restrict__ dose, const float* __restrict__ dens,
         const uint8_t* __restrict__ mat, const Tally* __restrict__ tally, const uint32_t* __restrict__ vox,
-        double toDose, size_t n, float invScale, uint4* __restrict__ out, const BrickMarks marks)
+        DoseScale toDose, size_t n, float invScale, uint4* __restrict__ out, const BrickMarks marks)
     {
         for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
              i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -601,7 +602,7 @@ namespace {
                 rho = __uint_as_float(w & 0xffffff00u);
                 m = static_cast<int>(w & 0xffu);
                 // air (material 0) enters with zero dose, as the worker's readout deletes it
-                d = rho > 0.0f && m != 0 ? static_cast<float>(tally[i].e * (toDose / rho)) : 0.0f;
+                d = rho > 0.0f && m != 0 ? static_cast<float>(tally[i].e * dev::doseFactor(toDose, w)) : 0.0f;
                 if (marks.active && m != 0) {
                     const uint32_t v = static_cast<uint32_t>(i);
                     const uint32_t row = v / static_cast<uint32_t>(marks.nx);
@@ -817,7 +818,7 @@ cudaError_t launchTransposeWeights(const __nv_bfloat16* w, __nv_bfloat16* wt, in
 }
 
 cudaError_t launchPrepareInput(const float* dose, const float* dens, const uint8_t* mat, const Tally* tally,
-    const uint32_t* vox, double toDose, size_t n, float invScale, __nv_bfloat16* out, cudaStream_t s,
+    const uint32_t* vox, DoseScale toDose, size_t n, float invScale, __nv_bfloat16* out, cudaStream_t s,
     const BrickMarks* marks)
 {
     const BrickMarks none {};

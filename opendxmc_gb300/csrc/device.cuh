@@ -403,6 +403,22 @@ namespace dev {
         atomicAdd(&tally[v].n, 1ull);
     }
 
+    // toDose / rho of a packed voxel word, 0 without density; the same double as the
+    // division gives (see DoseScale).  FP64 runs at 2 lanes a clock and SM here, and a
+    // division is some ten FP64 operations: one 8-byte load of a table that stays in L1
+    // (a material's +-2 % of density are a few hundred entries) takes its place.
+    __device__ __forceinline__ double doseFactor(const DoseScale& c, uint32_t word)
+    {
+        const uint32_t bits = word & 0xffffff00u;
+        if (bits == 0u)
+            return 0.0;
+        const int e = static_cast<int>(bits >> 23); // densities are positive
+        if (!c.factors || e == 0)
+            return c.toDose / static_cast<double>(__uint_as_float(bits));
+        const long long f = __double_as_longlong(__ldg(c.factors + (bits >> 8 & 0x7fffu)));
+        return __longlong_as_double(f - (static_cast<long long>(e - 127) << 52));
+    }
+
     // relative bowtie weight of tube `tube` at |fan angle| a (1 when that tube has none)
     __device__ __forceinline__ float bowtieAt(const DevBowtie* __restrict__ b, int tube, float a)
     {

@@ -96,6 +96,17 @@ struct alignas(32) Tally {
     unsigned long long pad;
 };
 
+// Dose per unit energy of a voxel: toDose / rho.  A packed density has 15 mantissa bits,
+// so with rho = m 2^k, 1 <= m < 2, the quotient is one of kDoseFactors correctly rounded
+// ones (`factors`, filled by launchDoseFactors for toDose) times an exact power of two.
+// Without the table (nullptr: a toDose whose factors might leave the normal range) it is
+// divided.
+struct DoseScale {
+    double toDose = 0.0;
+    const double* factors = nullptr;
+};
+constexpr int kDoseFactors = 1 << 15;
+
 struct DevJob {
     // world
     const uint32_t* vox;
@@ -220,8 +231,9 @@ cudaError_t launchMaterialBox(const uint32_t* vox, int nx, int ny, int nz, int* 
 cudaError_t launchMaterialBox(const uint8_t* mat, int nx, int ny, int nz, int* box, cudaStream_t s);
 cudaError_t launchCellBound(const uint32_t* vox, int nx, int ny, int nz, int ncx, int ncy, int ncz, const float* ratio,
     float* bound, cudaStream_t s);
-cudaError_t launchFinalize(const Tally* tally, const uint32_t* vox, size_t n, double energy_to_dose,
-    double n_histories, double* dose, double* var, unsigned long long* count, cudaStream_t s);
+cudaError_t launchDoseFactors(double toDose, double* factors, cudaStream_t s);
+cudaError_t launchFinalize(const Tally* tally, const uint32_t* vox, size_t n, DoseScale scale, double n_histories,
+    double* dose, double* var, unsigned long long* count, cudaStream_t s);
 cudaError_t launchSiddon(int n_rays, const float* o, const float* d, int nx, int ny, int nz, float sx, float sy,
     float sz, int cap, long long* idx, float* len, int* cnt, cudaStream_t s);
 cudaError_t launchSampleCompton(int n, const float* E, const DevMaterial* m, const float* ctab, int correction,
@@ -270,7 +282,7 @@ cudaError_t launchOrganTable(const uint8_t* organ, const double* dose, const dou
 cudaError_t launchWorldOrganTable(const uint8_t* organ, const Tally* tally, const uint32_t* vox, size_t n,
     double energy_to_dose, int air_mask, double voxel_volume, int n_organs, unsigned long long* cnt,
     double* sum_rho, double* sum_e, cudaStream_t s);
-cudaError_t launchDosePostprocess(const Tally* tally, const uint32_t* vox, size_t n, double energy_to_dose,
+cudaError_t launchDosePostprocess(const Tally* tally, const uint32_t* vox, size_t n, DoseScale scale,
     double n_histories, int air_mask, unsigned long long* max_bits, double* dose, double* var, double* count,
     int* micro, cudaStream_t s);
 

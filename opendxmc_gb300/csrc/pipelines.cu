@@ -226,22 +226,21 @@ namespace {
     }
 
     // ---------------------------------------------------------------- dose post-processing
-    __device__ __forceinline__ double voxelDose(const Tally& r, uint32_t w, double toDose, int airMask)
+    __device__ __forceinline__ double voxelDose(double e, uint32_t w, const DoseScale& scale, int airMask)
     {
-        const float rho = __uint_as_float(w & 0xffffff00u);
         if (airMask && (w & 0xffu) == 0u)
             return 0.0;
-        return rho > 0.0f ? r.e * (toDose / rho) : 0.0;
+        return e * doseFactor(scale, w);
     }
 
     // maximum dose (non-negative doubles order like their bit patterns)
     __global__ void doseMaxKernel(const Tally* __restrict__ t, const uint32_t* __restrict__ vox, size_t n,
-        double toDose, int airMask, unsigned long long* __restrict__ maxBits)
+        DoseScale scale, int airMask, unsigned long long* __restrict__ maxBits)
     {
         double m = 0.0;
         for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
              i += static_cast<size_t>(gridDim.x) * blockDim.x)
-            m = fmax(m, voxelDose(t[i], vox[i], toDose, airMask));
+            m = fmax(m, voxelDose(t[i].e, vox[i], scale, airMask));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
             m = fmax(m, __shfl_xor_sync(kFull, m, o));
@@ -250,7 +249,7 @@ namespace {
     }
 
     __global__ void postprocessKernel(const Tally* __restrict__ t, const uint32_t* __restrict__ vox, size_t n,
-        double toDose, double nh, int airMask, const unsigned long long* __restrict__ maxBits,
+        DoseScale scale, double nh, int airMask, const unsigned long long* __restrict__ maxBits,
         double* __restrict__ dose, double* __restrict__ var, double* __restrict__ count, int* __restrict__ micro)
     {
         const bool uGy = __longlong_as_double(static_cast<long long>(*maxBits)) < 1.0;
@@ -261,8 +260,7 @@ namespace {
             const Tally r = t[i];
             const uint32_t w = vox[i];
             const bool masked = airMask && (w & 0xffu) == 0u;
-            const float rho = __uint_as_float(w & 0xffffff00u);
-            const double s = rho > 0.0f ? toDose / rho : 0.0;
+            const double s = doseFactor(scale, w);
             if (dose) {
                 const double d = masked ? 0.0 : r.e * s;
                 dose[i] = uGy ? d * 1e3 : d;
@@ -324,7 +322,7 @@ cudaError_t launchWorldOrganTable(const uint8_t* organ, const Tally* tally, cons
     return cudaGetLastError();
 }
 
-cudaError_t launchDosePostprocess(const Tally* tally, const uint32_t* vox, size_t n, double energy_to_dose,
+cudaError_t launchDosePostprocess(const Tally* tally, const uint32_t* vox, size_t n, DoseScale scale,
     double n_histories, int air_mask, unsigned long long* max_bits, double* dose, double* var, double* count,
     int* micro, cudaStream_t s)
 {
@@ -332,8 +330,8 @@ cudaError_t launchDosePostprocess(const Tally* tally, const uint32_t* vox, size_
     if (e != cudaSuccess)
         return e;
     const int g = streamingGrid(n);
-    doseMaxKernel<<<g, 256, 0, s>>>(tally, vox, n, energy_to_dose, air_mask, max_bits);
-    postprocessKernel<<<g, 256, 0, s>>>(tally, vox, n, energy_to_dose, n_histories, air_mask, max_bits, dose, var,
+    doseMaxKernel<<<g, 256, 0, s>>>(tally, vox, n, scale, air_mask, max_bits);
+    postprocessKernel<<<g, 256, 0, s>>>(tally, vox, n, scale, n_histories, air_mask, max_bits, dose, var,
         count, micro);
     return cudaGetLastError();
 }
