@@ -108,38 +108,75 @@ namespace dev {
     //                  / (A^2 - rho^2).
     // Accepted when E' > 0 and E - E' exceeds the shell's binding; false after
     // kPzTries draws (the caller then samples a new angle).
+    //
+    // What a trip costs decides the rate here, since a warp waits for its unluckiest lane:
+    //   * above every binding energy the shell comes from the material's running sums (one
+    //     guide entry, a short scan) instead of two loops over up to 48 shells;
+    //   * the polar draw loops by itself, so that lanes meet at the power function;
+    //   * a shell bound more strongly than the Compton line's energy loss accepts only
+    //     p_z well below zero: rho < rho_b, the rho of E' = E - binding.  A draw short of
+    //     it, by a bound wider than the roundings of both, is dropped on a hardware power
+    //     function, or on its sign alone.
+    // The accepted draws, and so the histories, are those of the plain loop.  1e7
+    // histories of a CBCT run at level 2: 4.36 -> 3.60 ms.
     template <class U>
     __device__ bool dopplerEnergy(float E, float A, float omu, const DevMaterial* __restrict__ M, U& r, float& Ep)
     {
         const int ns = M->nShell;
-        float tot = 0.0f;
-        for (int k = 0; k < ns; ++k)
-            if (__ldg(&M->shellBinding[k]) < E)
-                tot += __ldg(&M->shellElectrons[k]);
-        const float target = r.u() * tot;
         int sh = -1;
-        float acc = 0.0f;
-        for (int k = 0; k < ns; ++k) {
-            if (__ldg(&M->shellBinding[k]) < E) {
-                sh = k;
-                acc += __ldg(&M->shellElectrons[k]);
-                if (target <= acc)
-                    break;
+        if (ns > 0 && E > __ldg(&M->shellTop)) {
+            const float u = r.u();
+            const float target = u * __ldg(&M->shellCum[ns - 1]);
+            sh = M->shellStart[static_cast<int>(u * 64.0f)];
+            while (sh < ns - 1 && target > __ldg(&M->shellCum[sh]))
+                ++sh;
+        } else {
+            float tot = 0.0f;
+            for (int k = 0; k < ns; ++k)
+                if (__ldg(&M->shellBinding[k]) < E)
+                    tot += __ldg(&M->shellElectrons[k]);
+            const float target = r.u() * tot;
+            float acc = 0.0f;
+            for (int k = 0; k < ns; ++k) {
+                if (__ldg(&M->shellBinding[k]) < E) {
+                    sh = k;
+                    acc += __ldg(&M->shellElectrons[k]);
+                    if (target <= acc)
+                        break;
+                }
             }
+            if (sh < 0)
+                return false;
         }
-        if (sh < 0)
-            return false;
         const float bind = __ldg(&M->shellBinding[sh]);
         const float ps = __ldg(&M->shellMomentum[sh]);
         const float c = 1.0f - omu;
         const float am = A - c;
         const float sin2 = omu * (2.0f - omu);
-        for (int t = 0; t < kPzTries; ++t) {
-            const float a = 2.0f * r.u() - 1.0f;
-            const float b = 2.0f * r.u() - 1.0f;
-            const float w = a * a + b * b;
-            if (w >= 1.0f)
-                continue;
+        // |rho_b|^2 where rho_b < 0, else 0: of E' = E - bind + 2e-5 E, so that a draw on
+        // the near side of it fails the test below whatever its rounding
+        float need2 = 0.0f;
+        {
+            const float be = __fdividef(bind, E) - 2e-5f, x = 1.0f - be, loss = A - 1.0f;
+            const float lack = be - loss * x - 4e-7f * (1.0f + loss);
+            if (lack > 0.0f) {
+                const float n2 = __fdividef(lack * lack, be * be + 2.0f * x * omu);
+                need2 = fminf(n2, 0.25f) * 0.999f;
+            }
+        }
+        const float ps2 = ps * ps;
+        for (int t = 0;;) {
+            float a, w;
+            do {
+                if (t == kPzTries)
+                    return false;
+                ++t;
+                a = 2.0f * r.u() - 1.0f;
+                const float b = 2.0f * r.u() - 1.0f;
+                w = a * a + b * b;
+            } while (w >= 1.0f
+                || (need2 > 0.0f
+                    && (a >= 0.0f || ps2 * a * a * (__powf(w, -0.4f) - 1.0f + 1e-5f) * 1.001f < need2 * w)));
             const float rho = ps * a * sqrtf((powf(w, -0.4f) - 1.0f) / w);
             const float rho2 = rho * rho;
             const float den = A * A - rho2;
@@ -152,7 +189,6 @@ namespace dev {
                 return true;
             }
         }
-        return false;
     }
 
     // 1 - cos theta from a material's angle quantile table (row ie of tab, interpolated
@@ -232,17 +268,26 @@ namespace dev {
     __device__ float samplePhotoFluorescence(float E, const DevMaterial* __restrict__ M, U& r)
     {
         const int n = M->n;
-        float tot = 0.0f;
-        for (int i = 0; i < n; ++i)
-            tot += photoShare(E, M, i);
-        const float target = r.u() * tot;
         int e = n - 1;
-        float acc = 0.0f;
-        for (int i = 0; i < n; ++i) {
-            acc += photoShare(E, M, i);
-            if (target <= acc) {
-                e = i;
-                break;
+        if (E >= __ldg(&M->edgeTop)) { // no share is below an edge
+            const float target = r.u() * __ldg(&M->z4Cum[n - 1]);
+            for (int i = 0; i < n; ++i)
+                if (target <= __ldg(&M->z4Cum[i])) {
+                    e = i;
+                    break;
+                }
+        } else {
+            float tot = 0.0f;
+            for (int i = 0; i < n; ++i)
+                tot += photoShare(E, M, i);
+            const float target = r.u() * tot;
+            float acc = 0.0f;
+            for (int i = 0; i < n; ++i) {
+                acc += photoShare(E, M, i);
+                if (target <= acc) {
+                    e = i;
+                    break;
+                }
             }
         }
         if (E < __ldg(&M->eK[e]))

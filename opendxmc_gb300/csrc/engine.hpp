@@ -54,6 +54,13 @@ struct DevMaterial {
     float shellElectrons[3 * DXMCG_MAX_ELEMENTS];
     float shellBinding[3 * DXMCG_MAX_ELEMENTS];
     float shellMomentum[3 * DXMCG_MAX_ELEMENTS];
+    // above every edge (E > shellTop, E >= edgeTop) the sums over shells and elements do
+    // not depend on E: their running sums, and per 64th of the shells' total the first
+    // shell a target in it can fall on
+    float shellTop, edgeTop;
+    float shellCum[3 * DXMCG_MAX_ELEMENTS];
+    float z4Cum[DXMCG_MAX_ELEMENTS];
+    uint8_t shellStart[64];
 };
 
 struct alignas(16) DevExposure {

@@ -123,6 +123,28 @@ DevMaterial toDevMaterial(const dxmcg_material& m)
         d.shellBinding[k] = static_cast<float>(s.shellBinding[k]);
         d.shellMomentum[k] = static_cast<float>(s.shellMomentum[k]);
     }
+    // running sums in the order, and with the FP32 additions, of the samplers' loops
+    float acc = 0.0f;
+    d.edgeTop = 0.0f;
+    for (int i = 0; i < d.n; ++i) {
+        acc += d.nZ4[i];
+        d.z4Cum[i] = acc;
+        d.edgeTop = std::max(d.edgeTop, std::max(d.eK[i], d.eL[i]));
+    }
+    acc = 0.0f;
+    d.shellTop = 0.0f;
+    for (int k = 0; k < d.nShell; ++k) {
+        acc += d.shellElectrons[k];
+        d.shellCum[k] = acc;
+        d.shellTop = std::max(d.shellTop, d.shellBinding[k]);
+    }
+    for (int c = 0; c < 64; ++c) {
+        const float least = static_cast<float>(c) * 0.015625f * acc; // of the targets u * acc with 64 u >= c
+        int k = 0;
+        while (k + 1 < d.nShell && least > d.shellCum[k])
+            ++k;
+        d.shellStart[c] = static_cast<uint8_t>(k);
+    }
     return d;
 }
 
