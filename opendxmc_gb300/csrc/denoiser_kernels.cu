@@ -220,6 +220,147 @@ namespace {
             }
     }
 
+    // ------------------------------------------------------------------ forward conv, small grids
+    // The same sums in the same order (input slices, then taps) on bricks of 8 x 4 x 2
+    // voxels and 16 output channels: an eighth of conv3Kernel's brick and half its
+    // channels, so that a volume of a few thousand voxels still gives every SM a CTA.  A
+    // warp owns 16 voxels (8 x 2) and all 16 channels: a chain of 27 Cin / 16 dependent
+    // MMAs (23 cycles each), with the fragments of tap t + 3 read while tap t multiplies
+    // and the slices arriving through a ring of kSmallStages cp.async stages.  A slice
+    // takes about 1 us, bound by the shared-memory pipe: two fragment loads and a share of
+    // the copies for every two MMAs.
+    constexpr int kSmallStages = 3;
+    constexpr int kSmallHaloVox = 4 * 6 * 10;
+    constexpr int kSmallHalo = kSmallHaloVox * 32;
+    constexpr int kSmallStage = kSmallHalo + 27 * 16 * 32;
+
+    __global__ void __launch_bounds__(128) conv3SmallKernel(const ConvIn in, int D, int H, int W, int Cin,
+        const __nv_bfloat16* __restrict__ wgt, const float* __restrict__ bias, int Cout, int relu,
+        __nv_bfloat16* __restrict__ out)
+    {
+        extern __shared__ __align__(128) unsigned char smem[];
+        const int nbx = (W + 7) >> 3, nby = (H + 3) >> 2, nbz = (D + 1) >> 1;
+        int brick = static_cast<int>(blockIdx.x);
+        const int x0 = (brick % nbx) * 8;
+        brick /= nbx;
+        const int y0 = (brick % nby) * 4;
+        brick /= nby;
+        const int z0 = (brick % nbz) * 2;
+        const int bi = brick / nbz;
+        const int n0 = blockIdx.y * 16;
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int nChunks = Cin >> 4;
+        // this thread's share of a slice, 16 bytes a copy: the halo voxels (tid >> 1) + 64 k
+        // (their index in a full- and a half-resolution input, or -1) and the weight rows
+        // tap = (tid >> 5) + 4 k of output channel (tid >> 1) & 15; half tid & 1
+        constexpr int kHaloCopies = (2 * kSmallHaloVox + 127) / 128;
+        constexpr int kWeightCopies = (27 * 16 * 2 + 127) / 128;
+        const int tid = static_cast<int>(threadIdx.x), h = tid & 1;
+        int full[kHaloCopies], low[kHaloCopies];
+        unsigned haloDst[kHaloCopies];
+#pragma unroll
+        for (int k = 0; k < kHaloCopies; ++k) {
+            const int v = (tid >> 1) + 64 * k;
+            const int hz = v / 60, hy = (v / 10) % 6, hx = v % 10;
+            const int gz = z0 + hz - 1, gy = y0 + hy - 1, gx = x0 + hx - 1;
+            const bool ok = gz >= 0 && gz < D && gy >= 0 && gy < H && gx >= 0 && gx < W;
+            full[k] = ok ? ((bi * D + gz) * H + gy) * W + gx : -1;
+            low[k] = ok ? ((bi * (D >> 1) + (gz >> 1)) * (H >> 1) + (gy >> 1)) * (W >> 1) + (gx >> 1) : -1;
+            haloDst[k] = static_cast<unsigned>(v * 32 + ((h ^ ((hx >> 2) & 1)) << 4));
+        }
+        const int wco = (tid >> 1) & 15;
+        const unsigned wDst
+            = static_cast<unsigned>(kSmallHalo + (tid >> 1) * 32 + ((h ^ ((wco >> 2) & 1)) << 4));
+        const __nv_bfloat16* const wSrc
+            = wgt + (static_cast<size_t>(n0 + wco) * 27 + (tid >> 5)) * Cin + h * 8;
+        const auto load = [&](int chunk) {
+            const unsigned sbase = smemAddr(smem + (chunk % kSmallStages) * kSmallStage);
+            const int c0 = chunk * 16;
+            const bool inA = c0 < in.ca;
+            const int cs = inA ? in.ca : in.cb;
+            const __nv_bfloat16* src = (inA ? in.a + c0 : in.b + (c0 - in.ca)) + h * 8;
+            const bool half = inA && in.halfA;
+#pragma unroll
+            for (int k = 0; k < kHaloCopies; ++k) {
+                const int v = half ? low[k] : full[k];
+                if (k < kHaloCopies - 1 || tid + 128 * k < 2 * kSmallHaloVox)
+                    cpAsync16(sbase + haloDst[k], src + (v >= 0 ? static_cast<size_t>(v) * cs : 0), v >= 0);
+            }
+#pragma unroll
+            for (int k = 0; k < kWeightCopies; ++k)
+                if (k < kWeightCopies - 1 || (tid >> 5) + 4 * k < 27)
+                    cpAsync16(sbase + wDst + k * 64 * 32, wSrc + c0 + 4 * k * Cin, true);
+        };
+
+        const int q = lane >> 3, r = lane & 7;
+        // lane's A rows: voxel x = r, y = 2 (warp & 1) + (q & 1), z = warp >> 1; half q >> 1
+        unsigned aOff[3];
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx) {
+            const int hx = r + dx;
+            aOff[dx] = static_cast<unsigned>((((warp >> 1) * 6 + 2 * (warp & 1) + (q & 1)) * 10 + hx) * 32
+                + (((q >> 1) ^ ((hx >> 2) & 1)) << 4));
+        }
+        // its B rows: output channel co, half q & 1
+        const int bco = ((q >> 1) << 3) + r;
+        const unsigned bOff = static_cast<unsigned>(kSmallHalo + bco * 32 + (((q & 1) ^ ((bco >> 2) & 1)) << 4));
+
+        float acc[2][4] = {};
+        for (int c = 0; c < kSmallStages - 1; ++c) {
+            if (c < nChunks)
+                load(c);
+            cpAsyncCommit();
+        }
+        for (int chunk = 0; chunk < nChunks; ++chunk) {
+            cpAsyncWait<kSmallStages - 2>();
+            __syncthreads(); // slice `chunk` landed, and slice chunk - 1 was read by all
+            if (chunk + kSmallStages - 1 < nChunks)
+                load(chunk + kSmallStages - 1);
+            cpAsyncCommit();
+            const unsigned sbase = smemAddr(smem + (chunk % kSmallStages) * kSmallStage);
+            unsigned a[4][4], b[4][4];
+            const auto fragments = [&](int tap, unsigned (&fa)[4], unsigned (&fb)[4]) {
+                const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
+                ldsm4(sbase + aOff[dx] + (dz * 60 + dy * 10) * 32, fa[0], fa[1], fa[2], fa[3]);
+                ldsm4(sbase + bOff + tap * 512, fb[0], fb[1], fb[2], fb[3]);
+            };
+#pragma unroll
+            for (int tap = 0; tap < 3; ++tap)
+                fragments(tap, a[tap], b[tap]);
+#pragma unroll
+            for (int tap = 0; tap < 27; ++tap) {
+                const int k = tap & 3;
+                if (tap + 3 < 27)
+                    fragments(tap + 3, a[(tap + 3) & 3], b[(tap + 3) & 3]);
+                mma16816(acc[0], a[k][0], a[k][1], a[k][2], a[k][3], b[k][0], b[k][1]);
+                mma16816(acc[1], a[k][0], a[k][1], a[k][2], a[k][3], b[k][2], b[k][3]);
+            }
+        }
+
+        const int g = lane >> 2, t = lane & 3;
+        const int z = z0 + (warp >> 1), x = x0 + g;
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const int y = y0 + 2 * (warp & 1) + hf;
+            if (z >= D || y >= H || x >= W)
+                continue;
+            __nv_bfloat16* o = out + (((static_cast<size_t>(bi) * D + z) * H + y) * W + x) * Cout + n0 + 2 * t;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float v0 = acc[j][2 * hf], v1 = acc[j][2 * hf + 1];
+                if (bias) {
+                    v0 += bias[n0 + 8 * j + 2 * t];
+                    v1 += bias[n0 + 8 * j + 2 * t + 1];
+                }
+                if (relu) {
+                    v0 = fmaxf(v0, 0.0f);
+                    v1 = fmaxf(v1, 0.0f);
+                }
+                *reinterpret_cast<__nv_bfloat162*>(o + 8 * j) = __floats2bfloat162_rn(v0, v1);
+            }
+        }
+    }
+
     // ------------------------------------------------------------------ weight gradient
     // dW[co][tap][ci] += sum over output voxels v of dz[v][co] * x[v + off(tap)][ci].
     // grid: x = CTAs looping over bricks, y = output-channel tile, z = input slice.
@@ -686,13 +827,18 @@ namespace {
         }
     }
 
-    int grid1d(size_t items)
+    int smCount()
     {
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        return sms > 0 ? sms : 1;
+    }
+
+    int grid1d(size_t items)
+    {
         const size_t blocks = (items + 255) / 256;
-        const size_t cap = static_cast<size_t>(sms > 0 ? sms : 1) * 8;
+        const size_t cap = static_cast<size_t>(smCount()) * 8;
         return static_cast<int>(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
     }
 } // namespace
@@ -708,6 +854,9 @@ cudaError_t conv3Configure()
         e = cudaFuncSetAttribute(conv3Kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
             static_cast<int>(conv3SmemBytes(32)));
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(conv3SmallKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            kSmallStages * kSmallStage);
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(wgradKernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
             static_cast<int>(wgradSmemBytes(16)));
     if (e == cudaSuccess)
@@ -722,7 +871,17 @@ cudaError_t launchConv3(const ConvIn& in, int B, int D, int H, int W, int Cin, c
     if (Cin % 16 || Cout % 16 || (in.ca % 16) || (in.b && in.cb % 16) || in.ca + (in.b ? in.cb : 0) != Cin)
         return cudaErrorInvalidValue;
     const int bricks = B * ((D + 7) / 8) * ((H + 7) / 8) * ((W + 7) / 8);
-    if (Cout % 32 == 0) {
+    // the small bricks where conv3Kernel would leave three quarters of the SMs without a
+    // CTA (voxel indices are ints there).  8^3 voxels, 128 to 128 channels: 56 -> 12 us;
+    // 8 x 8^3: 55 -> 36 us; 16^3, 192 to 64: 83 -> 22 us.  From a quarter of the SMs on,
+    // conv3Kernel's reuse wins: 32^3, 96 to 32 channels (64 CTAs) 43 against 45 us, 8 x 16^3
+    // 64 to 64 (128 CTAs) 30 against 51 us.
+    if (4 * bricks * (Cout / (Cout % 32 == 0 ? 32 : 16)) <= smCount()
+        && static_cast<size_t>(B) * D * H * W < (1ull << 31)) {
+        const int small = B * ((D + 1) / 2) * ((H + 3) / 4) * ((W + 7) / 8);
+        conv3SmallKernel<<<dim3(small, Cout / 16), 128, kSmallStages * kSmallStage, s>>>(in, D, H, W, Cin, w, bias,
+            Cout, relu ? 1 : 0, out);
+    } else if (Cout % 32 == 0) {
         conv3Kernel<32><<<dim3(bricks, Cout / 32), 256, conv3SmemBytes(32), s>>>(in, D, H, W, Cin, w, bias, Cout,
             relu ? 1 : 0, out);
     } else {
