@@ -318,7 +318,7 @@ void noteStops(dxmcg_world* w, const DevCounters& c)
         w->stopsPerStep = static_cast<double>(stops) / static_cast<double>(c.visits);
 }
 
-LaunchShape chooseShape(const dxmcg_world* w, const dxmcg_run_options& o, int ktrack, bool batch = false)
+LaunchShape chooseShape(const dxmcg_world* w, const dxmcg_run_options& o, int ktrack)
 {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, w->device);
@@ -326,8 +326,7 @@ LaunchShape chooseShape(const dxmcg_world* w, const dxmcg_run_options& o, int kt
     s.block = o.block_size > 0 ? o.block_size : 256;
     s.block = std::max(32, std::min(256, s.block / 32 * 32));
     // one wave of resident blocks: the kernel is persistent and pulls work from its queue
-    const int resident = batch ? transportMaxBlocksPerSMBatch(s.block, ktrack)
-                               : transportMaxBlocksPerSM(s.block, ktrack);
+    const int resident = transportMaxBlocksPerSM(s.block, ktrack);
     const int per = o.blocks_per_sm > 0 ? std::min(o.blocks_per_sm, resident) : resident;
     s.grid = std::max(1, sms) * per;
     s.interact_batch = std::min(32, std::max(0, o.interact_batch));
@@ -367,37 +366,33 @@ int deviceErrors(const DevCounters& c, const char* what)
 
 } // namespace
 
-// Several (world, beam) jobs run by one persistent launch over a shared history
-// queue; the launch (counter reset + kernel) is a CUDA graph replayed by each run.
-// Batches run in one of two ways, both captured once as a CUDA graph and replayed.
-// Per job (when the jobs average at least kPerJobHistories): each job is one launch
-// of the single-job kernel, on kBatchStreams streams, so that one job's blocks take
-// the SMs another job's tail frees.  Shared queue (smaller jobs): one launch of the
-// batch kernel over the concatenated history ranges, whose per-lane job descriptors
-// cost about 5 % per history against the single-job kernel.
-constexpr uint64_t kPerJobHistories = 1ull << 21;
-constexpr int kBatchStreams = 4;
+// Several (world, beam) jobs, each one launch of the single-job kernel, captured once as a
+// CUDA graph and replayed by each run.  Jobs that average kLargeJob histories or more
+// fill the GPU one after another, on kLargeStreams streams so that one job's blocks take
+// the SMs another job's tail frees; one world at a time keeps its voxels and tally in L2.
+// Smaller jobs would mostly be tails: they run side by side on up to kSmallStreams
+// streams, each with twice its share of the resident blocks, so that blocks of the jobs
+// still running replace those of jobs that are done.  Eight jobs of 1e5 to 2e6 histories:
+// 0.74 ms in one launch over a shared queue (whose lanes read their job's descriptor
+// from memory), 0.48 ms side by side, 0.80 ms one after another.
+constexpr uint64_t kLargeJob = 1ull << 21;
+constexpr int kLargeStreams = 4, kSmallStreams = 32;
 
 struct dxmcg_batch {
     int device = 0;
     int tracking = DXMCG_TRACK_WOODCOCK;
-    bool perJob = false;
     std::vector<DevJob> hostJobs;
     std::vector<LaunchShape> jobShapes;
     DeviceBuffer<DevCounters> jobCounters;
-    cudaStream_t side[kBatchStreams] = {};
+    std::vector<cudaStream_t> side;
+    std::vector<cudaEvent_t> join;
     cudaEvent_t fork = nullptr;
-    cudaEvent_t join[kBatchStreams] = {};
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<dxmcg_world*> worlds;
     std::vector<uint64_t> nHist;
     std::vector<double> calibration;
     std::vector<std::unique_ptr<JobBuffers>> inputs;
-    DeviceBuffer<DevJob> jobs;
-    DeviceBuffer<unsigned long long> offsets;
-    DeviceBuffer<DevCounters> counters;
-    LaunchShape shape;
     uint64_t total = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -421,12 +416,10 @@ struct dxmcg_batch {
             cudaEventDestroy(ev1);
         if (fork)
             cudaEventDestroy(fork);
-        for (int k = 0; k < kBatchStreams; ++k) {
-            if (join[k])
-                cudaEventDestroy(join[k]);
-            if (side[k])
-                cudaStreamDestroy(side[k]);
-        }
+        for (cudaEvent_t e : join)
+            cudaEventDestroy(e);
+        for (cudaStream_t t : side)
+            cudaStreamDestroy(t);
         if (stream)
             cudaStreamDestroy(stream);
     }
@@ -1205,8 +1198,8 @@ DXMCG_API int dxmcg_batch_create(int n_jobs, dxmcg_world* const* worlds, const d
     DXMCG_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     DXMCG_CUDA(cudaEventCreate(&b->ev0));
     DXMCG_CUDA(cudaEventCreate(&b->ev1));
-    std::vector<DevJob> J(n_jobs);
-    std::vector<unsigned long long> off(n_jobs + 1, 0ull);
+    std::vector<DevJob>& J = b->hostJobs;
+    J.resize(n_jobs);
     // one gather-skip decision for the whole batch, from opts[0] and the voxel words
     // of all its (distinct) worlds: they share L2 during the launch
     size_t voxelBytes = 0;
@@ -1229,40 +1222,41 @@ DXMCG_API int dxmcg_batch_create(int n_jobs, dxmcg_world* const* worlds, const d
         b->worlds.push_back(worlds[j]);
         b->nHist.push_back(n);
         b->calibration.push_back(cal);
-        off[j + 1] = off[j] + n;
+        b->total += n;
     }
     // a world's macro cells are rebuilt when a later job asks for another size
     if (tracking == DXMCG_TRACK_MACRO)
         for (int j = 0; j < n_jobs; ++j)
             if (J[j].mb != worlds[j]->macroB || J[j].mscale != worlds[j]->mscale.p)
                 return fail(DXMCG_ERR_ARGUMENT, "batch_create: jobs on one world must use one macro_cell");
-    b->total = off[n_jobs];
     DXMCG_CUDA(cudaSetDevice(b->device));
-    DXMCG_CUDA(b->jobs.alloc(n_jobs));
-    DXMCG_CUDA(b->offsets.alloc(n_jobs + 1));
-    DXMCG_CUDA(b->counters.alloc(1));
-    DXMCG_CUDA(cudaMemcpyAsync(b->jobs.p, J.data(), n_jobs * sizeof(DevJob), cudaMemcpyHostToDevice, b->stream));
-    DXMCG_CUDA(cudaMemcpyAsync(b->offsets.p, off.data(), off.size() * sizeof(unsigned long long),
-        cudaMemcpyHostToDevice, b->stream));
-    DXMCG_CUDA(cudaStreamSynchronize(b->stream));
-    // the occupancy query also loads the kernel, so the later graph capture loads nothing
-    // Woodcock jobs run the two-region instance when any of them has a box; in it, a
-    // job without one (boxOn 0) never leaves the first region
     for (int j = 0; j < n_jobs; ++j)
         if (kernelTracking(J[j]) == kTrackWoodcockBox)
             b->tracking = kTrackWoodcockBox;
-    b->shape = chooseShape(worlds[0], opts[0], b->tracking, true);
-    b->perJob = b->total >= kPerJobHistories * static_cast<uint64_t>(n_jobs);
-    if (b->perJob) {
-        b->hostJobs = J;
-        for (int j = 0; j < n_jobs; ++j)
-            b->jobShapes.push_back(chooseShape(worlds[j], opts[j], kernelTracking(J[j])));
-        DXMCG_CUDA(b->jobCounters.alloc(n_jobs));
-        DXMCG_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-        for (int k = 0; k < kBatchStreams; ++k) {
-            DXMCG_CUDA(cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking));
-            DXMCG_CUDA(cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming));
+    // the occupancy query also loads the kernel, so the later graph capture loads nothing
+    const bool large = b->total >= kLargeJob * static_cast<uint64_t>(n_jobs);
+    const int streams = std::min(n_jobs, large ? kLargeStreams : kSmallStreams);
+    for (int j = 0; j < n_jobs; ++j) {
+        LaunchShape sh = chooseShape(worlds[j], opts[j], kernelTracking(J[j]));
+        if (!large) {
+            // twice the job's share of the blocks that run at a time, 128 histories a block
+            // at least
+            const double share = 2.0 * n_jobs / streams * static_cast<double>(b->nHist[j])
+                / static_cast<double>(std::max<uint64_t>(b->total, 1));
+            const double blocks = std::min(std::ceil(sh.grid * share), std::ceil(b->nHist[j] / 128.0));
+            sh.grid = static_cast<int>(std::max(1.0, std::min<double>(sh.grid, blocks)));
         }
+        b->jobShapes.push_back(sh);
+    }
+    DXMCG_CUDA(b->jobCounters.alloc(n_jobs));
+    DXMCG_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+    for (int k = 0; k < streams; ++k) {
+        cudaStream_t t = nullptr;
+        DXMCG_CUDA(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
+        b->side.push_back(t);
+        cudaEvent_t ev = nullptr;
+        DXMCG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        b->join.push_back(ev);
     }
     *out = b.release();
     return DXMCG_OK;
@@ -1293,27 +1287,20 @@ DXMCG_API int dxmcg_batch_run(dxmcg_batch* b, dxmcg_stats* stats)
     const int nJobs = static_cast<int>(b->worlds.size());
     if (!b->exec) {
         DXMCG_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = cudaSuccess;
-        if (b->perJob) {
-            // fork to the side streams, one launch per job round-robin, join
-            e = cudaMemsetAsync(b->jobCounters.p, 0, nJobs * sizeof(DevCounters), b->stream);
+        // fork to the side streams, one launch per job round-robin, join
+        const int streams = static_cast<int>(b->side.size());
+        cudaError_t e = cudaMemsetAsync(b->jobCounters.p, 0, nJobs * sizeof(DevCounters), b->stream);
+        if (e == cudaSuccess)
+            e = cudaEventRecord(b->fork, b->stream);
+        for (int k = 0; k < streams && e == cudaSuccess; ++k)
+            e = cudaStreamWaitEvent(b->side[k], b->fork, 0);
+        for (int j = 0; j < nJobs && e == cudaSuccess; ++j)
+            e = launchTransport(b->hostJobs[j], b->nHist[j], b->jobCounters.p + j, b->jobShapes[j],
+                b->side[j % streams]);
+        for (int k = 0; k < streams && e == cudaSuccess; ++k) {
+            e = cudaEventRecord(b->join[k], b->side[k]);
             if (e == cudaSuccess)
-                e = cudaEventRecord(b->fork, b->stream);
-            for (int k = 0; k < kBatchStreams && e == cudaSuccess; ++k)
-                e = cudaStreamWaitEvent(b->side[k], b->fork, 0);
-            for (int j = 0; j < nJobs && e == cudaSuccess; ++j)
-                e = launchTransport(b->hostJobs[j], b->nHist[j], b->jobCounters.p + j, b->jobShapes[j],
-                    b->side[j % kBatchStreams]);
-            for (int k = 0; k < kBatchStreams && e == cudaSuccess; ++k) {
-                e = cudaEventRecord(b->join[k], b->side[k]);
-                if (e == cudaSuccess)
-                    e = cudaStreamWaitEvent(b->stream, b->join[k], 0);
-            }
-        } else {
-            e = cudaMemsetAsync(b->counters.p, 0, sizeof(DevCounters), b->stream);
-            if (e == cudaSuccess)
-                e = launchTransportBatch(b->tracking, b->jobs.p, b->offsets.p, nJobs, b->total, b->counters.p,
-                    b->shape, b->stream);
+                e = cudaStreamWaitEvent(b->stream, b->join[k], 0);
         }
         cudaGraph_t g = nullptr;
         const cudaError_t ee = cudaStreamEndCapture(b->stream, &g);
@@ -1329,19 +1316,14 @@ DXMCG_API int dxmcg_batch_run(dxmcg_batch* b, dxmcg_stats* stats)
     DXMCG_CUDA(cudaGraphLaunch(b->exec, b->stream));
     DXMCG_CUDA(cudaEventRecord(b->ev1, b->stream));
     DevCounters c {};
-    if (b->perJob) {
-        std::vector<DevCounters> each(nJobs);
-        DXMCG_CUDA(cudaMemcpyAsync(each.data(), b->jobCounters.p, nJobs * sizeof(DevCounters),
-            cudaMemcpyDeviceToHost, b->stream));
-        DXMCG_CUDA(cudaStreamSynchronize(b->stream));
-        for (int j = 0; j < nJobs; ++j) {
-            addCounters(c, each[j]);
-            if (b->tracking == DXMCG_TRACK_WOODCOCK || b->tracking == kTrackWoodcockBox)
-                noteStops(b->worlds[j], each[j]);
-        }
-    } else {
-        DXMCG_CUDA(cudaMemcpyAsync(&c, b->counters.p, sizeof(c), cudaMemcpyDeviceToHost, b->stream));
-        DXMCG_CUDA(cudaStreamSynchronize(b->stream));
+    std::vector<DevCounters> each(nJobs);
+    DXMCG_CUDA(cudaMemcpyAsync(each.data(), b->jobCounters.p, nJobs * sizeof(DevCounters), cudaMemcpyDeviceToHost,
+        b->stream));
+    DXMCG_CUDA(cudaStreamSynchronize(b->stream));
+    for (int j = 0; j < nJobs; ++j) {
+        addCounters(c, each[j]);
+        if (b->tracking == DXMCG_TRACK_WOODCOCK || b->tracking == kTrackWoodcockBox)
+            noteStops(b->worlds[j], each[j]);
     }
     float ms = 0.0f;
     DXMCG_CUDA(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
@@ -1355,13 +1337,10 @@ DXMCG_API int dxmcg_batch_run(dxmcg_batch* b, dxmcg_stats* stats)
         stats->dose_scale = kKeVToMilliGrayGram / b->worlds[0]->voxelVolume;
         stats->calibration = b->calibration[0];
         const bool wood = b->tracking == DXMCG_TRACK_WOODCOCK || b->tracking == kTrackWoodcockBox;
-        stats->woodcock_steps = wood ? (b->perJob ? b->jobShapes[0].woodcock_steps : b->shape.woodcock_steps) : 0;
+        stats->woodcock_steps = wood ? b->jobShapes[0].woodcock_steps : 0;
         stats->two_region = 0;
-        if (b->perJob)
-            for (const auto& hj : b->hostJobs)
-                stats->two_region |= hj.boxOn;
-        else
-            stats->two_region = b->tracking == kTrackWoodcockBox ? 1 : 0;
+        for (const auto& hj : b->hostJobs)
+            stats->two_region |= hj.boxOn;
     }
     return deviceErrors(c, "batch_run");
 }

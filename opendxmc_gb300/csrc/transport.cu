@@ -179,15 +179,10 @@ namespace {
         return rng.u() * muc < mu;
     }
 
-    // MULTI: one queue over the concatenated history ranges of nJobs jobs (offsets[j]
-    // is the first global history of job j, offsets[nJobs] the total); each lane
-    // reads its job's descriptor from `jobs`.  Otherwise J0 is the only job.
-    template <int TRACKING, bool PACKED, bool MULTI>
-    __global__ void __launch_bounds__(256) transportKernel(const DevJob J0, const DevJob* __restrict__ jobs,
-        const unsigned long long* __restrict__ offsets, int nJobs, unsigned long long h_end,
+    template <int TRACKING, bool PACKED>
+    __global__ void __launch_bounds__(256) transportKernel(const DevJob J, unsigned long long h_end,
         DevCounters* __restrict__ ctr, int refillBatch, int interactBatch, int)
     {
-        int jid = 0;
         // event counters per warp (no block-wide barrier: warps finish independently)
         __shared__ unsigned long long sCountAll[256 / 32][cNum];
         const unsigned lane = threadIdx.x & 31u;
@@ -236,24 +231,11 @@ namespace {
                 const bool start = st == kDead && rank < avail;
                 bool entered = false;
                 if (start) {
-                    unsigned long long h = poolNext + rank;
-                    if (MULTI) { // the queue spans all jobs: find this history's job
-                        int lo = 0, hi = nJobs;
-                        while (hi - lo > 1) {
-                            const int mid = (lo + hi) >> 1;
-                            if (__ldg(offsets + mid) <= h)
-                                lo = mid;
-                            else
-                                hi = mid;
-                        }
-                        jid = lo;
-                        h -= __ldg(offsets + lo);
-                    }
-                    const DevJob& Jr = MULTI ? jobs[jid] : J0;
-                    rng.init(Jr.key, h);
-                    sampleSource(Jr, h, ph, rng);
+                    const unsigned long long h = poolNext + rank;
+                    rng.init(J.key, h);
+                    sampleSource(J, h, ph, rng);
                     sum[kSumSource].add(ph.w * ph.E);
-                    entered = enterGrid(Jr, ph);
+                    entered = enterGrid(J, ph);
                     if (entered) {
                         st = kStepping;
                         steps = 0;
@@ -261,11 +243,11 @@ namespace {
                         if (TRACKING == DXMCG_TRACK_SIDDON)
                             gridPos(ph.E, ec.ie, ec.fe);
                         else
-                            ec.set(Jr, ph.E);
+                            ec.set(J, ph.E);
                         if (TRACKING == DXMCG_TRACK_MACRO) {
-                            cx = min(static_cast<int>(ph.px / Jr.cellL[0]), Jr.mc[0] - 1);
-                            cy = min(static_cast<int>(ph.py / Jr.cellL[1]), Jr.mc[1] - 1);
-                            cz = min(static_cast<int>(ph.pz / Jr.cellL[2]), Jr.mc[2] - 1);
+                            cx = min(static_cast<int>(ph.px / J.cellL[0]), J.mc[0] - 1);
+                            cy = min(static_cast<int>(ph.py / J.cellL[1]), J.mc[1] - 1);
+                            cz = min(static_cast<int>(ph.pz / J.cellL[2]), J.mc[2] - 1);
                         }
                     } else {
                         sum[kSumEscaped].add(ph.w * ph.E);
@@ -279,9 +261,6 @@ namespace {
                     atomicAdd(&sCount[cMissed], static_cast<unsigned long long>(__popc(mStart & ~mIn)));
                 }
             }
-
-            // the lane's job, after the refill may have changed it
-            const DevJob& J = MULTI ? jobs[jid] : J0;
 
             // ---- interact
             const int nPark = __popc(parked);
@@ -449,49 +428,44 @@ namespace {
 
 namespace {
     // kernel instance for a tracking mode on the packed (world) or unpacked
-    // (caller-owned arrays) voxel layout, single job or a batch of jobs, with n_mats
-    // materials; nullptr where no instance exists
-    TransportFn kernelFor(int tracking, bool packed, bool multi, int n_mats)
+    // (caller-owned arrays) voxel layout with n_mats materials; nullptr where no instance
+    // exists
+    TransportFn kernelFor(int tracking, bool packed, int n_mats)
     {
-        if (tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox)
-            return woodcockKernelFor(packed, tracking == kTrackWoodcockBox, multi, n_mats);
-        const bool siddon = tracking == DXMCG_TRACK_SIDDON;
-        if (!siddon && (tracking != DXMCG_TRACK_MACRO || !packed))
-            return nullptr;
-        if (multi)
-            return siddon ? transportKernel<DXMCG_TRACK_SIDDON, true, true>
-                          : transportKernel<DXMCG_TRACK_MACRO, true, true>;
-        if (!packed)
-            return transportKernel<DXMCG_TRACK_SIDDON, false, false>;
-        return siddon ? transportKernel<DXMCG_TRACK_SIDDON, true, false>
-                      : transportKernel<DXMCG_TRACK_MACRO, true, false>;
+        switch (tracking) {
+        case DXMCG_TRACK_WOODCOCK: return woodcockKernelFor(packed, false, n_mats);
+        case kTrackWoodcockBox: return woodcockKernelFor(packed, true, n_mats);
+        case DXMCG_TRACK_SIDDON:
+            return packed ? transportKernel<DXMCG_TRACK_SIDDON, true> : transportKernel<DXMCG_TRACK_SIDDON, false>;
+        case DXMCG_TRACK_MACRO: return packed ? transportKernel<DXMCG_TRACK_MACRO, true> : nullptr;
+        default: return nullptr;
+        }
     }
 
-    cudaError_t launchWith(int tracking, bool packed, const DevJob& job, const DevJob* jobs,
-        const unsigned long long* offsets, int nJobs, unsigned long long h_end, DevCounters* ctr, LaunchShape shape,
+    cudaError_t launch(bool packed, const DevJob& job, unsigned long long h_end, DevCounters* ctr, LaunchShape shape,
         cudaStream_t s)
     {
-        const bool multi = jobs != nullptr;
+        const int tracking = kernelTracking(job);
         const bool woodcock = tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox;
-        const TransportFn fn = kernelFor(tracking, packed, multi, job.n_mats);
+        const TransportFn fn = kernelFor(tracking, packed, job.n_mats);
         if (!fn)
             return cudaErrorInvalidValue;
         const int refill = shape.refill_batch > 0 ? shape.refill_batch : (woodcock ? kWoodcockRefillBatch : 8);
         const int interact
             = shape.interact_batch > 0 ? shape.interact_batch : (woodcock ? kWoodcockInteractBatch : 8);
         const int wsteps = shape.woodcock_steps > 0 ? shape.woodcock_steps : 8;
-        const size_t smem = woodcock ? woodcockSharedBytes(shape.block, multi, job.n_mats) : 0;
-        fn<<<shape.grid, shape.block, smem, s>>>(job, jobs, offsets, nJobs, h_end, ctr, refill, interact, wsteps);
+        const size_t smem = woodcock ? woodcockSharedBytes(shape.block, job.n_mats) : 0;
+        fn<<<shape.grid, shape.block, smem, s>>>(job, h_end, ctr, refill, interact, wsteps);
         return cudaGetLastError();
     }
 
     // resident blocks per SM of the instance that needs most shared memory
-    int residentBlocks(int tracking, bool packed, bool multi, int block)
+    int residentBlocks(int tracking, bool packed, int block)
     {
         int n = 0;
         const bool woodcock = tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox;
-        const TransportFn fn = kernelFor(tracking, packed, multi, kSharedTableMaterials);
-        const size_t smem = woodcock ? woodcockSharedBytes(block, multi, kSharedTableMaterials) : 0;
+        const TransportFn fn = kernelFor(tracking, packed, kSharedTableMaterials);
+        const size_t smem = woodcock ? woodcockSharedBytes(block, kSharedTableMaterials) : 0;
         if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) != cudaSuccess)
             return 1;
         return n > 0 ? n : 1;
@@ -501,34 +475,23 @@ namespace {
 cudaError_t launchTransport(const DevJob& job, unsigned long long h_end, DevCounters* ctr, LaunchShape shape,
     cudaStream_t s)
 {
-    return launchWith(kernelTracking(job), true, job, nullptr, nullptr, 1, h_end, ctr, shape, s);
+    return launch(true, job, h_end, ctr, shape, s);
 }
 
 cudaError_t launchTransportUnpacked(const DevJob& job, unsigned long long h_end, DevCounters* ctr,
     LaunchShape shape, cudaStream_t s)
 {
-    return launchWith(kernelTracking(job), false, job, nullptr, nullptr, 1, h_end, ctr, shape, s);
+    return launch(false, job, h_end, ctr, shape, s);
 }
 
-cudaError_t launchTransportBatch(int tracking, const DevJob* jobs, const unsigned long long* offsets, int nJobs,
-    unsigned long long h_end, DevCounters* ctr, LaunchShape shape, cudaStream_t s)
-{
-    if (!jobs || !offsets || nJobs < 1)
-        return cudaErrorInvalidValue;
-    const DevJob unused {};
-    return launchWith(tracking, true, unused, jobs, offsets, nJobs, h_end, ctr, shape, s);
-}
+int transportMaxBlocksPerSMUnpacked(int block, int tracking) { return residentBlocks(tracking, false, block); }
 
-int transportMaxBlocksPerSMBatch(int block, int tracking) { return residentBlocks(tracking, true, true, block); }
-
-int transportMaxBlocksPerSMUnpacked(int block, int tracking) { return residentBlocks(tracking, false, false, block); }
-
-int transportMaxBlocksPerSM(int block, int tracking) { return residentBlocks(tracking, true, false, block); }
+int transportMaxBlocksPerSM(int block, int tracking) { return residentBlocks(tracking, true, block); }
 
 int transportRegistersPerThread(int tracking)
 {
     cudaFuncAttributes a {};
-    const TransportFn fn = kernelFor(tracking, true, false, kSharedTableMaterials);
+    const TransportFn fn = kernelFor(tracking, true, kSharedTableMaterials);
     return fn && cudaFuncGetAttributes(&a, fn) == cudaSuccess ? a.numRegs : -1;
 }
 

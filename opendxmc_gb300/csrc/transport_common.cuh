@@ -89,14 +89,12 @@ namespace {
 
 } // namespace
 
-using TransportFn = void (*)(const DevJob, const DevJob*, const unsigned long long*, int, unsigned long long,
-    DevCounters*, int, int, int);
+using TransportFn = void (*)(const DevJob, unsigned long long, DevCounters*, int, int, int);
 
-// woodcock.cu: the Woodcock kernel's instance for a voxel layout, one region or two, a
-// batch or a single job of n_mats materials; its dynamic shared memory at a block size;
-// its default batch sizes
-TransportFn woodcockKernelFor(bool packed, bool box, bool multi, int n_mats);
-size_t woodcockSharedBytes(int block, bool multi, int n_mats);
+// woodcock.cu: the Woodcock kernel's instance for a voxel layout, one region or two and
+// n_mats materials; its dynamic shared memory at a block size; its default batch sizes
+TransportFn woodcockKernelFor(bool packed, bool box, int n_mats);
+size_t woodcockSharedBytes(int block, int n_mats);
 extern const int kWoodcockRefillBatch, kWoodcockInteractBatch;
 // materials whose attenuation tables a block holds in shared memory: with the photon
 // pools of 8 warps, as many as fit the 48 KB a launch may use without opting in

@@ -198,44 +198,33 @@ namespace {
     // spreads a short run over all warps: 1e5 histories 0.203 -> 0.115 ms.
     constexpr int kSlots = 64;
 
-    template <bool MULTI>
-    __host__ __device__ constexpr size_t poolBytes()
-    {
-        return kSlots * 64 + 6 * 32 * sizeof(float) + 10 * sizeof(unsigned long long) + (MULTI ? kSlots * 4 : 0);
-    }
+    constexpr size_t kPoolBytes = kSlots * 64 + 6 * 32 * sizeof(float) + 10 * sizeof(unsigned long long);
 
-    // MULTI: one queue over the concatenated history ranges of nJobs jobs (offsets[j]
-    // is the first global history of job j, offsets[nJobs] the total); each lane
-    // reads its job's descriptor from `jobs`.  Otherwise J0 is the only job.
-    // TAB: the block keeps J0's attenuation tables in shared memory, behind the pools.
-    template <bool PACKED, bool BOX, bool MULTI, bool TAB>
-    __global__ void __launch_bounds__(256, 4) woodcockKernel(const DevJob J0, const DevJob* __restrict__ jobs,
-        const unsigned long long* __restrict__ offsets, int nJobs, unsigned long long h_end,
+    // TAB: the block keeps the job's attenuation tables in shared memory, behind the pools.
+    template <bool PACKED, bool BOX, bool TAB>
+    __global__ void __launch_bounds__(256, 4) woodcockKernel(const DevJob J, unsigned long long h_end,
         DevCounters* __restrict__ ctr, int refillBatch, int interactBatch, int woodcockSteps)
     {
         extern __shared__ __align__(16) unsigned char sRaw[];
         const int lane = static_cast<int>(threadIdx.x & 31u);
         const unsigned ltMask = (1u << lane) - 1u;
         const int warps = static_cast<int>(blockDim.x >> 5);
-        unsigned char* const base = sRaw + (threadIdx.x >> 5) * poolBytes<MULTI>();
+        unsigned char* const base = sRaw + (threadIdx.x >> 5) * kPoolBytes;
         // slot state: A position, energy; B direction, weight; C generator; D in flight:
         // {packed, fe, majorant, its inverse}, parked: {packed, fe, voxel, material}
         float4* const A = reinterpret_cast<float4*>(base);
         float* const sums = reinterpret_cast<float*>(A + 4 * kSlots) + lane; // [2K] sum, [2K + 1] compensation, x 32
         unsigned long long* const counts = reinterpret_cast<unsigned long long*>(sums - lane + 6 * 32);
-        int* const jids = reinterpret_cast<int*>(counts + 10);
-        float* const sTot = reinterpret_cast<float*>(sRaw + warps * poolBytes<MULTI>());
+        float* const sTot = reinterpret_cast<float*>(sRaw + warps * kPoolBytes);
 
 #pragma unroll
         for (int k = 0; k < 6; ++k)
             sums[32 * k] = 0.0f;
         if (lane < 10)
             counts[lane] = 0ull;
-        if (MULTI)
-            jids[lane] = jids[lane + 32] = 0;
         if (TAB) {
-            for (int i = static_cast<int>(threadIdx.x); i < J0.n_mats * kTableNE; i += static_cast<int>(blockDim.x))
-                sTot[i] = __ldg(&J0.tot[i].x);
+            for (int i = static_cast<int>(threadIdx.x); i < J.n_mats * kTableNE; i += static_cast<int>(blockDim.x))
+                sTot[i] = __ldg(&J.tot[i].x);
             __syncthreads();
         }
 
@@ -256,16 +245,13 @@ namespace {
         const auto count = [&](BlockCount c, unsigned mask) { // lane 0 only
             counts[c] += static_cast<unsigned long long>(__popc(mask));
         };
-        const auto store = [&](int slot, const Photon& ph, const Rng& rng, unsigned packed, float fe, float z, float w,
-                               int jid) {
+        const auto store = [&](int slot, const Photon& ph, const Rng& rng, unsigned packed, float fe, float z, float w) {
             float4* const p = A + slot;
             p[0] = make_float4(ph.px, ph.py, ph.pz, ph.E);
             p[kSlots] = make_float4(ph.dx, ph.dy, ph.dz, ph.w);
             p[2 * kSlots] = make_float4(__uint_as_float(rng.s0), __uint_as_float(rng.s1), __uint_as_float(rng.s2),
                 __uint_as_float(rng.s3));
             p[3 * kSlots] = make_float4(__uint_as_float(packed), fe, z, w);
-            if (MULTI)
-                jids[slot] = jid;
         };
 
         for (;;) {
@@ -295,27 +281,13 @@ namespace {
                 const unsigned long long rank = static_cast<unsigned long long>(lane);
                 const unsigned long long n = min(static_cast<unsigned long long>(nFree), avail + avail2);
                 const bool start = rank < n;
-                unsigned long long h = rank < avail ? next + rank : base2 + (rank - avail);
+                const unsigned long long h = rank < avail ? next + rank : base2 + (rank - avail);
                 Photon ph;
                 Rng rng;
                 EnergyCache ec { 0, 0.0f, 0.0f, 0.0f };
                 unsigned packed = kPackFresh;
-                int jid = 0;
                 bool entered = false;
                 if (start) {
-                    if (MULTI) { // the queue spans all jobs: find this history's job
-                        int lo = 0, hi = nJobs;
-                        while (hi - lo > 1) {
-                            const int mid = (lo + hi) >> 1;
-                            if (__ldg(offsets + mid) <= h)
-                                lo = mid;
-                            else
-                                hi = mid;
-                        }
-                        jid = lo;
-                        h -= __ldg(offsets + lo);
-                    }
-                    const DevJob& J = MULTI ? jobs[jid] : J0;
                     rng.init(J.key, h);
                     sampleSource(J, h, ph, rng);
                     addSum(kSumSource, ph.w * ph.E);
@@ -343,7 +315,7 @@ namespace {
                 }
                 const unsigned mIn = __ballot_sync(kFull, entered);
                 if (entered)
-                    store(nFly + __popc(mIn & ltMask), ph, rng, packed, ec.fe, ec.mmax, ec.invMmax, jid);
+                    store(nFly + __popc(mIn & ltMask), ph, rng, packed, ec.fe, ec.mmax, ec.invMmax);
                 nFly += __popc(mIn);
                 if (lane == 0) {
                     counts[cHist] += n;
@@ -355,10 +327,8 @@ namespace {
                 const bool has = lane < n;
                 const float4* const src = A + (kSlots - nPark + (has ? lane : 0));
                 const float4 a = src[0], b = src[kSlots], c = src[2 * kSlots], d = src[3 * kSlots];
-                const int jid = MULTI ? jids[kSlots - nPark + (has ? lane : 0)] : 0;
                 nPark -= n;
                 __syncwarp(); // before the pushes overwrite what other lanes read
-                const DevJob& J = MULTI ? jobs[jid] : J0;
                 Photon ph { a.x, a.y, a.z, b.x, b.y, b.z, a.w, b.w };
                 Rng rng { __float_as_uint(c.x), __float_as_uint(c.y), __float_as_uint(c.z), __float_as_uint(c.w) };
                 const unsigned packed = __float_as_uint(d.x);
@@ -435,7 +405,7 @@ namespace {
                 if (alive)
                     store(nFly + __popc(mAlive & ltMask), ph, rng,
                         static_cast<unsigned>(ec.ie) | (outer ? kPackOuter : 0u) | (packed >> kPackSteps << kPackSteps),
-                        ec.fe, ec.mmax, ec.invMmax, jid);
+                        ec.fe, ec.mmax, ec.invMmax);
                 nFly += __popc(mAlive);
                 const unsigned mFirst = __ballot_sync(kFull, has && (packed & kPackFresh) != 0u);
                 const unsigned mP = __ballot_sync(kFull, photo);
@@ -465,9 +435,7 @@ namespace {
                 nFly -= n;
                 const float4* const src = A + (nFly + (has ? lane : 0));
                 const float4 a = src[0], b = src[kSlots], c = src[2 * kSlots], d = src[3 * kSlots];
-                const int jid = MULTI ? jids[nFly + (has ? lane : 0)] : 0;
                 __syncwarp(); // before the pushes overwrite what other lanes read
-                const DevJob& J = MULTI ? jobs[jid] : J0;
                 Photon ph { a.x, a.y, a.z, b.x, b.y, b.z, a.w, b.w };
                 Rng rng { __float_as_uint(c.x), __float_as_uint(c.y), __float_as_uint(c.z), __float_as_uint(c.w) };
                 unsigned packed = __float_as_uint(d.x);
@@ -510,7 +478,7 @@ namespace {
                 const unsigned mOn = __ballot_sync(kFull, on), mReal = __ballot_sync(kFull, real);
                 if (on || real)
                     store(real ? kSlots - 1 - nPark - __popc(mReal & ltMask) : nFly + __popc(mOn & ltMask), ph, rng,
-                        packed, ec.fe, real ? __uint_as_float(v) : ec.mmax, real ? __int_as_float(m) : ec.invMmax, jid);
+                        packed, ec.fe, real ? __uint_as_float(v) : ec.mmax, real ? __int_as_float(m) : ec.invMmax);
                 nFly += __popc(mOn);
                 nPark += __popc(mReal);
             } else {
@@ -543,33 +511,31 @@ namespace {
     }
 
     template <bool PACKED, bool BOX>
-    TransportFn single(bool tab)
+    TransportFn instance(bool tab)
     {
-        return tab ? woodcockKernel<PACKED, BOX, false, true> : woodcockKernel<PACKED, BOX, false, false>;
+        return tab ? woodcockKernel<PACKED, BOX, true> : woodcockKernel<PACKED, BOX, false>;
     }
 } // namespace
 
 // lanes a warp wants of a kind before it runs that kind's phase
 extern const int kWoodcockRefillBatch = 28, kWoodcockInteractBatch = 28;
 
-TransportFn woodcockKernelFor(bool packed, bool box, bool multi, int n_mats)
+TransportFn woodcockKernelFor(bool packed, bool box, int n_mats)
 {
     const bool tab = n_mats <= kSharedTableMaterials;
-    if (multi)
-        return box ? woodcockKernel<true, true, true, false> : woodcockKernel<true, false, true, false>;
     if (packed)
-        return box ? single<true, true>(tab) : single<true, false>(tab);
-    return box ? single<false, true>(tab) : single<false, false>(tab);
+        return box ? instance<true, true>(tab) : instance<true, false>(tab);
+    return box ? instance<false, true>(tab) : instance<false, false>(tab);
 }
 
-size_t woodcockSharedBytes(int block, bool multi, int n_mats)
+size_t woodcockSharedBytes(int block, int n_mats)
 {
-    const size_t pools = static_cast<size_t>(block / 32) * (multi ? poolBytes<true>() : poolBytes<false>());
-    const bool tab = !multi && n_mats <= kSharedTableMaterials;
+    const size_t pools = static_cast<size_t>(block / 32) * kPoolBytes;
+    const bool tab = n_mats <= kSharedTableMaterials;
     return pools + (tab ? static_cast<size_t>(n_mats) * kTableNE * sizeof(float) : 0);
 }
 
 // the tables and pools of 8 warps fit the 48 KB a launch may use without opting in
-static_assert(8 * poolBytes<false>() + kSharedTableMaterials * kTableNE * sizeof(float) <= 48 * 1024, "shared memory");
+static_assert(8 * kPoolBytes + kSharedTableMaterials * kTableNE * sizeof(float) <= 48 * 1024, "shared memory");
 
 } // namespace dxmcg
