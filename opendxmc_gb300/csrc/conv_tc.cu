@@ -10,10 +10,10 @@
 //   * the slice's weights of all 27 taps, the three z-taps of each in-plane tap
 //     q = 3 (dy + 1) + (dx + 1) stacked along N: row n = (1 - dz) * NT + co of the
 //     B operand of q, half h, at q * 3*NT*32 + h * 3*NT*16 + n * 16,
-// in the tensor cores' no-swizzle K-major layout, so that the A operand of a tap is
-// the halo seen through a descriptor: row r = 8 y + x of halo plane hz reads halo
-// voxel (hz, y + dy + 1, x + dx + 1): 8 consecutive x are one core matrix,
-// consecutive y are 160 bytes apart (SBO), the channel halves one plane apart (LBO).
+// (no swizzle, K-major), so that the A operand of a tap is the halo seen through a
+// descriptor: row r = 8 y + x of halo plane hz reads halo voxel (hz, y + dy + 1,
+// x + dx + 1): 8 consecutive x are 256 bytes, consecutive y 320 bytes apart (SBO); the
+// swizzle goes by the address, whichever voxel the tap starts at.
 // Output slice o accumulates in TMEM columns [o NT, o NT + NT).  One M = 128 MMA per
 // (halo plane hz, in-plane tap q) multiplies plane hz by the stacked weights of q and
 // writes from column (hz - 2) NT: its block n / NT = 1 - dz lands on output slice
@@ -139,8 +139,8 @@ namespace {
         static constexpr int ZT = NT == 64 ? 4 : 8;          // output z-slices per brick
         static constexpr int HZ = ZT + 2, HY = 18, HX = 10;  // halo extent
         static constexpr int kVox = HZ * HY * HX;
-        static constexpr uint32_t kPlane = kVox * 16;        // one 8-channel half of the halo
-        static constexpr uint32_t kHalo = 2 * kPlane;        // one halo buffer (two in the pipeline)
+        static constexpr uint32_t kHalo = kVox * 32;         // one halo buffer (two in the pipeline)
+        static_assert(kHalo % 256 == 0, "the swizzle pattern repeats every 256 bytes");
         static constexpr uint32_t kTapBytes = NT * 32;
         static constexpr uint32_t kStackBytes = 3 * kTapBytes; // the z-taps of one in-plane tap
         static constexpr uint32_t kWeights = 27 * kTapBytes;  // one 16-channel input slice
@@ -153,12 +153,12 @@ namespace {
         // dynamic shared memory: one halo buffer per pipeline stage (two or three), then the
         // weights -- every slice's when they fit (resident), else one buffer per stage
         static constexpr int kMaxStages = 3;
-        static constexpr uint32_t kMaxSmem = 227 * 1024 - 256;
+        static constexpr uint32_t kMaxSmem = 227 * 1024 - 256; // static shared memory beside it
         static constexpr uint32_t smemFor(int nSlices, bool resident, int stages)
         {
-            return stages * kHalo + (resident ? nSlices : stages) * kWeights;
+            return 256 + stages * kHalo + (resident ? nSlices : stages) * kWeights; // 256: alignment
         }
-        static_assert(2 * kHalo + 2 * kWeights <= kMaxSmem, "pipeline buffers exceed shared memory");
+        static_assert(256 + 2 * kHalo + 2 * kWeights <= kMaxSmem, "pipeline buffers exceed shared memory");
     };
 
     struct TcTile {
@@ -178,36 +178,46 @@ namespace {
         return p;
     }
 
+    // byte offset of the 16-byte half h of halo voxel v
+    __device__ __forceinline__ uint32_t haloOffset(int v, int h)
+    {
+        return static_cast<uint32_t>(v * 32 + ((h ^ (v >> 2 & 1)) << 4));
+    }
+
     // mapA / mapB: 5-D tensor maps (C, W, H, D, B) of the full-resolution inputs a and b
-    // with a box of (8, 10, 18, ZT + 2, 1), used when useTma: the box of channel half h
-    // lands as halo plane h.  Slices of an upsampled input (halfA) are expanded by the
-    // producer threads from the low-resolution voxels; without tensor maps the halo is
-    // gathered with cp.async.
+    // with a box of (16, 10, 18, ZT + 2, 1), used when useTma.  Slices of
+    // an upsampled input (halfA) are expanded by the producer threads from the
+    // low-resolution voxels; without tensor maps the halo is gathered with cp.async.
     //
     // One persistent CTA per SM (and output-channel tile blockIdx.y) works through its
     // items -- (brick, input slice) pairs, bricks blockIdx.x, blockIdx.x + gridDim.x, ...
     // in order, each brick's slices in order -- with warp-specialised roles that hand
     // work over through mbarriers only, never a CTA barrier:
-    //   * warp 0 (one thread) issues each item's MMAs into its brick's accumulator set
-    //     (the two sets alternate between bricks), commits them to empty[stage] and,
-    //     after a brick's last slice, to accFull[set].  An issuing thread stalls while
-    //     the tensor pipe's queue is full, so no other role waits on it;
-    //   * warps 1-3 (producers) stage item i into stage i mod S once the MMAs of the
+    //   * warp 0 waits as a whole and one elected lane issues each item's MMAs into its
+    //     brick's accumulator set (the two sets alternate between bricks) and commits them
+    //     to empty[stage] and, after a brick's last slice, to accFull[set].  An issuing thread
+    //     stalls while the tensor pipe's queue is full, so no other role waits on it.  Under
+    //     `threadIdx.x == 0` the issue itself took 72 cycles an MMA, elected 50 to 55, of
+    //     the 45 the tensor pipe needs: 16 to 16 channels on 200 x 264 x 232 voxels 272 ->
+    //     213 us without an output to store, 247 with one, and 220 with whole-sector halos;
+    //   * warps 1-7 (producers) stage item i into stage i mod S once the MMAs of the
     //     item that used it before released it (S = 2 or 3 stages, a launch parameter):
-    //     the halo by TMA (completing on tmaFull) or by their own
-    //     copies / upsampling expansion, and the slice's weights unless every slice's
-    //     weights stay resident; then they arrive on full[stage];
-    //   * warps 4-7 (one TMEM lane quarter each) wait for accFull, read the brick's sums
+    //     the halo by TMA (completing on tmaFull) or by their own copies / upsampling
+    //     expansion, and the slice's weights unless every slice's weights stay resident;
+    //     then they arrive on full[stage].  The expansion is what they are many for: 48 (32
+    //     upsampled) to 16 channels took 924 us with three such warps, 580 with seven;
+    //   * warps 8-11 (one TMEM lane quarter each) wait for accFull, read the brick's sums
     //     back (bias, ReLU, bf16 store), zero them and arrive on accEmpty[set].
     // Every wait is bounded; a role that gives up raises the CTA's abort flag, the
     // others leave at their next wait, and what is in flight (TMA, MMAs, copies) is
     // awaited before the shared and tensor memory are given back.
-    constexpr int kProducers = 96;   // warps 1-3
-    constexpr int kEpilogue = 128;   // warps 4-7
+    constexpr int kProducers = 224;  // warps 1-7
+    constexpr int kEpilogue = 128;   // warps 8-11
+    constexpr int kConvThreads = 384;
     constexpr uint32_t kPolls = 1u << 24;
 
     template <int NT>
-    __global__ void __launch_bounds__(256, 1) conv3TcKernel(const nn::ConvIn in, int D, int H, int W, int Cin,
+    __global__ void __launch_bounds__(kConvThreads, 1) conv3TcKernel(const nn::ConvIn in, int D, int H, int W, int Cin,
         const __nv_bfloat16* __restrict__ wgt, const float* __restrict__ bias, int Cout, int relu,
         __nv_bfloat16* __restrict__ out, const __grid_constant__ CUtensorMap mapA,
         const __grid_constant__ CUtensorMap mapB, int useTma, int tiles, int weightsResident, int stages,
@@ -215,7 +225,7 @@ namespace {
     {
         using S = ConvTcShape<NT>;
         constexpr int ZT = S::ZT;
-        extern __shared__ __align__(128) unsigned char smem[];
+        extern __shared__ __align__(256) unsigned char smemRaw[];
         __shared__ __align__(8) uint64_t full[S::kMaxStages];    // producers' copies of stage b visible
         __shared__ __align__(8) uint64_t tmaFull[S::kMaxStages]; // the TMA halo of stage b landed
         __shared__ __align__(8) uint64_t empty[S::kMaxStages];   // the MMAs reading stage b are done
@@ -228,7 +238,9 @@ namespace {
         const int warp = t >> 5;
         const int n0 = blockIdx.y * NT;
         const int nSlices = Cin >> 4;
-        const uint32_t sbase = umma::smemAddr(smem);
+        // the swizzle goes by address bits: the buffers start on a multiple of 256
+        const uint32_t sbase = (umma::smemAddr(smemRaw) + 255u) & ~255u;
+        unsigned char* const smem = smemRaw + (sbase - umma::smemAddr(smemRaw));
         const uint32_t wbase = sbase + stages * S::kHalo;
         // this CTA's bricks: blockIdx.x, blockIdx.x + gridDim.x, ... of the brick list
         // (ep.list, ep.listLen entries) or of all `tiles` bricks
@@ -261,11 +273,13 @@ namespace {
         umma::fenceAfterSync();
         const uint32_t tm = tmemBase;
         const uint32_t laneBase = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-        // zero both accumulator sets (warp w: lanes 32 (w % 4).., half of the columns)
+        // zero both accumulator sets (warp w < 8: lanes 32 (w % 4).., half of the columns)
+        if (warp < 8) {
 #pragma unroll
-        for (int c = 0; c < static_cast<int>(S::kAcc); c += 16)
-            umma::tmemZero16(tm + laneBase + (warp >> 2) * S::kAcc + c);
-        umma::storeWait();
+            for (int c = 0; c < static_cast<int>(S::kAcc); c += 16)
+                umma::tmemZero16(tm + laneBase + (warp >> 2) * S::kAcc + c);
+            umma::storeWait();
+        }
 
         // a slice's weights for all taps, z-taps stacked per in-plane tap (cp.async by the
         // threads [first, first + count))
@@ -283,7 +297,7 @@ namespace {
         };
         if (weightsResident) {
             for (int sl = 0; sl < nSlices; ++sl)
-                stageWeights(sl, wbase + sl * S::kWeights, 0, 256);
+                stageWeights(sl, wbase + sl * S::kWeights, 0, kConvThreads);
             asm volatile("cp.async.commit_group;\n" ::);
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         }
@@ -299,36 +313,37 @@ namespace {
         // whether the halo of slice sl comes by TMA (uniform over the CTA)
         const auto byTma = [&](int sl) {
             const bool inA = sl * 16 < in.ca;
-            return useTma && !(inA && in.halfA) && (sbase & 127u) == 0u;
+            return useTma && !(inA && in.halfA);
         };
 
         if (warp == 0) {
             // ------------------------------------------------------------ MMA issuer
-            if (t == 0) {
-                bool ok = true;
-                uint32_t tmaPhase = 0; // bit b: phase of tmaFull[b] (only TMA items complete it)
-                for (int it = 0; it < nItems && ok; ++it) {
-                    const int b = it % stages;
-                    const uint32_t use = static_cast<uint32_t>(it / stages);
-                    const int sl = it % nSlices;
-                    const int k = it / nSlices; // this CTA's brick number
-                    const int set = k & 1;
-                    ok = umma::mbarWaitOrAbort(&full[b], use & 1u, hp, abortp);
-                    if (ok && byTma(sl)) {
-                        ok = umma::mbarWaitOrAbort(&tmaFull[b], tmaPhase >> b & 1u, hp, abortp);
-                        tmaPhase ^= 1u << b;
-                    }
-                    if (ok && sl == 0 && k >= 2)
-                        ok = umma::mbarWaitOrAbort(&accEmpty[set], static_cast<uint32_t>((k >> 1) - 1) & 1u, hp,
-                            abortp);
-                    if (!ok)
-                        break;
-                    umma::fenceAfterSync();
-                    // plane hz feeds output slices hz - dz1 for dz1 = dz + 1 in [lo, hi]; the
-                    // stacked B rows of those z-taps start at row (2 - hi) NT and land from
-                    // column (hz - hi) NT.  Descriptor start addresses are in 16-byte units in
-                    // the low 14 bits (shared memory < 256 KB): offsets are added directly.
-                    const uint64_t aBase = umma::smemDescriptor(sbase + b * S::kHalo, S::kPlane, S::HX * 16);
+            const bool one = umma::electOne();
+            bool ok = true;
+            uint32_t tmaPhase = 0; // bit b: phase of tmaFull[b] (only TMA items complete it)
+            for (int it = 0; it < nItems && ok; ++it) {
+                const int b = it % stages;
+                const uint32_t use = static_cast<uint32_t>(it / stages);
+                const int sl = it % nSlices;
+                const int k = it / nSlices; // this CTA's brick number
+                const int set = k & 1;
+                ok = umma::mbarWaitOrAbort(&full[b], use & 1u, hp, abortp);
+                if (ok && byTma(sl)) {
+                    ok = umma::mbarWaitOrAbort(&tmaFull[b], tmaPhase >> b & 1u, hp, abortp);
+                    tmaPhase ^= 1u << b;
+                }
+                if (ok && sl == 0 && k >= 2)
+                    ok = umma::mbarWaitOrAbort(&accEmpty[set], static_cast<uint32_t>((k >> 1) - 1) & 1u, hp,
+                        abortp);
+                if (!ok)
+                    break;
+                umma::fenceAfterSync();
+                // plane hz feeds output slices hz - dz1 for dz1 = dz + 1 in [lo, hi]; the
+                // stacked B rows of those z-taps start at row (2 - hi) NT and land from
+                // column (hz - hi) NT.  Descriptor start addresses are in 16-byte units in
+                // the low 14 bits (shared memory < 256 KB): offsets are added directly.
+                if (one) {
+                    const uint64_t aBase = umma::smemDescriptorSwizzle32(sbase + b * S::kHalo, S::HX * 32);
                     const uint64_t bBase = umma::smemDescriptor(
                         wbase + (weightsResident ? sl : b) * S::kWeights, 3 * NT * 16, 128);
                     const uint32_t dBase = tm + set * S::kAcc;
@@ -338,13 +353,13 @@ namespace {
                         const int hi = hz < 2 ? hz : 2;
                         const uint32_t idesc = umma::instrDescriptorBf16(128, (hi - lo + 1) * NT);
                         const uint32_t d = dBase + (hz - hi) * NT;
-                        const uint64_t aPlane = aBase + static_cast<uint64_t>(hz * S::HY * S::HX);
+                        const uint64_t aPlane = aBase + static_cast<uint64_t>(hz * S::HY * S::HX * 2);
                         const uint64_t bPlane = bBase + static_cast<uint64_t>(((2 - hi) * NT * 16) >> 4);
 #pragma unroll
                         for (int q = 0; q < 9; ++q) {
                             const int dy1 = q / 3, dx1 = q % 3;
                             umma::mmaBf16<umma::Collector::kNone>(d,
-                                aPlane + static_cast<uint64_t>(dy1 * S::HX + dx1),
+                                aPlane + static_cast<uint64_t>((dy1 * S::HX + dx1) * 2),
                                 bPlane + static_cast<uint64_t>((q * S::kStackBytes) >> 4), idesc, true);
                         }
                     }
@@ -352,14 +367,16 @@ namespace {
                     if (sl == nSlices - 1)
                         umma::commit(&accFull[set]);
                 }
-                if (!ok)
-                    *abortp = 1;
-                // nothing issued may still run when the memory is given back
-                umma::commit(&drain);
-                if (!umma::mbarWait(&drain, 0, kPolls))
-                    *abortp = 1;
+                __syncwarp(); // no lane waits on a barrier whose phase ran ahead of it
             }
-        } else if (warp < 4) {
+            if (!ok)
+                *abortp = 1;
+            // nothing issued may still run when the memory is given back
+            if (one)
+                umma::commit(&drain);
+            if (!umma::mbarWait(&drain, 0, kPolls))
+                *abortp = 1;
+        } else if (warp < 8) {
             // ------------------------------------------------------------ producers
             const int pt = t - 32; // 0 .. kProducers - 1
             uint32_t tmaPending = 0, tmaPhase = 0;
@@ -391,7 +408,6 @@ namespace {
                         const CUtensorMap* m = inA ? &mapA : &mapB;
                         umma::mbarArriveExpectTx(&tmaFull[b], S::kHalo);
                         umma::tmaLoad5d(dst, m, cc, p.x0 - 1, p.y0 - 1, p.z0 - 1, p.b, &tmaFull[b]);
-                        umma::tmaLoad5d(dst + S::kPlane, m, cc + 8, p.x0 - 1, p.y0 - 1, p.z0 - 1, p.b, &tmaFull[b]);
                         tmaPending |= 1u << b;
                     }
                 } else if (half) {
@@ -426,14 +442,15 @@ namespace {
                                 const int lz = v / (S::LY * S::LX), ly = (v / S::LX) % S::LY, lx = v % S::LX;
                                 // children at halo (2 lz - 1 + cz, ...): z0, y0 and x0 are even
                                 const int hz0 = 2 * lz - 1, hy0 = 2 * ly - 1, hx0 = 2 * lx - 1;
-                                unsigned char* base = dstp + h * S::kPlane;
+                                const int v0 = (hz0 * S::HY + hy0) * S::HX + hx0;
+                                const bool in[6] = { hz0 >= 0, hz0 + 1 < S::HZ, hy0 >= 0, hy0 + 1 < S::HY, hx0 >= 0,
+                                    hx0 + 1 < S::HX };
 #pragma unroll
                                 for (int c = 0; c < 8; ++c) {
-                                    const int hz = hz0 + (c >> 2), hy = hy0 + ((c >> 1) & 1), hx = hx0 + (c & 1);
-                                    if (static_cast<unsigned>(hz) < static_cast<unsigned>(S::HZ)
-                                        && static_cast<unsigned>(hy) < static_cast<unsigned>(S::HY)
-                                        && static_cast<unsigned>(hx) < static_cast<unsigned>(S::HX))
-                                        *reinterpret_cast<uint4*>(base + ((hz * S::HY + hy) * S::HX + hx) * 16)
+                                    const int cz = c >> 2, cy = (c >> 1) & 1, cx = c & 1;
+                                    if (in[cz] && in[2 + cy] && in[4 + cx])
+                                        *reinterpret_cast<uint4*>(
+                                            dstp + haloOffset(v0 + (cz * S::HY + cy) * S::HX + cx, h))
                                             = lowv[k];
                                 }
                             }
@@ -449,7 +466,7 @@ namespace {
                         const __nv_bfloat16* q = inside
                             ? src + ((((static_cast<size_t>(p.b) * D + gz) * H + gy) * W + gx) * cs + cc + h * 8)
                             : src;
-                        cpAsync16(dst + h * S::kPlane + v * 16, q, inside);
+                        cpAsync16(dst + haloOffset(v, h), q, inside);
                     }
                 }
                 if (!weightsResident)
@@ -495,26 +512,43 @@ namespace {
                 const int y = p.y0 + (row >> 3), x = p.x0 + (row & 7);
                 const bool inPlane = y < H && x < W;
                 const uint32_t acc = tm + laneBase + set * S::kAcc;
+                // two slices of a 16-channel group at a time; the next two are on their way
+                // from TMEM while these are packed and stored
+                constexpr int kPairs = (NT / 16) * (ZT / 2);
+                const auto pairAddr = [&](int i) { return acc + 2 * (i % (ZT / 2)) * NT + 16 * (i / (ZT / 2)); };
+                static_assert(kPairs % 2 == 0, "");
+                uint32_t raw[2][2][16];
+                umma::tmemLoad16Start(pairAddr(0), raw[0][0]);
+                umma::tmemLoad16Start(pairAddr(0) + NT, raw[0][1]);
+                float bv[16];
+                // the double buffer's index is a constant only in unrolled code: two a trip
 #pragma unroll 1
-                for (int c = 0; c < NT; c += 16) {
-                    float bv[16];
+                for (int i0 = 0; i0 < kPairs; i0 += 2) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        bv[j] = bias ? __ldg(bias + n0 + c + j) : 0.0f;
-#pragma unroll 1
-                    for (int o = 0; o < ZT; o += 2) {
+                    for (int u = 0; u < 2; ++u) {
+                        const int i = i0 + u;
+                        const int c = 16 * (i / (ZT / 2)), o = 2 * (i % (ZT / 2));
+                        umma::loadWait(raw[u][0], raw[u][1]);
+                        if (i + 1 < kPairs) {
+                            umma::tmemLoad16Start(pairAddr(i + 1), raw[u ^ 1][0]);
+                            umma::tmemLoad16Start(pairAddr(i + 1) + NT, raw[u ^ 1][1]);
+                        }
+                        umma::tmemZero16(pairAddr(i));
+                        umma::tmemZero16(pairAddr(i) + NT);
+                        if (o == 0) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                bv[j] = bias ? __ldg(bias + n0 + c + j) : 0.0f;
+                        }
                         float r[2][16]; // the bf16 outputs of slices o and o + 1, as floats
 #pragma unroll
                         for (int s2 = 0; s2 < 2; ++s2) {
-                            float v[16];
-                            const uint32_t ta = acc + (o + s2) * NT + c;
-                            umma::tmemLoad16(ta, v);
-                            umma::tmemZero16(ta);
                             uint4 pk[2];
                             __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(pk);
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
-                                float a0 = v[2 * j] + bv[2 * j], a1 = v[2 * j + 1] + bv[2 * j + 1];
+                                float a0 = __uint_as_float(raw[u][s2][2 * j]) + bv[2 * j],
+                                      a1 = __uint_as_float(raw[u][s2][2 * j + 1]) + bv[2 * j + 1];
                                 if (relu) {
                                     a0 = fmaxf(a0, 0.0f);
                                     a1 = fmaxf(a1, 0.0f);
@@ -615,7 +649,7 @@ namespace {
     }
 
     // 5-D map (C, W, H, D, B) of a channels-last bf16 tensor with a halo box
-    // (8, 10, 18, hz, 1); false if it cannot be made (the kernel then uses cp.async)
+    // (16, 10, 18, hz, 1) in the 32-byte swizzle; false if it cannot be made (the kernel then uses cp.async)
     bool haloTensorMap(CUtensorMap* m, const void* base, int B, int D, int H, int W, int C, int hz)
     {
         const auto encode = tensorMapEncoder();
@@ -625,10 +659,10 @@ namespace {
             static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(B) };
         const cuuint64_t row = static_cast<cuuint64_t>(C) * 2;
         const cuuint64_t strides[4] = { row, row * W, row * W * H, row * W * H * D };
-        const cuuint32_t box[5] = { 8, 10, 18, static_cast<cuuint32_t>(hz), 1 };
+        const cuuint32_t box[5] = { 16, 10, 18, static_cast<cuuint32_t>(hz), 1 };
         const cuuint32_t step[5] = { 1, 1, 1, 1, 1 };
         return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, step,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
             == CUDA_SUCCESS;
     }
@@ -664,7 +698,7 @@ namespace {
         const int stages = 2;
         const int gy = Cout / NT;
         const int gx = std::max(1, std::min(tiles, sms / gy));
-        conv3TcKernel<NT><<<dim3(gx, gy), 256, S::smemFor(nSlices, resident, stages), s>>>(in, D, H, W, Cin, w, bias,
+        conv3TcKernel<NT><<<dim3(gx, gy), kConvThreads, S::smemFor(nSlices, resident, stages), s>>>(in, D, H, W, Cin, w, bias,
             Cout, relu ? 1 : 0, out, mapA, mapB, tma ? 1 : 0, tiles, resident ? 1 : 0, stages, ep);
         return cudaGetLastError();
     }

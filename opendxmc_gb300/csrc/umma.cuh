@@ -33,6 +33,15 @@ namespace umma {
         return d;       // base offset 0, LBO mode 0, layout type 0 (no swizzle)
     }
 
+    // The same for a K-major operand of 32-byte rows (16 bf16) in the 32-byte swizzle: the
+    // two 16-byte halves of a row are exchanged where bit 7 of its address is set, as a
+    // SWIZZLE_32B tensor map writes them into a buffer aligned to 256 bytes; 8 rows are 256
+    // consecutive bytes, groups of 8 rows sbo bytes apart.
+    __device__ __forceinline__ uint64_t smemDescriptorSwizzle32(uint32_t saddr, uint32_t sbo)
+    {
+        return smemDescriptor(saddr, 16, sbo) | 6ull << 61;
+    }
+
     // Instruction descriptor of kind::f16: D in FP32, A and B bf16, both K-major,
     // M x N (M = 64 or 128; N a multiple of 8 for M = 64, of 16 for M = 128).
     __host__ __device__ constexpr uint32_t instrDescriptorBf16(int M, int N)
@@ -98,6 +107,16 @@ namespace umma {
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
                          smemAddr(bar))
                      : "memory");
+    }
+
+    // One lane of a converged warp.  Issuing tcgen05 instructions under this predicate,
+    // with the loop around it run by the whole warp, lets the compiler keep descriptors in
+    // uniform registers; under `threadIdx.x == 0` every operand is moved there anew.
+    __device__ __forceinline__ bool electOne()
+    {
+        uint32_t p;
+        asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+        return p != 0u;
     }
 
     // ---- mbarrier
@@ -197,6 +216,28 @@ namespace umma {
 #pragma unroll
         for (int i = 0; i < 16; ++i)
             v[i] = __uint_as_float(r[i]);
+    }
+
+    // The same in two parts, so that several loads are in flight before one wait: the
+    // registers hold the values only after loadWait, which takes them as operands.
+    __device__ __forceinline__ void tmemLoad16Start(uint32_t taddr, uint32_t (&r)[16])
+    {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
+                     "[%16];\n"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                     "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+                     "=r"(r[14]), "=r"(r[15])
+                     : "r"(taddr));
+    }
+    __device__ __forceinline__ void loadWait(uint32_t (&r)[16], uint32_t (&q)[16])
+    {
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+                     : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
+                     "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]),
+                     "+r"(r[14]), "+r"(r[15])::"memory");
+        asm volatile("" : "+r"(q[0]), "+r"(q[1]), "+r"(q[2]), "+r"(q[3]), "+r"(q[4]), "+r"(q[5]), "+r"(q[6]),
+                     "+r"(q[7]), "+r"(q[8]), "+r"(q[9]), "+r"(q[10]), "+r"(q[11]), "+r"(q[12]), "+r"(q[13]),
+                     "+r"(q[14]), "+r"(q[15])::"memory");
     }
 
     // registers -> TMEM: zeroes 16 consecutive FP32 columns of this warp's 32 lanes
