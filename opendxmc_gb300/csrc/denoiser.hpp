@@ -25,7 +25,6 @@ struct ConvIn {
 };
 
 size_t conv3SmemBytes(int nt);
-size_t wgradSmemBytes(int nt);
 cudaError_t conv3Configure(); // opt the kernels into their shared-memory size (once per device)
 
 // Options of the tcgen05 convolution beyond launchConv3's:

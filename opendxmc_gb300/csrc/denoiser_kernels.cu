@@ -14,6 +14,7 @@
 // FP32 accumulation; rows are loaded with ldmatrix from shared memory whose
 // 16-byte halves are XOR-swizzled so that the eight rows of a matrix fall in
 // distinct banks.
+#include <algorithm>
 #include <cstdint>
 
 #include <cuda_bf16.h>
@@ -363,103 +364,171 @@ namespace {
 
     // ------------------------------------------------------------------ weight gradient
     // dW[co][tap][ci] += sum over output voxels v of dz[v][co] * x[v + off(tap)][ci].
-    // grid: x = CTAs looping over bricks, y = output-channel tile, z = input slice.
-    // Warp w owns taps w, w+8, w+16 (and 24 for w < 3) and keeps their partial sums
-    // in registers across all its bricks; one atomic flush per CTA at the end.
-    template <int NT>
-    __global__ void __launch_bounds__(256, 1) wgradKernel(const ConvIn in, const __nv_bfloat16* __restrict__ dz,
-        int D, int H, int W, int Cin, int Cout, int nBricks, float* __restrict__ dW)
+    // grid: x = CTAs looping over bricks, y = 16-output-channel tile, z = input slice.
+    //
+    // bf16 mma.sync with the voxels as the K dimension (for tcgen05 the channel counts, 16
+    // at level 0, would be M and N: a quarter of its narrowest tile).  Its rate, one
+    // m16n8k16 per two cycles and SM, is the bound to reach, and shared memory must not
+    // stand before it.  So warp (p, g) owns the nine taps of z-plane p and the brick's
+    // z-slices 2 g, 2 g + 1: a 16-voxel step (two rows of 8) multiplies one fragment of dz
+    // with 9 x 2 fragments of x, and of the four halo rows those need, two stay in
+    // registers from the step before: 4 ldmatrix.x4 for 18 MMAs.  (One tap a warp and step,
+    // re-reading dz for each tap, took 2 for 2.)  Bricks arrive through three cp.async stages;
+    // the four z-groups' sums meet in shared memory and leave by one atomic per weight and
+    // CTA.  8 x 64^3 voxels: 16 to 16 channels 190 -> 92 us (48 at the MMA rate), 48 to 16
+    // 794 -> 271 us; with two stages 95 and 281 us.
+    constexpr int kWgradThreads = 384;
+    constexpr int kWgradStage = kHaloBytes + 512 * 32;
+
+    __global__ void __launch_bounds__(kWgradThreads, 1) wgradKernel(const ConvIn in,
+        const __nv_bfloat16* __restrict__ dz, int D, int H, int W, int Cin, int Cout, int nBricks,
+        float* __restrict__ dW)
     {
         extern __shared__ __align__(128) unsigned char smem[];
-        constexpr int kRow = NT * 2; // bytes of one voxel's NT gradient values
-        constexpr int kChunks = NT / 8;
-        const unsigned haloBase = smemAddr(smem);
-        const unsigned dzBase = haloBase + kHaloBytes;
-        const int n0 = blockIdx.y * NT;
+        const int n0 = blockIdx.y * 16;
         const int c0 = blockIdx.z * 16;
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         const int q = lane >> 3, r = lane & 7;
-        const int nSlots = warp < 3 ? 4 : 3;
+        const int plane = warp % 3, group = warp / 3;
 
-        float acc[4][NT / 16][2][4];
+        // this thread's copies of a brick, 16 bytes each: halo voxels (tid >> 1) + 192 k and
+        // output voxels (tid >> 1) + 192 k, half tid & 1.  A brick starts on a multiple of 8
+        // on each axis, so their offsets from its first voxel, in a half-resolution input
+        // too, are the same for every brick.
+        constexpr int kXCopies = (2 * kHaloVox + kWgradThreads - 1) / kWgradThreads;
+        constexpr int kZCopies = (2 * 512 + kWgradThreads - 1) / kWgradThreads;
+        const int tid = static_cast<int>(threadIdx.x), h = tid & 1;
+        const bool inA = c0 < in.ca;
+        const int cs = inA ? in.ca : in.cb;
+        const __nv_bfloat16* const xSrc = (inA ? in.a + c0 : in.b + (c0 - in.ca)) + h * 8;
+        const int sh = inA && in.halfA ? 1 : 0;
+        const int Ds = D >> sh, Hs = H >> sh, Ws = W >> sh;
+        int xRel[kXCopies];
+        unsigned xAt[kXCopies]; // hz, hy, hx
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
-#pragma unroll
-            for (int m = 0; m < NT / 16; ++m)
-#pragma unroll
-                for (int n = 0; n < 2; ++n)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        acc[s][m][n][k] = 0.0f;
-
-        for (int brick = blockIdx.x; brick < nBricks; brick += gridDim.x) {
+        for (int k = 0; k < kXCopies; ++k) {
+            const int v = (tid >> 1) + (kWgradThreads / 2) * k;
+            const int hz = v / 100, hy = (v / 10) % 10, hx = v % 10;
+            // (hz - 1) >> 1 rounds down, as the voxel's own index shifted does
+            xRel[k] = (((hz - 1) >> sh) * Hs + ((hy - 1) >> sh)) * Ws + ((hx - 1) >> sh);
+            xAt[k] = static_cast<unsigned>(hz | hy << 8 | hx << 16);
+        }
+        const auto load = [&](int brick, int stage) {
+            const unsigned base = smemAddr(smem + stage * kWgradStage);
             const BrickPos p = brickOf(brick, D, H, W);
-            loadHalo(in, c0, p, D, H, W, haloBase);
-            for (int i = threadIdx.x; i < 512 * kChunks; i += blockDim.x) {
-                const int v = i / kChunks, c = i % kChunks;
-                const int z = p.z0 + (v >> 6), y = p.y0 + ((v >> 3) & 7), x = p.x0 + (v & 7);
-                const bool ok = z < D && y < H && x < W;
-                const __nv_bfloat16* src
-                    = ok ? dz + ((((static_cast<size_t>(p.b) * D + z) * H + y) * W + x) * Cout + n0 + c * 8) : dz;
-                const int key = NT == 32 ? ((v >> 1) & 3) : ((v >> 2) & 1);
-                cpAsync16(dzBase + v * kRow + ((c ^ key) << 4), src, ok);
-            }
-            cpAsyncCommit();
-            cpAsyncWait<0>();
-            __syncthreads();
+            const long long x0 = ((static_cast<long long>(p.b) * Ds + (p.z0 >> sh)) * Hs + (p.y0 >> sh)) * Ws
+                + (p.x0 >> sh);
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                if (s >= nSlots)
+            for (int k = 0; k < kXCopies; ++k) {
+                const int v = (tid >> 1) + (kWgradThreads / 2) * k;
+                if (k == kXCopies - 1 && v >= kHaloVox)
                     break;
-                const int tap = warp + 8 * s;
-                const int dzt = tapDz(tap), dyt = tapDy(tap), dxt = tapDx(tap);
-#pragma unroll 2
-                for (int ks = 0; ks < 32; ++ks) {
-                    // voxels 16 ks .. 16 ks + 15 of the brick: z = ks / 4, y = 2 (ks % 4) + (row >= 8)
-                    const int zz = ks >> 2, yb = (ks & 3) * 2;
-                    // B: x rows (k = voxel), 8 input channels per matrix, transposed
-                    unsigned b00, b01, b10, b11;
-                    {
-                        const int yy = yb + (q & 1);
-                        const int hz = zz + dzt + 1, hy = yy + dyt + 1, hx = r + dxt + 1;
-                        const int v = (hz * 10 + hy) * 10 + hx;
-                        const int h = q >> 1;
-                        ldsm4t(haloBase + v * 32 + ((h ^ ((hx >> 2) & 1)) << 4), b00, b01, b10, b11);
-                    }
+                const int hx = static_cast<int>(xAt[k] >> 16);
+                const bool ok = static_cast<unsigned>(p.z0 - 1 + static_cast<int>(xAt[k] & 0xffu))
+                        < static_cast<unsigned>(D)
+                    && static_cast<unsigned>(p.y0 - 1 + static_cast<int>(xAt[k] >> 8 & 0xffu))
+                        < static_cast<unsigned>(H)
+                    && static_cast<unsigned>(p.x0 - 1 + hx) < static_cast<unsigned>(W);
+                cpAsync16(base + v * 32 + ((h ^ (hx >> 2 & 1)) << 4), ok ? xSrc + (x0 + xRel[k]) * cs : xSrc, ok);
+            }
+            const long long z0 = ((static_cast<long long>(p.b) * D + p.z0) * H + p.y0) * W + p.x0;
 #pragma unroll
-                    for (int m = 0; m < NT / 16; ++m) {
-                        // A: dz rows (k = voxel) x 8 output channels per matrix, transposed
-                        const int vrow = ks * 16 + ((q >> 1) << 3) + r;
-                        const int c = m * 2 + (q & 1);
-                        const int key = NT == 32 ? ((vrow >> 1) & 3) : ((vrow >> 2) & 1);
-                        unsigned a0, a1, a2, a3;
-                        ldsm4t(dzBase + vrow * kRow + ((c ^ key) << 4), a0, a1, a2, a3);
-                        mma16816(acc[s][m][0], a0, a1, a2, a3, b00, b01);
-                        mma16816(acc[s][m][1], a0, a1, a2, a3, b10, b11);
+            for (int k = 0; k < kZCopies; ++k) {
+                const int v = (tid >> 1) + (kWgradThreads / 2) * k;
+                if (k == kZCopies - 1 && v >= 512)
+                    break;
+                const int z = v >> 6, y = v >> 3 & 7, x = v & 7;
+                const bool ok = p.z0 + z < D && p.y0 + y < H && p.x0 + x < W;
+                cpAsync16(base + kHaloBytes + v * 32 + ((h ^ (v >> 2 & 1)) << 4),
+                    ok ? dz + (z0 + (z * H + y) * W + x) * Cout + n0 + h * 8 : dz, ok);
+            }
+        };
+
+        float acc[9][2][4];
+#pragma unroll
+        for (int t = 0; t < 9; ++t)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    acc[t][n][k] = 0.0f;
+
+        // this lane's addresses: x rows (halo row q >> 1, voxel r + dx, half q & 1) and dz rows
+        // (row q >> 1 of the step, voxel r, half q & 1)
+        unsigned xOff[3];
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx) {
+            const int hx = r + dx;
+            xOff[dx] = static_cast<unsigned>(((q >> 1) * 10 + hx) * 32 + (((q & 1) ^ ((hx >> 2) & 1)) << 4));
+        }
+        const unsigned zOff = static_cast<unsigned>(
+            kHaloBytes + (((q >> 1) << 3) + r) * 32 + (((q & 1) ^ ((r >> 2) & 1)) << 4));
+
+        // stage i mod 3 holds the CTA's brick i; brick i + 2 loads over brick i - 1, which
+        // the barrier tells every warp is done with
+        const int first = static_cast<int>(blockIdx.x), hop = static_cast<int>(gridDim.x);
+        for (int i = 0; i < 2; ++i) {
+            if (first + i * hop < nBricks)
+                load(first + i * hop, i);
+            cpAsyncCommit();
+        }
+        for (int brick = first, stage = 0; brick < nBricks; brick += hop, stage = stage == 2 ? 0 : stage + 1) {
+            cpAsyncWait<1>();
+            __syncthreads();
+            if (brick + 2 * hop < nBricks)
+                load(brick + 2 * hop, stage == 0 ? 2 : stage - 1);
+            cpAsyncCommit();
+            const unsigned base = smemAddr(smem + stage * kWgradStage);
+#pragma unroll 1
+            for (int s = 0; s < 2; ++s) {
+                const int z = 2 * group + s;
+                const unsigned xBase = base + (z + plane) * (100 * 32);
+                const unsigned zBase = base + zOff + z * (64 * 32);
+                unsigned b[4][3][2]; // halo rows (rotating), dx, channel half
+                const auto rows = [&](int hy) { // halo rows hy and hy + 1
+#pragma unroll
+                    for (int dx = 0; dx < 3; ++dx)
+                        ldsm4t(xBase + xOff[dx] + hy * 320, b[hy & 3][dx][0], b[hy & 3][dx][1],
+                            b[(hy + 1) & 3][dx][0], b[(hy + 1) & 3][dx][1]);
+                };
+                rows(0);
+#pragma unroll
+                for (int yb = 0; yb < 8; yb += 2) {
+                    rows(yb + 2);
+                    unsigned a0, a1, a2, a3;
+                    ldsm4t(zBase + yb * 256, a0, a1, a2, a3);
+#pragma unroll
+                    for (int t = 0; t < 9; ++t) {
+                        const int dy = t / 3, dx = t % 3;
+                        const int r0 = (yb + dy) & 3, r1 = (yb + dy + 1) & 3;
+                        mma16816(acc[t][0], a0, a1, a2, a3, b[r0][dx][0], b[r1][dx][0]);
+                        mma16816(acc[t][1], a0, a1, a2, a3, b[r0][dx][1], b[r1][dx][1]);
                     }
                 }
             }
-            __syncthreads(); // the next brick's loads overwrite the staging
         }
 
-        const int g = lane >> 2, t = lane & 3;
+        // the z-groups' sums, one group after the other, then one atomic a weight
+        float* sum = reinterpret_cast<float*>(smem); // [16 co][27 taps][16 ci]
+        cpAsyncWait<0>();
+        const int g = lane >> 2, tq = lane & 3;
+        for (int turn = 0; turn < 4; ++turn) {
+            __syncthreads();
+            if (group != turn)
+                continue;
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            if (s >= nSlots)
-                break;
-            const int tap = warp + 8 * s;
-#pragma unroll
-            for (int m = 0; m < NT / 16; ++m)
+            for (int t = 0; t < 9; ++t)
 #pragma unroll
                 for (int n = 0; n < 2; ++n)
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        const int co = n0 + m * 16 + g + ((k >> 1) << 3);
-                        const int ci = c0 + n * 8 + 2 * t + (k & 1);
-                        if (co < Cout)
-                            atomicAdd(dW + (static_cast<size_t>(co) * 27 + tap) * Cin + ci, acc[s][m][n][k]);
+                        float* w = sum + ((g + ((k >> 1) << 3)) * 27 + 9 * plane + t) * 16 + n * 8 + 2 * tq + (k & 1);
+                        *w = turn ? *w + acc[t][n][k] : acc[t][n][k];
                     }
         }
+        __syncthreads();
+        for (int i = threadIdx.x; i < 16 * 27 * 16; i += kWgradThreads)
+            atomicAdd(dW + static_cast<size_t>(n0 * 27 + (i >> 4)) * Cin + c0 + (i & 15), sum[i]);
     }
 
     // ------------------------------------------------------------------ elementwise passes
@@ -844,7 +913,6 @@ namespace {
 } // namespace
 
 size_t conv3SmemBytes(int nt) { return 2 * static_cast<size_t>(kHaloBytes + 27 * nt * 32); }
-size_t wgradSmemBytes(int nt) { return static_cast<size_t>(kHaloBytes) + 512 * nt * 2; }
 
 cudaError_t conv3Configure()
 {
@@ -857,11 +925,7 @@ cudaError_t conv3Configure()
         e = cudaFuncSetAttribute(conv3SmallKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
             kSmallStages * kSmallStage);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(wgradKernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            static_cast<int>(wgradSmemBytes(16)));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(wgradKernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            static_cast<int>(wgradSmemBytes(32)));
+        e = cudaFuncSetAttribute(wgradKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * kWgradStage);
     return e;
 }
 
@@ -896,19 +960,12 @@ cudaError_t launchWgrad(const ConvIn& in, const __nv_bfloat16* dz, int B, int D,
 {
     if (Cin % 16 || Cout % 16)
         return cudaErrorInvalidValue;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int bricks = B * ((D + 7) / 8) * ((H + 7) / 8) * ((W + 7) / 8);
-    const int nt = Cout % 32 == 0 ? 32 : 16;
-    const int tiles = (Cout / nt) * (Cin / 16);
-    int gx = (2 * sms + tiles - 1) / tiles;
-    gx = gx < 1 ? 1 : (gx > bricks ? bricks : gx);
-    const dim3 grid(gx, Cout / nt, Cin / 16);
-    if (nt == 32)
-        wgradKernel<32><<<grid, 256, wgradSmemBytes(32), s>>>(in, dz, D, H, W, Cin, Cout, bricks, dW);
-    else
-        wgradKernel<16><<<grid, 256, wgradSmemBytes(16), s>>>(in, dz, D, H, W, Cin, Cout, bricks, dW);
+    const int tiles = (Cout / 16) * (Cin / 16);
+    // one CTA an SM: as many per tile as fill the SMs once
+    const int gx = std::max(1, std::min(bricks, smCount() / tiles));
+    wgradKernel<<<dim3(gx, Cout / 16, Cin / 16), kWgradThreads, 3 * kWgradStage, s>>>(in, dz, D, H, W, Cin, Cout,
+        bricks, dW);
     return cudaGetLastError();
 }
 
