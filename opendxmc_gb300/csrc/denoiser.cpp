@@ -47,7 +47,6 @@ struct dxmcg_denoiser {
     // activations and gradients of the current shape, per level
     int B = 0, D = 0, H = 0, W = 0;
     std::vector<DevBuf<bf16>> x, ea, eb, da, db, gx, gea, geb, gda, gdb, dcat;
-    DevBuf<bf16> dz;
     DevBuf<float> pred;
     DevBuf<double> loss;
     // world path: input channels, denoised dose and the normalisation sums, kept
@@ -91,7 +90,6 @@ int ensureShape(dxmcg_denoiser* d, int B, int D, int H, int W)
         vec->clear();
         vec->resize(L);
     }
-    size_t dzMax = 0;
     for (int l = 0; l < L; ++l) {
         const size_t n = d->nvox(l);
         const size_t c = d->ch[l];
@@ -110,9 +108,7 @@ int ensureShape(dxmcg_denoiser* d, int B, int D, int H, int W)
             NN_CUDA(d->gdb[l].reserve(n * c));
             NN_CUDA(d->dcat[l].reserve(n * (c + d->ch[l + 1])));
         }
-        dzMax = std::max(dzMax, n * c);
     }
-    NN_CUDA(d->dz.reserve(dzMax));
     NN_CUDA(d->pred.reserve(d->nvox(0)));
     NN_CUDA(d->loss.reserve(1));
     return DXMCG_OK;
@@ -120,8 +116,14 @@ int ensureShape(dxmcg_denoiser* d, int B, int D, int H, int W)
 
 int refreshWeights(dxmcg_denoiser* d, cudaStream_t s)
 {
-    for (const auto& ly : d->layers)
-        NN_CUDA(nn::launchTransposeWeights(d->pb.p + ly.w, d->wt.p + ly.wt, ly.cout, ly.cin, s));
+    nn::LayerTable t; // at most 5 levels: 18 layers
+    for (const auto& ly : d->layers) {
+        t.cout[t.n] = ly.cout;
+        t.cin[t.n] = ly.cin;
+        t.w[t.n] = ly.w;
+        t.wt[t.n++] = ly.wt;
+    }
+    NN_CUDA(nn::launchTransposeWeights(d->pb.p, d->wt.p, t, s));
     return DXMCG_OK;
 }
 
@@ -391,28 +393,31 @@ int forward(dxmcg_denoiser* d, const bf16* input, cudaStream_t s, float* pred = 
     return DXMCG_OK;
 }
 
-// relu backward + weight/bias gradients, and the input gradient when dxOut
-int layerBack(dxmcg_denoiser* d, int k, const nn::ConvIn& xin, const bf16* y, const bf16* dy, bf16* dxOut, int l,
+// weight and bias gradients of layer k from dz, the gradient before its ReLU; with dxOut
+// also the input gradient, through the ReLU whose output `mask` is (null: none)
+int layerBack(dxmcg_denoiser* d, int k, const nn::ConvIn& xin, const bf16* dz, bf16* dxOut, const bf16* mask, int l,
     cudaStream_t s)
 {
     const auto& ly = d->layers[k];
     const int Dl = d->D >> l, Hl = d->H >> l, Wl = d->W >> l;
-    NN_CUDA(nn::launchReluBackward(dy, y, d->dz.p, d->nvox(l), ly.cout, d->g.p + ly.b, s));
-    NN_CUDA(nn::launchWgrad(xin, d->dz.p, d->B, Dl, Hl, Wl, ly.cin, ly.cout, d->g.p + ly.w, s));
+    NN_CUDA(nn::launchWgrad(xin, dz, d->B, Dl, Hl, Wl, ly.cin, ly.cout, d->g.p + ly.w, d->g.p + ly.b, s));
     if (dxOut) {
         if (useTensorCores(d, Dl, Hl, Wl, ly.cin)) {
             nn::ConvOptions o;
             o.handoverPolls = d->waitPolls;
-            NN_CUDA(nn::launchConv3Tc(plain(d->dz.p, ly.cout), d->B, Dl, Hl, Wl, ly.cout, d->wt.p + ly.wt, nullptr,
+            o.mask = mask;
+            NN_CUDA(nn::launchConv3Tc(plain(dz, ly.cout), d->B, Dl, Hl, Wl, ly.cout, d->wt.p + ly.wt, nullptr,
                 ly.cin, false, dxOut, s, &o));
         }
         else
-            NN_CUDA(nn::launchConv3(plain(d->dz.p, ly.cout), d->B, Dl, Hl, Wl, ly.cout, d->wt.p + ly.wt, nullptr,
-                ly.cin, false, dxOut, s));
+            NN_CUDA(nn::launchConv3(plain(dz, ly.cout), d->B, Dl, Hl, Wl, ly.cout, d->wt.p + ly.wt, nullptr,
+                ly.cin, false, dxOut, s, mask));
     }
     return DXMCG_OK;
 }
 
+// Every ReLU is applied where its gradient is made (the head, the concat split, an input
+// gradient), so that each gradient is written once and read as the dz of its layer.
 int backward(dxmcg_denoiser* d, const bf16* input, const float* target, cudaStream_t s)
 {
     NN_CUDA(cudaMemsetAsync(d->g.p, 0, d->nParams * sizeof(float), s));
@@ -424,25 +429,26 @@ int backward(dxmcg_denoiser* d, const bf16* input, const float* target, cudaStre
     int rc;
     // decoder, from the head towards the bottleneck
     for (int l = 0; l < L - 1; ++l) {
-        if ((rc = layerBack(d, d->decB(l), plain(d->da[l].p, d->ch[l]), d->db[l].p, d->gdb[l].p, d->gda[l].p, l, s))
+        if ((rc = layerBack(d, d->decB(l), plain(d->da[l].p, d->ch[l]), d->gdb[l].p, d->gda[l].p, d->da[l].p, l, s))
             != DXMCG_OK)
             return rc;
-        if ((rc = layerBack(d, d->decA(l), decIn(d, l), d->da[l].p, d->gda[l].p, d->dcat[l].p, l, s)) != DXMCG_OK)
+        if ((rc = layerBack(d, d->decA(l), decIn(d, l), d->gda[l].p, d->dcat[l].p, nullptr, l, s)) != DXMCG_OK)
             return rc;
-        bf16* du = l + 1 < L - 1 ? d->gdb[l + 1].p : d->geb[L - 1].p;
-        NN_CUDA(nn::launchSplitConcatGrad(d->dcat[l].p, d->ch[l + 1], d->ch[l], nullptr, du, nullptr, d->B,
+        const bool inner = l + 1 < L - 1; // the upsampled input is a decoder's output
+        NN_CUDA(nn::launchSplitConcatGrad(d->dcat[l].p, d->ch[l + 1], d->ch[l], nullptr,
+            inner ? d->db[l + 1].p : d->eb[L - 1].p, inner ? d->gdb[l + 1].p : d->geb[L - 1].p, nullptr, nullptr, d->B,
             d->D >> l, d->H >> l, d->W >> l, s));
     }
     // encoder, from the bottleneck down
     for (int l = L - 1; l >= 0; --l) {
         if (l < L - 1)
-            NN_CUDA(nn::launchSplitConcatGrad(d->dcat[l].p, d->ch[l + 1], d->ch[l], d->gx[l + 1].p, nullptr,
-                d->geb[l].p, d->B, d->D >> l, d->H >> l, d->W >> l, s));
-        if ((rc = layerBack(d, d->encB(l), plain(d->ea[l].p, d->ch[l]), d->eb[l].p, d->geb[l].p, d->gea[l].p, l, s))
+            NN_CUDA(nn::launchSplitConcatGrad(d->dcat[l].p, d->ch[l + 1], d->ch[l], d->gx[l + 1].p, nullptr, nullptr,
+                d->eb[l].p, d->geb[l].p, d->B, d->D >> l, d->H >> l, d->W >> l, s));
+        if ((rc = layerBack(d, d->encB(l), plain(d->ea[l].p, d->ch[l]), d->geb[l].p, d->gea[l].p, d->ea[l].p, l, s))
             != DXMCG_OK)
             return rc;
-        if ((rc = layerBack(d, d->encA(l), encIn(d, l, input), d->ea[l].p, d->gea[l].p, l > 0 ? d->gx[l].p : nullptr,
-                 l, s))
+        if ((rc = layerBack(d, d->encA(l), encIn(d, l, input), d->gea[l].p, l > 0 ? d->gx[l].p : nullptr, nullptr, l,
+                 s))
             != DXMCG_OK)
             return rc;
     }

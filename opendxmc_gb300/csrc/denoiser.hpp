@@ -36,6 +36,8 @@ cudaError_t conv3Configure(); // opt the kernels into their shared-memory size (
 //   head:   for a 16-channel output, the 1x1x1 head (16 weights, then the bias) in
 //           place of the output, exactly as launchHead without a target: headPred[v]
 //           = the prediction, headOut[v] = it times headScale (either may be null);
+//   mask:   the output where `mask` (its layout) is positive, 0 elsewhere: an input
+//           gradient times the derivative of the ReLU whose output `mask` is;
 //   handoverPolls: polls of each wait by which one role of the kernel hands work to
 //           another before it gives up (0: 2^24); the waits for copies and MMAs already
 //           in flight keep the default limit, so a kernel that gives up still returns
@@ -48,6 +50,7 @@ struct ConvOptions {
     float* headPred = nullptr;
     double* headOut = nullptr;
     double headScale = 1.0;
+    const __nv_bfloat16* mask = nullptr;
     uint32_t handoverPolls = 0;
 };
 
@@ -98,27 +101,38 @@ struct BrickListJobs {
     }
 };
 cudaError_t launchBrickLists(const BrickListJobs& jobs, cudaStream_t s);
-// out = act(conv3(in) + bias), act = relu or identity; bias may be null
+// out = act(conv3(in) + bias), act = relu or identity; bias and mask (as ConvOptions') may
+// be null
 cudaError_t launchConv3(const ConvIn& in, int B, int D, int H, int W, int Cin, const __nv_bfloat16* w,
-    const float* bias, int Cout, bool relu, __nv_bfloat16* out, cudaStream_t s);
-// dW[co][t][ci] += sum_v dz[v][co] x[v + off(t)][ci]  (FP32 atomics)
+    const float* bias, int Cout, bool relu, __nv_bfloat16* out, cudaStream_t s,
+    const __nv_bfloat16* mask = nullptr);
+// dW[co][t][ci] += sum_v dz[v][co] x[v + off(t)][ci], db[co] += sum_v dz[v][co]  (FP32 atomics)
 cudaError_t launchWgrad(const ConvIn& in, const __nv_bfloat16* dz, int B, int D, int H, int W, int Cin, int Cout,
-    float* dW, cudaStream_t s);
-// dz = dy * (y > 0), db += sum over voxels of dz
-cudaError_t launchReluBackward(const __nv_bfloat16* dy, const __nv_bfloat16* y, __nv_bfloat16* dz, size_t nvox,
-    int C, float* db, cudaStream_t s);
+    float* dW, float* db, cudaStream_t s);
 cudaError_t launchAvgPool(const __nv_bfloat16* x, __nv_bfloat16* out, int B, int D, int H, int W, int C,
     cudaStream_t s);
-// du (half res) = sum of children of dcat[:, :cu]; de = dcat[:, cu:] + dxNext(parent) / 8 (either may be null)
+// du (half res) = sum of children of dcat[:, :cu] where yu > 0; de = dcat[:, cu:] +
+// dxNext(parent) / 8 where ye > 0 (either may be null); 0 elsewhere
 cudaError_t launchSplitConcatGrad(const __nv_bfloat16* dcat, int cu, int cs, const __nv_bfloat16* dxNext,
-    __nv_bfloat16* du, __nv_bfloat16* de, int B, int D, int H, int W, cudaStream_t s);
-// head: pred = d . w + b; with a target also the L1 loss sum and the gradients
+    const __nv_bfloat16* yu, __nv_bfloat16* du, const __nv_bfloat16* ye, __nv_bfloat16* de, int B, int D, int H, int W,
+    cudaStream_t s);
+// head: pred = d . w + b; with a target also the L1 loss sum and the gradients (dd: of the
+// last convolution before its ReLU, 0 where d is)
 cudaError_t launchHead(const __nv_bfloat16* d, int C0, const float* hw, size_t nvox, const float* target,
     float* pred, double predScale, double* predOut, __nv_bfloat16* dd, float* dhw, double* lossSum, cudaStream_t s);
 cudaError_t launchAdam(float* p, const float* g, float* m, float* v, __nv_bfloat16* pb, size_t n, float lr, float b1,
     float b2, float eps, float c1, float c2, cudaStream_t s);
 cudaError_t launchToBf16(const float* p, __nv_bfloat16* pb, size_t n, cudaStream_t s);
-cudaError_t launchTransposeWeights(const __nv_bfloat16* w, __nv_bfloat16* wt, int Cout, int Cin, cudaStream_t s);
+// where the layers' weights lie in the parameter vector (w) and transposed (wt)
+constexpr int kMaxLayers = 18;
+struct LayerTable {
+    int n = 0;
+    int cout[kMaxLayers] = {}, cin[kMaxLayers] = {};
+    size_t w[kMaxLayers] = {}, wt[kMaxLayers] = {};
+};
+// the input gradients' weights (taps flipped, channels exchanged) of every layer
+cudaError_t launchTransposeWeights(const __nv_bfloat16* w, __nv_bfloat16* wt, const LayerTable& layers,
+    cudaStream_t s);
 // Bricks to mark while the input is prepared from a world: active[b] = 1 for each
 // brick b holding a voxel whose material is not 0 (bricks of bx, by, bz voxels, cx and
 // cy of them along x and y, x fastest; the grid nx voxels along x, ny along y).  The

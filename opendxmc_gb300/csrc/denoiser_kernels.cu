@@ -114,11 +114,23 @@ namespace {
         }
     }
 
+    // two channels at index `at` of a convolution's output, 0 where mask is not positive
+    __device__ __forceinline__ void storePair(__nv_bfloat16* out, const __nv_bfloat16* mask, size_t at, float v0,
+        float v1)
+    {
+        if (mask) {
+            const float2 m = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(mask + at));
+            v0 = m.x > 0.0f ? v0 : 0.0f;
+            v1 = m.y > 0.0f ? v1 : 0.0f;
+        }
+        *reinterpret_cast<__nv_bfloat162*>(out + at) = __floats2bfloat162_rn(v0, v1);
+    }
+
     // ------------------------------------------------------------------ forward conv
     template <int NT>
     __global__ void __launch_bounds__(256, 1) conv3Kernel(const ConvIn in, int D, int H, int W, int Cin,
         const __nv_bfloat16* __restrict__ wgt, const float* __restrict__ bias, int Cout, int relu,
-        __nv_bfloat16* __restrict__ out)
+        __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ mask)
     {
         extern __shared__ __align__(128) unsigned char smem[];
         constexpr int kWBytes = 27 * NT * 32;
@@ -201,7 +213,7 @@ namespace {
                 const int y = p.y0 + 2 * i + hf, x = p.x0 + g;
                 if (z >= D || y >= H || x >= W)
                     continue;
-                __nv_bfloat16* o = out + (((static_cast<size_t>(p.b) * D + z) * H + y) * W + x) * Cout;
+                const size_t at = (((static_cast<size_t>(p.b) * D + z) * H + y) * W + x) * Cout;
 #pragma unroll
                 for (int j = 0; j < NT / 8; ++j) {
                     const int co = n0 + 8 * j + 2 * t;
@@ -216,7 +228,7 @@ namespace {
                         v0 = fmaxf(v0, 0.0f);
                         v1 = fmaxf(v1, 0.0f);
                     }
-                    *reinterpret_cast<__nv_bfloat162*>(o + co) = __floats2bfloat162_rn(v0, v1);
+                    storePair(out, mask, at + co, v0, v1);
                 }
             }
     }
@@ -237,7 +249,7 @@ namespace {
 
     __global__ void __launch_bounds__(128) conv3SmallKernel(const ConvIn in, int D, int H, int W, int Cin,
         const __nv_bfloat16* __restrict__ wgt, const float* __restrict__ bias, int Cout, int relu,
-        __nv_bfloat16* __restrict__ out)
+        __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ mask)
     {
         extern __shared__ __align__(128) unsigned char smem[];
         const int nbx = (W + 7) >> 3, nby = (H + 3) >> 2, nbz = (D + 1) >> 1;
@@ -345,7 +357,7 @@ namespace {
             const int y = y0 + 2 * (warp & 1) + hf;
             if (z >= D || y >= H || x >= W)
                 continue;
-            __nv_bfloat16* o = out + (((static_cast<size_t>(bi) * D + z) * H + y) * W + x) * Cout + n0 + 2 * t;
+            const size_t at = (((static_cast<size_t>(bi) * D + z) * H + y) * W + x) * Cout + n0 + 2 * t;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 float v0 = acc[j][2 * hf], v1 = acc[j][2 * hf + 1];
@@ -357,13 +369,14 @@ namespace {
                     v0 = fmaxf(v0, 0.0f);
                     v1 = fmaxf(v1, 0.0f);
                 }
-                *reinterpret_cast<__nv_bfloat162*>(o + 8 * j) = __floats2bfloat162_rn(v0, v1);
+                storePair(out, mask, at + 8 * j, v0, v1);
             }
         }
     }
 
     // ------------------------------------------------------------------ weight gradient
     // dW[co][tap][ci] += sum over output voxels v of dz[v][co] * x[v + off(tap)][ci].
+    // and db[co] += sum of dz[v][co] (by the CTAs of input slice 0, from the same fragments).
     // grid: x = CTAs looping over bricks, y = 16-output-channel tile, z = input slice.
     //
     // bf16 mma.sync with the voxels as the K dimension (for tcgen05 the channel counts, 16
@@ -377,12 +390,17 @@ namespace {
     // the four z-groups' sums meet in shared memory and leave by one atomic per weight and
     // CTA.  8 x 64^3 voxels: 16 to 16 channels 190 -> 92 us (48 at the MMA rate), 48 to 16
     // 794 -> 271 us; with two stages 95 and 281 us.
+    __device__ __forceinline__ float pairSum(unsigned p) // of two bf16
+    {
+        return __uint_as_float(p << 16) + __uint_as_float(p & 0xffff0000u);
+    }
+
     constexpr int kWgradThreads = 384;
     constexpr int kWgradStage = kHaloBytes + 512 * 32;
 
     __global__ void __launch_bounds__(kWgradThreads, 1) wgradKernel(const ConvIn in,
         const __nv_bfloat16* __restrict__ dz, int D, int H, int W, int Cin, int Cout, int nBricks,
-        float* __restrict__ dW)
+        float* __restrict__ dW, float* __restrict__ db)
     {
         extern __shared__ __align__(128) unsigned char smem[];
         const int n0 = blockIdx.y * 16;
@@ -453,6 +471,8 @@ namespace {
                 for (int k = 0; k < 4; ++k)
                     acc[t][n][k] = 0.0f;
 
+        const bool bias = blockIdx.z == 0 && plane == 0;
+        float sb[2] = { 0.0f, 0.0f }; // dz of output channels lane / 4 and lane / 4 + 8
         // this lane's addresses: x rows (halo row q >> 1, voxel r + dx, half q & 1) and dz rows
         // (row q >> 1 of the step, voxel r, half q & 1)
         unsigned xOff[3];
@@ -497,6 +517,10 @@ namespace {
                     rows(yb + 2);
                     unsigned a0, a1, a2, a3;
                     ldsm4t(zBase + yb * 256, a0, a1, a2, a3);
+                    if (bias) {
+                        sb[0] += pairSum(a0) + pairSum(a2);
+                        sb[1] += pairSum(a1) + pairSum(a3);
+                    }
 #pragma unroll
                     for (int t = 0; t < 9; ++t) {
                         const int dy = t / 3, dx = t % 3;
@@ -529,6 +553,15 @@ namespace {
         __syncthreads();
         for (int i = threadIdx.x; i < 16 * 27 * 16; i += kWgradThreads)
             atomicAdd(dW + static_cast<size_t>(n0 * 27 + (i >> 4)) * Cin + c0 + (i & 15), sum[i]);
+        if (bias) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                sb[j] += __shfl_xor_sync(0xffffffffu, sb[j], 1);
+                sb[j] += __shfl_xor_sync(0xffffffffu, sb[j], 2);
+                if (tq == 0)
+                    atomicAdd(db + n0 + g + 8 * j, sb[j]);
+            }
+        }
     }
 
     // ------------------------------------------------------------------ elementwise passes
@@ -552,40 +585,14 @@ namespace {
         return u;
     }
 
-    // dz = dy * (y > 0), and db[c] += sum dz[., c].  Items are 8 channels (16 B); the
-    // grid stride is a multiple of C/8, so each thread keeps one channel group.
-    __global__ void reluBackwardKernel(const uint4* __restrict__ dy, const uint4* __restrict__ y,
-        uint4* __restrict__ dz, size_t items, int groups, float* __restrict__ db)
+    // f where y > 0, 0 elsewhere
+    __device__ __forceinline__ void reluMask(float (&f)[8], const uint4& y)
     {
-        __shared__ float sdb[256];
-        for (int i = threadIdx.x; i < 256; i += blockDim.x)
-            sdb[i] = 0.0f;
-        __syncthreads();
-        float s[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
-        const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-        const size_t i0 = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
-        for (size_t i = i0; i < items; i += stride) {
-            float a[8], b[8];
-            unpack8(dy[i], a);
-            unpack8(y[i], b);
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-                a[k] = b[k] > 0.0f ? a[k] : 0.0f;
-            const uint4 o = pack8(a);
-            dz[i] = o;
-            float c[8];
-            unpack8(o, c); // the bias gradient sums what the other gradients see
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-                s[k] += c[k];
-        }
-        const int grp = static_cast<int>(i0 % groups);
+        float m[8];
+        unpack8(y, m);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-            atomicAdd(&sdb[grp * 8 + k], s[k]);
-        __syncthreads();
-        for (int c = threadIdx.x; c < groups * 8; c += blockDim.x)
-            atomicAdd(db + c, sdb[c]);
+            f[k] = m[k] > 0.0f ? f[k] : 0.0f;
     }
 
     // x_{l+1} = mean over the 2x2x2 children (half resolution output)
@@ -623,9 +630,11 @@ namespace {
 
     // Gradient of the decoder's concat input, split: du (half resolution, channels
     // [0, cu)) = sum of the 2x2x2 children; de (full resolution, channels [cu, cu+cs))
-    // = dcat + dxNext(parent) / 8, the skip path plus the pooled path of the encoder.
+    // = dcat + dxNext(parent) / 8, the skip path plus the pooled path of the encoder; both
+    // through the ReLU they go back to (yu, ye: its outputs).
     __global__ void splitConcatGradKernel(const uint4* __restrict__ dcat, int gu, int gs,
-        const uint4* __restrict__ dxNext, uint4* __restrict__ du, uint4* __restrict__ de, int B, int D, int H, int W)
+        const uint4* __restrict__ dxNext, const uint4* __restrict__ yu, uint4* __restrict__ du,
+        const uint4* __restrict__ ye, uint4* __restrict__ de, int B, int D, int H, int W)
     {
         const int gc = gu + gs;
         const int Dh = D >> 1, Hh = H >> 1, Wh = W >> 1;
@@ -653,6 +662,7 @@ namespace {
                     for (int k = 0; k < 8; ++k)
                         s[k] += f[k];
                 }
+                reluMask(s, yu[i]);
                 du[i] = pack8(s);
             } else {
                 const size_t j = i - nU;
@@ -670,13 +680,15 @@ namespace {
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
                     a[k] += n[k] * 0.125f;
+                reluMask(a, ye[j]);
                 de[j] = pack8(a);
             }
         }
     }
 
     // Head: pred = d . w + b per voxel; in training also the L1 loss and its
-    // gradients (dd = g w, dw += g d, db += g with g = sign(pred - target) / N).
+    // gradients (dd = g w through the ReLU that d comes from, dw += g d, db += g with g =
+    // sign(pred - target) / N).
     template <int C0>
     __global__ void headKernel(const __nv_bfloat16* __restrict__ d, const float* __restrict__ hw, size_t nvox,
         const float* __restrict__ target, float invN, float* __restrict__ pred, double predScale,
@@ -722,7 +734,7 @@ namespace {
 #pragma unroll
                 for (int c = 0; c < C0; ++c) {
                     gw[c] = fmaf(g, x[c], gw[c]);
-                    o[c] = g * w[c];
+                    o[c] = x[c] > 0.0f ? g * w[c] : 0.0f;
                 }
                 uint4* dst = reinterpret_cast<uint4*>(dd + v * C0);
 #pragma unroll
@@ -737,7 +749,12 @@ namespace {
         }
         if (!target)
             return;
-        // warp sums, then one atomic per warp
+        // warp sums, block sums, then one atomic per block and sum: the addresses are the same
+        // for all, and one atomic per warp held the pass (8 x 64^3 voxels: 196 -> 38 us).  The
+        // bias' own sum stays at an atomic per warp: its terms are all +-invN, round alike,
+        // and in coarser steps it comes out up to 3e-5 of itself elsewhere.
+        __shared__ float part[8][C0 + 1];
+        const int warp = threadIdx.x >> 5;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             gb += __shfl_xor_sync(0xffffffffu, gb, o);
@@ -749,9 +766,19 @@ namespace {
         if ((threadIdx.x & 31) == 0) {
 #pragma unroll
             for (int c = 0; c < C0; ++c)
-                atomicAdd(dhw + c, gw[c]);
+                part[warp][c] = gw[c];
+            part[warp][C0] = loss;
             atomicAdd(dhw + C0, gb);
-            atomicAdd(lossSum, static_cast<double>(loss));
+        }
+        __syncthreads();
+        if (threadIdx.x < C0 + 1) {
+            float v = 0.0f;
+            for (int w = 0; w < 8; ++w)
+                v += part[w][threadIdx.x];
+            if (threadIdx.x < C0)
+                atomicAdd(dhw + threadIdx.x, v);
+            else
+                atomicAdd(lossSum, static_cast<double>(v));
         }
     }
 
@@ -781,17 +808,19 @@ namespace {
             pb[i] = __float2bfloat16_rn(p[i]);
     }
 
-    // dgrad weights: Wt[ci][t][co] = W[co][26 - t][ci]
+    // dgrad weights of every layer: Wt[ci][t][co] = W[co][26 - t][ci]
     __global__ void transposeWeightsKernel(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt,
-        int Cout, int Cin)
+        const LayerTable layers)
     {
-        const size_t n = static_cast<size_t>(Cout) * 27 * Cin;
-        for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
-             i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-            const int co = static_cast<int>(i % Cout);
-            const int t = static_cast<int>((i / Cout) % 27);
-            const int ci = static_cast<int>(i / (static_cast<size_t>(Cout) * 27));
-            wt[i] = w[(static_cast<size_t>(co) * 27 + (26 - t)) * Cin + ci];
+        for (int k = static_cast<int>(blockIdx.y); k < layers.n; k += static_cast<int>(gridDim.y)) {
+            const int Cout = layers.cout[k], Cin = layers.cin[k];
+            const __nv_bfloat16* const src = w + layers.w[k];
+            __nv_bfloat16* const dst = wt + layers.wt[k];
+            const int n = Cout * 27 * Cin;
+            for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+                const int co = i % Cout, t = (i / Cout) % 27, ci = i / (Cout * 27);
+                dst[i] = src[(co * 27 + (26 - t)) * Cin + ci];
+            }
         }
     }
 
@@ -930,7 +959,7 @@ cudaError_t conv3Configure()
 }
 
 cudaError_t launchConv3(const ConvIn& in, int B, int D, int H, int W, int Cin, const __nv_bfloat16* w,
-    const float* bias, int Cout, bool relu, __nv_bfloat16* out, cudaStream_t s)
+    const float* bias, int Cout, bool relu, __nv_bfloat16* out, cudaStream_t s, const __nv_bfloat16* mask)
 {
     if (Cin % 16 || Cout % 16 || (in.ca % 16) || (in.b && in.cb % 16) || in.ca + (in.b ? in.cb : 0) != Cin)
         return cudaErrorInvalidValue;
@@ -944,19 +973,19 @@ cudaError_t launchConv3(const ConvIn& in, int B, int D, int H, int W, int Cin, c
         && static_cast<size_t>(B) * D * H * W < (1ull << 31)) {
         const int small = B * ((D + 1) / 2) * ((H + 3) / 4) * ((W + 7) / 8);
         conv3SmallKernel<<<dim3(small, Cout / 16), 128, kSmallStages * kSmallStage, s>>>(in, D, H, W, Cin, w, bias,
-            Cout, relu ? 1 : 0, out);
+            Cout, relu ? 1 : 0, out, mask);
     } else if (Cout % 32 == 0) {
         conv3Kernel<32><<<dim3(bricks, Cout / 32), 256, conv3SmemBytes(32), s>>>(in, D, H, W, Cin, w, bias, Cout,
-            relu ? 1 : 0, out);
+            relu ? 1 : 0, out, mask);
     } else {
         conv3Kernel<16><<<dim3(bricks, Cout / 16), 256, conv3SmemBytes(16), s>>>(in, D, H, W, Cin, w, bias, Cout,
-            relu ? 1 : 0, out);
+            relu ? 1 : 0, out, mask);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launchWgrad(const ConvIn& in, const __nv_bfloat16* dz, int B, int D, int H, int W, int Cin, int Cout,
-    float* dW, cudaStream_t s)
+    float* dW, float* db, cudaStream_t s)
 {
     if (Cin % 16 || Cout % 16)
         return cudaErrorInvalidValue;
@@ -965,18 +994,7 @@ cudaError_t launchWgrad(const ConvIn& in, const __nv_bfloat16* dz, int B, int D,
     // one CTA an SM: as many per tile as fill the SMs once
     const int gx = std::max(1, std::min(bricks, smCount() / tiles));
     wgradKernel<<<dim3(gx, Cout / 16, Cin / 16), kWgradThreads, 3 * kWgradStage, s>>>(in, dz, D, H, W, Cin, Cout,
-        bricks, dW);
-    return cudaGetLastError();
-}
-
-cudaError_t launchReluBackward(const __nv_bfloat16* dy, const __nv_bfloat16* y, __nv_bfloat16* dz, size_t nvox,
-    int C, float* db, cudaStream_t s)
-{
-    if (C % 8 || 256 % (C / 8))
-        return cudaErrorInvalidValue;
-    const size_t items = nvox * (C / 8);
-    reluBackwardKernel<<<grid1d(items), 256, 0, s>>>(reinterpret_cast<const uint4*>(dy),
-        reinterpret_cast<const uint4*>(y), reinterpret_cast<uint4*>(dz), items, C / 8, db);
+        bricks, dW, db);
     return cudaGetLastError();
 }
 
@@ -990,13 +1008,14 @@ cudaError_t launchAvgPool(const __nv_bfloat16* x, __nv_bfloat16* out, int B, int
 }
 
 cudaError_t launchSplitConcatGrad(const __nv_bfloat16* dcat, int cu, int cs, const __nv_bfloat16* dxNext,
-    __nv_bfloat16* du, __nv_bfloat16* de, int B, int D, int H, int W, cudaStream_t s)
+    const __nv_bfloat16* yu, __nv_bfloat16* du, const __nv_bfloat16* ye, __nv_bfloat16* de, int B, int D, int H, int W,
+    cudaStream_t s)
 {
     const size_t items = (du ? static_cast<size_t>(B) * (D / 2) * (H / 2) * (W / 2) * (cu / 8) : 0)
         + (de ? static_cast<size_t>(B) * D * H * W * (cs / 8) : 0);
     splitConcatGradKernel<<<grid1d(items), 256, 0, s>>>(reinterpret_cast<const uint4*>(dcat), cu / 8, cs / 8,
-        reinterpret_cast<const uint4*>(dxNext), reinterpret_cast<uint4*>(du), reinterpret_cast<uint4*>(de), B, D, H,
-        W);
+        reinterpret_cast<const uint4*>(dxNext), reinterpret_cast<const uint4*>(yu), reinterpret_cast<uint4*>(du),
+        reinterpret_cast<const uint4*>(ye), reinterpret_cast<uint4*>(de), B, D, H, W);
     return cudaGetLastError();
 }
 
@@ -1027,9 +1046,10 @@ cudaError_t launchToBf16(const float* p, __nv_bfloat16* pb, size_t n, cudaStream
     return cudaGetLastError();
 }
 
-cudaError_t launchTransposeWeights(const __nv_bfloat16* w, __nv_bfloat16* wt, int Cout, int Cin, cudaStream_t s)
+cudaError_t launchTransposeWeights(const __nv_bfloat16* w, __nv_bfloat16* wt, const LayerTable& layers,
+    cudaStream_t s)
 {
-    transposeWeightsKernel<<<grid1d(static_cast<size_t>(Cout) * 27 * Cin), 256, 0, s>>>(w, wt, Cout, Cin);
+    transposeWeightsKernel<<<dim3(smCount(), std::max(1, layers.n)), 256, 0, s>>>(w, wt, layers);
     return cudaGetLastError();
 }
 
