@@ -5,12 +5,12 @@
 // transposed, flipped weights) of channels-last bf16 tensors as an implicit GEMM on
 // the tensor cores.  A CTA computes an output brick of 8 (x) x 16 (y) x ZT (z)
 // voxels and NT output channels.  Per 16-channel input slice it stages
-//   * the zero-padded input halo of 10 x 18 x (ZT + 2) voxels as two planes, one per
-//     8-channel half: voxel (hz, hy, hx) of half h at h * plane + ((hz*18 + hy)*10 + hx)*16,
+//   * the zero-padded input halo of 10 x 18 x (ZT + 2) voxels, voxel (hz, hy, hx) at
+//     ((hz*18 + hy)*10 + hx)*32 in the 32-byte swizzle (halves by address bit 7),
 //   * the slice's weights of all 27 taps, the three z-taps of each in-plane tap
 //     q = 3 (dy + 1) + (dx + 1) stacked along N: row n = (1 - dz) * NT + co of the
-//     B operand of q, half h, at q * 3*NT*32 + h * 3*NT*16 + n * 16,
-// (no swizzle, K-major), so that the A operand of a tap is the halo seen through a
+//     B operand of q, half h, at q * 3*NT*32 + h * 3*NT*16 + n * 16 (no swizzle),
+// both K-major, so that the A operand of a tap is the halo seen through a
 // descriptor: row r = 8 y + x of halo plane hz reads halo voxel (hz, y + dy + 1,
 // x + dx + 1): 8 consecutive x are 256 bytes, consecutive y 320 bytes apart (SBO); the
 // swizzle goes by the address, whichever voxel the tap starts at.
@@ -44,6 +44,7 @@
 
 #include "denoiser.hpp"
 #include "engine.hpp"
+#include "tensor_map.hpp"
 #include "umma.cuh"
 
 namespace dxmcg {
@@ -691,25 +692,6 @@ namespace {
         return fn;
     }
 
-    // 5-D map (C, W, H, D, B) of a channels-last bf16 tensor with a halo box
-    // (16, 10, 18, hz, 1) in the 32-byte swizzle; false if it cannot be made (the kernel then uses cp.async)
-    bool haloTensorMap(CUtensorMap* m, const void* base, int B, int D, int H, int W, int C, int hz)
-    {
-        const auto encode = tensorMapEncoder();
-        if (!encode || !base || (reinterpret_cast<uintptr_t>(base) & 15u))
-            return false;
-        const cuuint64_t dims[5] = { static_cast<cuuint64_t>(C), static_cast<cuuint64_t>(W),
-            static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(B) };
-        const cuuint64_t row = static_cast<cuuint64_t>(C) * 2;
-        const cuuint64_t strides[4] = { row, row * W, row * W * H, row * W * H * D };
-        const cuuint32_t box[5] = { 16, 10, 18, static_cast<cuuint32_t>(hz), 1 };
-        const cuuint32_t step[5] = { 1, 1, 1, 1, 1 };
-        return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, step,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
-            == CUDA_SUCCESS;
-    }
-
     template <int NT>
     cudaError_t launchTc(const nn::ConvIn& in, int B, int D, int H, int W, int Cin, const __nv_bfloat16* w,
         const float* bias, int Cout, bool relu, __nv_bfloat16* out, cudaStream_t s, const nn::ConvOptions& ep)
@@ -720,9 +702,9 @@ namespace {
         CUtensorMap mapA {}, mapB {};
         bool tma = true;
         if (in.a && !in.halfA)
-            tma = haloTensorMap(&mapA, in.a, B, D, H, W, in.ca, S::HZ);
+            tma = nn::brickTensorMap(&mapA, in.a, B, D, H, W, in.ca, 10, 18, S::HZ);
         if (tma && in.b)
-            tma = haloTensorMap(&mapB, in.b, B, D, H, W, in.cb, S::HZ);
+            tma = nn::brickTensorMap(&mapB, in.b, B, D, H, W, in.cb, 10, 18, S::HZ);
         // one persistent CTA per SM and output-channel tile, never more than bricks
         static const int sms = [] {
             int dev = 0, n = 0;
@@ -851,6 +833,29 @@ namespace {
 } // namespace
 
 namespace nn {
+    bool brickTensorMap(CUtensorMap* m, const void* base, int B, int D, int H, int W, int C, int bx, int by, int bz)
+    {
+        const auto encode = tensorMapEncoder();
+        if (!encode || !base || (reinterpret_cast<uintptr_t>(base) & 15u))
+            return false;
+        const cuuint64_t dims[5] = { static_cast<cuuint64_t>(C), static_cast<cuuint64_t>(W),
+            static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(B) };
+        const cuuint64_t row = static_cast<cuuint64_t>(C) * 2;
+        const cuuint64_t strides[4] = { row, row * W, row * W * H, row * W * H * D };
+        const cuuint32_t box[5] = { 16, static_cast<cuuint32_t>(bx), static_cast<cuuint32_t>(by),
+            static_cast<cuuint32_t>(bz), 1 };
+        const cuuint32_t step[5] = { 1, 1, 1, 1, 1 };
+        return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, step,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
+            == CUDA_SUCCESS;
+    }
+
+    cudaError_t convErrorFlags(unsigned** flags)
+    {
+        return cudaGetSymbolAddress(reinterpret_cast<void**>(flags), g_convTcError);
+    }
+
     cudaError_t conv3TcConfigure()
     {
         // the whole unified L1 / shared array as shared memory (one CTA per SM, with up to

@@ -155,16 +155,14 @@ int conv(dxmcg_denoiser* d, int k, const nn::ConvIn& in, int l, bf16* out, cudaS
     return DXMCG_OK;
 }
 
-// DXMCG_OK unless a tcgen05 convolution gave up waiting for its tensor-core work
-// (the kernel then skipped its output); call after a synchronisation
-int tensorCoreStatus(dxmcg_denoiser* d)
+// DXMCG_OK unless a tcgen05 convolution or a weight gradient gave up waiting for its copies
+// or tensor-core work (its output is then wrong); call after a synchronisation
+int tensorCoreStatus()
 {
-    if (!d->tensorCores)
-        return DXMCG_OK;
     unsigned flags = 0;
     NN_CUDA(nn::conv3TcErrors(&flags));
     if (flags)
-        return fail(DXMCG_ERR_DEVICE, "denoiser: a tensor-core convolution timed out waiting for its MMAs");
+        return fail(DXMCG_ERR_DEVICE, "denoiser: a tensor-core convolution timed out waiting for its copies or MMAs");
     return DXMCG_OK;
 }
 
@@ -618,7 +616,7 @@ namespace nn {
         if (hostOut)
             NN_CUDA(cudaMemcpyAsync(hostOut, d->worldOut.p, n * sizeof(double), cudaMemcpyDeviceToHost, s));
         NN_CUDA(cudaStreamSynchronize(s));
-        return tensorCoreStatus(d);
+        return tensorCoreStatus();
     }
 } // namespace nn
 } // namespace dxmcg
@@ -806,7 +804,7 @@ DXMCG_API int dxmcg_denoiser_backward(dxmcg_denoiser* d, const void* input, cons
         NN_CUDA(cudaMemcpyAsync(&h, d->loss.p, sizeof(double), cudaMemcpyDeviceToHost, s));
         NN_CUDA(cudaStreamSynchronize(s));
         *loss = h / static_cast<double>(d->nvox(0));
-        if ((rc = tensorCoreStatus(d)) != DXMCG_OK)
+        if ((rc = tensorCoreStatus()) != DXMCG_OK)
             return rc;
     }
     return DXMCG_OK;

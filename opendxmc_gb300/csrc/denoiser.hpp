@@ -26,6 +26,8 @@ struct ConvIn {
 
 size_t conv3SmemBytes(int nt);
 cudaError_t conv3Configure(); // opt the kernels into their shared-memory size (once per device)
+cudaError_t wgradConfigure(); // the same for launchWgrad's (conv3Configure calls it)
+int smCount();                // of the current device
 
 // Options of the tcgen05 convolution beyond launchConv3's:
 //   list:   device array of output-brick indices (conv3TcBrickDims, x fastest, then y,
@@ -60,6 +62,7 @@ cudaError_t conv3TcConfigure();
 cudaError_t launchConv3Tc(const ConvIn& in, int B, int D, int H, int W, int Cin, const __nv_bfloat16* w,
     const float* bias, int Cout, bool relu, __nv_bfloat16* out, cudaStream_t s, const ConvOptions* ep = nullptr);
 cudaError_t conv3TcErrors(unsigned* flags);
+cudaError_t convErrorFlags(unsigned** flags); // where kernels set what conv3TcErrors reads
 // CTAs of the tcgen05 launch for this shape (a grid under one CTA per SM leaves the
 // tensor cores of the other SMs idle: the caller then takes launchConv3)
 int conv3TcCtas(int B, int D, int H, int W, int Cout);

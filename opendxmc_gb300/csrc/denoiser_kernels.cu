@@ -53,12 +53,6 @@ namespace {
                      : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
                      : "r"(addr));
     }
-    __device__ __forceinline__ void ldsm4t(unsigned addr, unsigned& r0, unsigned& r1, unsigned& r2, unsigned& r3)
-    {
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                     : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                     : "r"(addr));
-    }
     // D = A (16x16, row) * B (16x8, col) + D, bf16 inputs, f32 accumulators
     __device__ __forceinline__ void mma16816(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
         unsigned b0, unsigned b1)
@@ -370,196 +364,6 @@ namespace {
                     v1 = fmaxf(v1, 0.0f);
                 }
                 storePair(out, mask, at + 8 * j, v0, v1);
-            }
-        }
-    }
-
-    // ------------------------------------------------------------------ weight gradient
-    // dW[co][tap][ci] += sum over output voxels v of dz[v][co] * x[v + off(tap)][ci].
-    // and db[co] += sum of dz[v][co] (by the CTAs of input slice 0, from the same fragments).
-    // grid: x = CTAs looping over bricks, y = 16-output-channel tile, z = input slice.
-    //
-    // bf16 mma.sync with the voxels as the K dimension (for tcgen05 the channel counts, 16
-    // at level 0, would be M and N: a quarter of its narrowest tile).  Its rate, one
-    // m16n8k16 per two cycles and SM, is the bound to reach, and shared memory must not
-    // stand before it.  So warp (p, g) owns the nine taps of z-plane p and the brick's
-    // z-slices 2 g, 2 g + 1: a 16-voxel step (two rows of 8) multiplies one fragment of dz
-    // with 9 x 2 fragments of x, and of the four halo rows those need, two stay in
-    // registers from the step before: 4 ldmatrix.x4 for 18 MMAs.  (One tap a warp and step,
-    // re-reading dz for each tap, took 2 for 2.)  Bricks arrive through three cp.async stages;
-    // the four z-groups' sums meet in shared memory and leave by one atomic per weight and
-    // CTA.  8 x 64^3 voxels: 16 to 16 channels 190 -> 92 us (48 at the MMA rate), 48 to 16
-    // 794 -> 271 us; with two stages 95 and 281 us.
-    __device__ __forceinline__ float pairSum(unsigned p) // of two bf16
-    {
-        return __uint_as_float(p << 16) + __uint_as_float(p & 0xffff0000u);
-    }
-
-    constexpr int kWgradThreads = 384;
-    constexpr int kWgradStage = kHaloBytes + 512 * 32;
-
-    __global__ void __launch_bounds__(kWgradThreads, 1) wgradKernel(const ConvIn in,
-        const __nv_bfloat16* __restrict__ dz, int D, int H, int W, int Cin, int Cout, int nBricks,
-        float* __restrict__ dW, float* __restrict__ db)
-    {
-        extern __shared__ __align__(128) unsigned char smem[];
-        const int n0 = blockIdx.y * 16;
-        const int c0 = blockIdx.z * 16;
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int q = lane >> 3, r = lane & 7;
-        const int plane = warp % 3, group = warp / 3;
-
-        // this thread's copies of a brick, 16 bytes each: halo voxels (tid >> 1) + 192 k and
-        // output voxels (tid >> 1) + 192 k, half tid & 1.  A brick starts on a multiple of 8
-        // on each axis, so their offsets from its first voxel, in a half-resolution input
-        // too, are the same for every brick.
-        constexpr int kXCopies = (2 * kHaloVox + kWgradThreads - 1) / kWgradThreads;
-        constexpr int kZCopies = (2 * 512 + kWgradThreads - 1) / kWgradThreads;
-        const int tid = static_cast<int>(threadIdx.x), h = tid & 1;
-        const bool inA = c0 < in.ca;
-        const int cs = inA ? in.ca : in.cb;
-        const __nv_bfloat16* const xSrc = (inA ? in.a + c0 : in.b + (c0 - in.ca)) + h * 8;
-        const int sh = inA && in.halfA ? 1 : 0;
-        const int Ds = D >> sh, Hs = H >> sh, Ws = W >> sh;
-        int xRel[kXCopies];
-        unsigned xAt[kXCopies]; // hz, hy, hx
-#pragma unroll
-        for (int k = 0; k < kXCopies; ++k) {
-            const int v = (tid >> 1) + (kWgradThreads / 2) * k;
-            const int hz = v / 100, hy = (v / 10) % 10, hx = v % 10;
-            // (hz - 1) >> 1 rounds down, as the voxel's own index shifted does
-            xRel[k] = (((hz - 1) >> sh) * Hs + ((hy - 1) >> sh)) * Ws + ((hx - 1) >> sh);
-            xAt[k] = static_cast<unsigned>(hz | hy << 8 | hx << 16);
-        }
-        const auto load = [&](int brick, int stage) {
-            const unsigned base = smemAddr(smem + stage * kWgradStage);
-            const BrickPos p = brickOf(brick, D, H, W);
-            const long long x0 = ((static_cast<long long>(p.b) * Ds + (p.z0 >> sh)) * Hs + (p.y0 >> sh)) * Ws
-                + (p.x0 >> sh);
-#pragma unroll
-            for (int k = 0; k < kXCopies; ++k) {
-                const int v = (tid >> 1) + (kWgradThreads / 2) * k;
-                if (k == kXCopies - 1 && v >= kHaloVox)
-                    break;
-                const int hx = static_cast<int>(xAt[k] >> 16);
-                const bool ok = static_cast<unsigned>(p.z0 - 1 + static_cast<int>(xAt[k] & 0xffu))
-                        < static_cast<unsigned>(D)
-                    && static_cast<unsigned>(p.y0 - 1 + static_cast<int>(xAt[k] >> 8 & 0xffu))
-                        < static_cast<unsigned>(H)
-                    && static_cast<unsigned>(p.x0 - 1 + hx) < static_cast<unsigned>(W);
-                cpAsync16(base + v * 32 + ((h ^ (hx >> 2 & 1)) << 4), ok ? xSrc + (x0 + xRel[k]) * cs : xSrc, ok);
-            }
-            const long long z0 = ((static_cast<long long>(p.b) * D + p.z0) * H + p.y0) * W + p.x0;
-#pragma unroll
-            for (int k = 0; k < kZCopies; ++k) {
-                const int v = (tid >> 1) + (kWgradThreads / 2) * k;
-                if (k == kZCopies - 1 && v >= 512)
-                    break;
-                const int z = v >> 6, y = v >> 3 & 7, x = v & 7;
-                const bool ok = p.z0 + z < D && p.y0 + y < H && p.x0 + x < W;
-                cpAsync16(base + kHaloBytes + v * 32 + ((h ^ (v >> 2 & 1)) << 4),
-                    ok ? dz + (z0 + (z * H + y) * W + x) * Cout + n0 + h * 8 : dz, ok);
-            }
-        };
-
-        float acc[9][2][4];
-#pragma unroll
-        for (int t = 0; t < 9; ++t)
-#pragma unroll
-            for (int n = 0; n < 2; ++n)
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    acc[t][n][k] = 0.0f;
-
-        const bool bias = blockIdx.z == 0 && plane == 0;
-        float sb[2] = { 0.0f, 0.0f }; // dz of output channels lane / 4 and lane / 4 + 8
-        // this lane's addresses: x rows (halo row q >> 1, voxel r + dx, half q & 1) and dz rows
-        // (row q >> 1 of the step, voxel r, half q & 1)
-        unsigned xOff[3];
-#pragma unroll
-        for (int dx = 0; dx < 3; ++dx) {
-            const int hx = r + dx;
-            xOff[dx] = static_cast<unsigned>(((q >> 1) * 10 + hx) * 32 + (((q & 1) ^ ((hx >> 2) & 1)) << 4));
-        }
-        const unsigned zOff = static_cast<unsigned>(
-            kHaloBytes + (((q >> 1) << 3) + r) * 32 + (((q & 1) ^ ((r >> 2) & 1)) << 4));
-
-        // stage i mod 3 holds the CTA's brick i; brick i + 2 loads over brick i - 1, which
-        // the barrier tells every warp is done with
-        const int first = static_cast<int>(blockIdx.x), hop = static_cast<int>(gridDim.x);
-        for (int i = 0; i < 2; ++i) {
-            if (first + i * hop < nBricks)
-                load(first + i * hop, i);
-            cpAsyncCommit();
-        }
-        for (int brick = first, stage = 0; brick < nBricks; brick += hop, stage = stage == 2 ? 0 : stage + 1) {
-            cpAsyncWait<1>();
-            __syncthreads();
-            if (brick + 2 * hop < nBricks)
-                load(brick + 2 * hop, stage == 0 ? 2 : stage - 1);
-            cpAsyncCommit();
-            const unsigned base = smemAddr(smem + stage * kWgradStage);
-#pragma unroll 1
-            for (int s = 0; s < 2; ++s) {
-                const int z = 2 * group + s;
-                const unsigned xBase = base + (z + plane) * (100 * 32);
-                const unsigned zBase = base + zOff + z * (64 * 32);
-                unsigned b[4][3][2]; // halo rows (rotating), dx, channel half
-                const auto rows = [&](int hy) { // halo rows hy and hy + 1
-#pragma unroll
-                    for (int dx = 0; dx < 3; ++dx)
-                        ldsm4t(xBase + xOff[dx] + hy * 320, b[hy & 3][dx][0], b[hy & 3][dx][1],
-                            b[(hy + 1) & 3][dx][0], b[(hy + 1) & 3][dx][1]);
-                };
-                rows(0);
-#pragma unroll
-                for (int yb = 0; yb < 8; yb += 2) {
-                    rows(yb + 2);
-                    unsigned a0, a1, a2, a3;
-                    ldsm4t(zBase + yb * 256, a0, a1, a2, a3);
-                    if (bias) {
-                        sb[0] += pairSum(a0) + pairSum(a2);
-                        sb[1] += pairSum(a1) + pairSum(a3);
-                    }
-#pragma unroll
-                    for (int t = 0; t < 9; ++t) {
-                        const int dy = t / 3, dx = t % 3;
-                        const int r0 = (yb + dy) & 3, r1 = (yb + dy + 1) & 3;
-                        mma16816(acc[t][0], a0, a1, a2, a3, b[r0][dx][0], b[r1][dx][0]);
-                        mma16816(acc[t][1], a0, a1, a2, a3, b[r0][dx][1], b[r1][dx][1]);
-                    }
-                }
-            }
-        }
-
-        // the z-groups' sums, one group after the other, then one atomic a weight
-        float* sum = reinterpret_cast<float*>(smem); // [16 co][27 taps][16 ci]
-        cpAsyncWait<0>();
-        const int g = lane >> 2, tq = lane & 3;
-        for (int turn = 0; turn < 4; ++turn) {
-            __syncthreads();
-            if (group != turn)
-                continue;
-#pragma unroll
-            for (int t = 0; t < 9; ++t)
-#pragma unroll
-                for (int n = 0; n < 2; ++n)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        float* w = sum + ((g + ((k >> 1) << 3)) * 27 + 9 * plane + t) * 16 + n * 8 + 2 * tq + (k & 1);
-                        *w = turn ? *w + acc[t][n][k] : acc[t][n][k];
-                    }
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < 16 * 27 * 16; i += kWgradThreads)
-            atomicAdd(dW + static_cast<size_t>(n0 * 27 + (i >> 4)) * Cin + c0 + (i & 15), sum[i]);
-        if (bias) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                sb[j] += __shfl_xor_sync(0xffffffffu, sb[j], 1);
-                sb[j] += __shfl_xor_sync(0xffffffffu, sb[j], 2);
-                if (tq == 0)
-                    atomicAdd(db + n0 + g + 8 * j, sb[j]);
             }
         }
     }
@@ -925,14 +729,6 @@ namespace {
         }
     }
 
-    int smCount()
-    {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        return sms > 0 ? sms : 1;
-    }
-
     int grid1d(size_t items)
     {
         const size_t blocks = (items + 255) / 256;
@@ -940,6 +736,14 @@ namespace {
         return static_cast<int>(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
     }
 } // namespace
+
+int smCount()
+{
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
+}
 
 size_t conv3SmemBytes(int nt) { return 2 * static_cast<size_t>(kHaloBytes + 27 * nt * 32); }
 
@@ -954,7 +758,7 @@ cudaError_t conv3Configure()
         e = cudaFuncSetAttribute(conv3SmallKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
             kSmallStages * kSmallStage);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(wgradKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * kWgradStage);
+        e = wgradConfigure();
     return e;
 }
 
@@ -981,20 +785,6 @@ cudaError_t launchConv3(const ConvIn& in, int B, int D, int H, int W, int Cin, c
         conv3Kernel<16><<<dim3(bricks, Cout / 16), 256, conv3SmemBytes(16), s>>>(in, D, H, W, Cin, w, bias, Cout,
             relu ? 1 : 0, out, mask);
     }
-    return cudaGetLastError();
-}
-
-cudaError_t launchWgrad(const ConvIn& in, const __nv_bfloat16* dz, int B, int D, int H, int W, int Cin, int Cout,
-    float* dW, float* db, cudaStream_t s)
-{
-    if (Cin % 16 || Cout % 16)
-        return cudaErrorInvalidValue;
-    const int bricks = B * ((D + 7) / 8) * ((H + 7) / 8) * ((W + 7) / 8);
-    const int tiles = (Cout / 16) * (Cin / 16);
-    // one CTA an SM: as many per tile as fill the SMs once
-    const int gx = std::max(1, std::min(bricks, smCount() / tiles));
-    wgradKernel<<<dim3(gx, Cout / 16, Cin / 16), kWgradThreads, 3 * kWgradStage, s>>>(in, dz, D, H, W, Cin, Cout,
-        bricks, dW, db);
     return cudaGetLastError();
 }
 
