@@ -135,9 +135,9 @@ namespace {
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n));
     }
 
-    template <int NT>
+    template <int NT, int ZT_>
     struct ConvTcShape {
-        static constexpr int ZT = NT == 64 ? 4 : 8;          // output z-slices per brick
+        static constexpr int ZT = ZT_;                       // output z-slices per brick
         static constexpr int HZ = ZT + 2, HY = 18, HX = 10;  // halo extent
         static constexpr int kVox = HZ * HY * HX;
         static constexpr uint32_t kHalo = kVox * 32;         // one halo buffer (two in the pipeline)
@@ -204,8 +204,8 @@ namespace {
     //   * warps 1-7 (producers) stage item i into stage i mod S once the MMAs of the
     //     item that used it before released it (S = 2 or 3 stages, a launch parameter):
     //     the halo by TMA (completing on tmaFull) or by their own copies / upsampling
-    //     expansion, and the slice's weights unless every slice's weights stay resident;
-    //     then they arrive on full[stage].  The expansion is what they are many for: 48 (32
+    //     expansion, and the slice's weights (where every slice's stay resident: with the
+    //     first brick only); then they arrive on full[stage].  The expansion is what they are many for: 48 (32
     //     upsampled) to 16 channels took 924 us with three such warps, 580 with seven;
     //   * warps 8-11 (one TMEM lane quarter each) wait for accFull, read the brick's sums
     //     back (bias, ReLU, bf16 store), zero them and arrive on accEmpty[set].
@@ -217,15 +217,14 @@ namespace {
     constexpr int kConvThreads = 384;
     constexpr uint32_t kPolls = 1u << 24;
 
-    template <int NT, bool MASK>
+    template <int NT, int ZT, bool MASK>
     __global__ void __launch_bounds__(kConvThreads, 1) conv3TcKernel(const nn::ConvIn in, int D, int H, int W, int Cin,
         const __nv_bfloat16* __restrict__ wgt, const float* __restrict__ bias, int Cout, int relu,
         __nv_bfloat16* __restrict__ out, const __grid_constant__ CUtensorMap mapA,
         const __grid_constant__ CUtensorMap mapB, int useTma, int tiles, int weightsResident, int stages,
         const nn::ConvOptions ep)
     {
-        using S = ConvTcShape<NT>;
-        constexpr int ZT = S::ZT;
+        using S = ConvTcShape<NT, ZT>;
         extern __shared__ __align__(256) unsigned char smemRaw[];
         __shared__ __align__(8) uint64_t full[S::kMaxStages];    // producers' copies of stage b visible
         __shared__ __align__(8) uint64_t tmaFull[S::kMaxStages]; // the TMA halo of stage b landed
@@ -282,26 +281,18 @@ namespace {
             umma::storeWait();
         }
 
-        // a slice's weights for all taps, z-taps stacked per in-plane tap (cp.async by the
-        // threads [first, first + count))
-        const auto stageWeights = [&](int sl, uint32_t dst, int first, int count) {
-            const int c0 = sl * 16;
-            for (int i = t - first; i < 27 * NT * 2; i += count) {
-                const int co = i % NT, th = i / NT; // th = tap * 2 + h, tap = 9 (dz + 1) + q
-                const int tap = th >> 1, h = th & 1;
-                const int dz1 = tap / 9, q = tap - 9 * dz1;
-                const bool valid = n0 + co < Cout;
-                const __nv_bfloat16* src
-                    = valid ? wgt + ((static_cast<size_t>(n0 + co) * 27 + tap) * Cin + c0 + h * 8) : wgt;
-                cpAsync16(dst + q * S::kStackBytes + h * (3 * NT * 16) + ((2 - dz1) * NT + co) * 16, src, valid);
+        // a slice's weights for all taps, z-taps stacked per in-plane tap, from the prepared
+        // weights: 54 blocks (in-plane tap, channel half, z-tap) of NT contiguous rows.  From
+        // the weights as they are stored each 16 bytes were a sector of their own: a brick of
+        // 12 slices of 8 x 16 x 2 voxels and 16 channels took 24 us, this way 21, and the
+        // network on 200 x 264 x 232 voxels 2105 -> 2011 us.  (A bulk copy per block takes ~80
+        // cycles, whatever its size: 35 us.)
+        const auto stageWeights = [&](int sl, uint32_t dst) {
+            for (int i = t - 32; i < 54 * NT; i += kProducers) {
+                const int blk = i / NT, row = i % NT; // dst: blocks in order, a stack is six
+                cpAsync16(dst + i * 16, wgt + ((static_cast<size_t>(sl) * 54 + blk) * Cout + n0 + row) * 8, true);
             }
         };
-        if (weightsResident) {
-            for (int sl = 0; sl < nSlices; ++sl)
-                stageWeights(sl, wbase + sl * S::kWeights, 0, kConvThreads);
-            asm volatile("cp.async.commit_group;\n" ::);
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        }
         umma::fenceProxyAsync();
         umma::fenceBeforeSync();
         __syncthreads();
@@ -404,11 +395,13 @@ namespace {
                 const bool half = inA && in.halfA;
                 const uint32_t dst = sbase + b * S::kHalo;
                 unsigned char* dstp = smem + b * S::kHalo;
+                // resident weights arrive with the first brick's items
+                if (!weightsResident || it < nSlices)
+                    stageWeights(sl, wbase + (weightsResident ? sl : b) * S::kWeights);
                 if (byTma(sl)) {
                     if (pt == 0) {
-                        const CUtensorMap* m = inA ? &mapA : &mapB;
                         umma::mbarArriveExpectTx(&tmaFull[b], S::kHalo);
-                        umma::tmaLoad5d(dst, m, cc, p.x0 - 1, p.y0 - 1, p.z0 - 1, p.b, &tmaFull[b]);
+                        umma::tmaLoad5d(dst, inA ? &mapA : &mapB, cc, p.x0 - 1, p.y0 - 1, p.z0 - 1, p.b, &tmaFull[b]);
                         tmaPending |= 1u << b;
                     }
                 } else if (half) {
@@ -470,8 +463,6 @@ namespace {
                         cpAsync16(dst + haloOffset(v, h), q, inside);
                     }
                 }
-                if (!weightsResident)
-                    stageWeights(sl, wbase + b * S::kWeights, 32, kProducers);
                 asm volatile("cp.async.commit_group;\n" ::);
                 asm volatile("cp.async.wait_group 0;\n" ::: "memory");
                 umma::fenceProxyAsync(); // generic-proxy writes, read next by the tensor cores
@@ -480,7 +471,7 @@ namespace {
             if (!ok)
                 *abortp = 1;
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-            // a TMA still in flight lands before the memory is given back
+            // a copy still in flight lands before the memory is given back
             if (pt == 0)
                 for (int b = 0; b < stages; ++b)
                     if (tmaPending >> b & 1u)
@@ -508,18 +499,19 @@ namespace {
                 const int y = p.y0 + (row >> 3), x = p.x0 + (row & 7);
                 const bool inPlane = y < H && x < W;
                 constexpr int kPairs = (NT / 16) * (ZT / 2);
+                constexpr int kMaskPairs = kPairs < 4 ? kPairs : 4;
                 // ReLU mask: read while the brick's MMAs run and kept as one bit a channel
                 // (read where it is used, it held the input gradient of 16 channels on
                 // 8 x 64^3 voxels at 109 us; unmasked 44, this way 56)
                 uint32_t mk[MASK ? kPairs : 1];
                 if constexpr (MASK) {
 #pragma unroll
-                    for (int i0 = 0; i0 < kPairs; i0 += 4) {
+                    for (int i0 = 0; i0 < kPairs; i0 += kMaskPairs) {
                         // all of a batch's loads before the first use (a voxel outside the
                         // volume reads one inside and is not stored)
-                        uint4 m4[8][2];
+                        uint4 m4[2 * kMaskPairs][2];
 #pragma unroll
-                        for (int v = 0; v < 8; ++v) {
+                        for (int v = 0; v < 2 * kMaskPairs; ++v) {
                             const int i = i0 + (v >> 1);
                             const int z = min(p.z0 + 2 * (i % (ZT / 2)) + (v & 1), D - 1);
                             const uint4* q = reinterpret_cast<const uint4*>(ep.mask
@@ -529,7 +521,7 @@ namespace {
                             m4[v][1] = __ldg(q + 1);
                         }
 #pragma unroll
-                        for (int v = 0; v < 8; ++v) {
+                        for (int v = 0; v < 2 * kMaskPairs; ++v) {
                             const __nv_bfloat162* m2 = reinterpret_cast<const __nv_bfloat162*>(m4[v]);
                             const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
                             if ((v & 1) == 0)
@@ -549,7 +541,7 @@ namespace {
                 // two slices of a 16-channel group at a time; the next two are on their way
                 // from TMEM while these are packed and stored
                 const auto pairAddr = [&](int i) { return acc + 2 * (i % (ZT / 2)) * NT + 16 * (i / (ZT / 2)); };
-                static_assert(kPairs % 4 == 0, "");
+                static_assert(kPairs % kMaskPairs == 0 && (kPairs == 1 || kPairs % 2 == 0), "");
                 uint32_t raw[2][2][16];
                 umma::tmemLoad16Start(pairAddr(0), raw[0][0]);
                 umma::tmemLoad16Start(pairAddr(0) + NT, raw[0][1]);
@@ -558,7 +550,7 @@ namespace {
 #pragma unroll 1
                 for (int i0 = 0; i0 < kPairs; i0 += 2) {
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) {
+                    for (int u = 0; u < (kPairs < 2 ? 1 : 2); ++u) {
                         const int i = i0 + u;
                         const int c = 16 * (i / (ZT / 2)), o = 2 * (i % (ZT / 2));
                         umma::loadWait(raw[u][0], raw[u][1]);
@@ -677,6 +669,11 @@ namespace {
         }
     }
 
+    int tilesOf(int B, int D, int H, int W, int zt)
+    {
+        return B * ((D + zt - 1) / zt) * ((H + 15) / 16) * ((W + 7) / 8);
+    }
+
     // cuTensorMapEncodeTiled from the driver, looked up once through the runtime
     PFN_cuTensorMapEncodeTiled_v12000 tensorMapEncoder()
     {
@@ -692,12 +689,12 @@ namespace {
         return fn;
     }
 
-    template <int NT>
+    template <int NT, int ZT>
     cudaError_t launchTc(const nn::ConvIn& in, int B, int D, int H, int W, int Cin, const __nv_bfloat16* w,
         const float* bias, int Cout, bool relu, __nv_bfloat16* out, cudaStream_t s, const nn::ConvOptions& ep)
     {
-        using S = ConvTcShape<NT>;
-        const int tiles = B * ((D + S::ZT - 1) / S::ZT) * ((H + 15) / 16) * ((W + 7) / 8);
+        using S = ConvTcShape<NT, ZT>;
+        const int tiles = tilesOf(B, D, H, W, ZT);
         // tensor maps of the full-resolution inputs (an upsampled a is expanded by the threads)
         CUtensorMap mapA {}, mapB {};
         bool tma = true;
@@ -716,15 +713,15 @@ namespace {
         if (sms <= 0)
             return cudaErrorLaunchOutOfResources;
         const int nSlices = Cin / 16;
-        // resident weights where they fit; two stages (a third, where it fits, measured no
-        // faster on the 512 x 512 x 400 inference: the tensor pipe, not the staging, is the
-        // bound)
-        const bool resident = S::smemFor(nSlices, true, 2) <= S::kMaxSmem;
-        const int stages = 2;
+        // resident weights where they fit and a CTA has several bricks; two stages then (a
+        // third, where it fits, measured no faster on the 512 x 512 x 400 inference: the tensor
+        // pipe, not the staging, is the bound), three for a CTA of one brick
         const int gy = Cout / NT;
         const int gx = std::max(1, std::min(tiles, sms / gy));
+        const bool resident = tiles > gx && S::smemFor(nSlices, true, 2) <= S::kMaxSmem;
+        const int stages = tiles <= gx && S::smemFor(nSlices, resident, 3) <= S::kMaxSmem ? 3 : 2;
         // the mask's registers would spill in the forward pass
-        (ep.mask ? conv3TcKernel<NT, true> : conv3TcKernel<NT, false>)<<<dim3(gx, gy), kConvThreads,
+        (ep.mask ? conv3TcKernel<NT, ZT, true> : conv3TcKernel<NT, ZT, false>)<<<dim3(gx, gy), kConvThreads,
             S::smemFor(nSlices, resident, stages), s>>>(in, D, H, W, Cin, w, bias, Cout, relu ? 1 : 0, out, mapA,
             mapB, tma ? 1 : 0, tiles, resident ? 1 : 0, stages, ep);
         return cudaGetLastError();
@@ -874,9 +871,9 @@ namespace nn {
             if (e == cudaSuccess)
                 e = configure(masked, smem);
         };
-        both(conv3TcKernel<16, false>, conv3TcKernel<16, true>, ConvTcShape<16>::kMaxSmem);
-        both(conv3TcKernel<32, false>, conv3TcKernel<32, true>, ConvTcShape<32>::kMaxSmem);
-        both(conv3TcKernel<64, false>, conv3TcKernel<64, true>, ConvTcShape<64>::kMaxSmem);
+        both(conv3TcKernel<16, 8, false>, conv3TcKernel<16, 8, true>, ConvTcShape<16, 8>::kMaxSmem);
+        both(conv3TcKernel<32, 8, false>, conv3TcKernel<32, 8, true>, ConvTcShape<32, 8>::kMaxSmem);
+        both(conv3TcKernel<64, 4, false>, conv3TcKernel<64, 4, true>, ConvTcShape<64, 4>::kMaxSmem);
         return e;
     }
 
@@ -891,10 +888,10 @@ namespace nn {
         if ((e.pooled && ((D | H | W) & 1)) || (e.head && Cout != 16))
             return cudaErrorInvalidValue;
         if (Cout % 64 == 0)
-            return launchTc<64>(in, B, D, H, W, Cin, w, bias, Cout, relu, out, s, e);
+            return launchTc<64, 4>(in, B, D, H, W, Cin, w, bias, Cout, relu, out, s, e);
         if (Cout % 32 == 0)
-            return launchTc<32>(in, B, D, H, W, Cin, w, bias, Cout, relu, out, s, e);
-        return launchTc<16>(in, B, D, H, W, Cin, w, bias, Cout, relu, out, s, e);
+            return launchTc<32, 8>(in, B, D, H, W, Cin, w, bias, Cout, relu, out, s, e);
+        return launchTc<16, 8>(in, B, D, H, W, Cin, w, bias, Cout, relu, out, s, e);
     }
 
     int conv3TcCtas(int B, int D, int H, int W, int Cout)
@@ -903,15 +900,15 @@ namespace nn {
             return B * ((D + zt - 1) / zt) * ((H + 15) / 16) * ((W + 7) / 8) * (Cout / nt);
         };
         if (Cout % 64 == 0)
-            return ctas(ConvTcShape<64>::ZT, 64);
+            return ctas(4, 64);
         if (Cout % 32 == 0)
-            return ctas(ConvTcShape<32>::ZT, 32);
-        return ctas(ConvTcShape<16>::ZT, 16);
+            return ctas(8, 32);
+        return ctas(8, 16);
     }
 
     void conv3TcBrickDims(int D, int H, int W, int Cout, int brick[3], int count[3])
     {
-        const int zt = Cout % 64 == 0 ? ConvTcShape<64>::ZT : (Cout % 32 == 0 ? ConvTcShape<32>::ZT : ConvTcShape<16>::ZT);
+        const int zt = Cout % 64 == 0 ? 4 : (Cout % 32 == 0 ? 8 : 8);
         brick[0] = 8;
         brick[1] = 16;
         brick[2] = zt;

@@ -36,7 +36,7 @@ struct dxmcg_denoiser {
     std::vector<Layer> layers;
     size_t head = 0, nParams = 0, nWt = 0;
     DevBuf<float> p, g, m, v;
-    DevBuf<bf16> pb, wt;
+    DevBuf<bf16> pb, wt, pbPrep, wtPrep; // weights, transposed, and both as the tcgen05 kernel reads them
     long step = 0;
     bool configured = false;
     bool tensorCores = true;  // tcgen05 convolutions (else warp-level mma.sync)
@@ -123,7 +123,7 @@ int refreshWeights(dxmcg_denoiser* d, cudaStream_t s)
         t.w[t.n] = ly.w;
         t.wt[t.n++] = ly.wt;
     }
-    NN_CUDA(nn::launchTransposeWeights(d->pb.p, d->wt.p, t, s));
+    NN_CUDA(nn::launchArrangeWeights(d->pb.p, d->wt.p, d->pbPrep.p, d->wtPrep.p, t, s));
     return DXMCG_OK;
 }
 
@@ -147,7 +147,7 @@ int conv(dxmcg_denoiser* d, int k, const nn::ConvIn& in, int l, bf16* out, cudaS
     if (tc) {
         nn::ConvOptions o = ep ? *ep : nn::ConvOptions {};
         o.handoverPolls = d->waitPolls;
-        NN_CUDA(nn::launchConv3Tc(in, d->B, Dl, Hl, Wl, ly.cin, d->pb.p + ly.w, d->p.p + ly.b, ly.cout, true, out, s,
+        NN_CUDA(nn::launchConv3Tc(in, d->B, Dl, Hl, Wl, ly.cin, d->pbPrep.p + ly.w, d->p.p + ly.b, ly.cout, true, out, s,
             &o));
     }
     else
@@ -404,7 +404,7 @@ int layerBack(dxmcg_denoiser* d, int k, const nn::ConvIn& xin, const bf16* dz, b
             nn::ConvOptions o;
             o.handoverPolls = d->waitPolls;
             o.mask = mask;
-            NN_CUDA(nn::launchConv3Tc(plain(dz, ly.cout), d->B, Dl, Hl, Wl, ly.cout, d->wt.p + ly.wt, nullptr,
+            NN_CUDA(nn::launchConv3Tc(plain(dz, ly.cout), d->B, Dl, Hl, Wl, ly.cout, d->wtPrep.p + ly.wt, nullptr,
                 ly.cin, false, dxOut, s, &o));
         }
         else
@@ -689,6 +689,8 @@ DXMCG_API int dxmcg_denoiser_create(const dxmcg_denoiser_config* c, dxmcg_denois
     NN_CUDA(d->v.reserve(d->nParams));
     NN_CUDA(d->pb.reserve(d->nParams));
     NN_CUDA(d->wt.reserve(d->nWt));
+    NN_CUDA(d->pbPrep.reserve(d->nParams));
+    NN_CUDA(d->wtPrep.reserve(d->nWt));
     *out = d.release();
     const int rc = dxmcg_denoiser_set_params(*out, h.data());
     if (rc != DXMCG_OK) {

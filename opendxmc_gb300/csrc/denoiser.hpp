@@ -56,8 +56,8 @@ struct ConvOptions {
     uint32_t handoverPolls = 0;
 };
 
-// tcgen05 (5th-generation tensor core) form of launchConv3 (conv_tc.cu); the same
-// arguments and result up to FP32 summation order, plus the optional epilogue work
+// tcgen05 (5th-generation tensor core) form of launchConv3 (conv_tc.cu): the same result,
+// plus the optional epilogue work; w are the prepared weights (launchArrangeWeights)
 cudaError_t conv3TcConfigure();
 cudaError_t launchConv3Tc(const ConvIn& in, int B, int D, int H, int W, int Cin, const __nv_bfloat16* w,
     const float* bias, int Cout, bool relu, __nv_bfloat16* out, cudaStream_t s, const ConvOptions* ep = nullptr);
@@ -133,9 +133,10 @@ struct LayerTable {
     int cout[kMaxLayers] = {}, cin[kMaxLayers] = {};
     size_t w[kMaxLayers] = {}, wt[kMaxLayers] = {};
 };
-// the input gradients' weights (taps flipped, channels exchanged) of every layer
-cudaError_t launchTransposeWeights(const __nv_bfloat16* w, __nv_bfloat16* wt, const LayerTable& layers,
-    cudaStream_t s);
+// of every layer's weights: the input gradient's (wt: taps flipped, channels exchanged) and
+// both as launchConv3Tc reads them (wPrep at the offsets of w, wtPrep at those of wt)
+cudaError_t launchArrangeWeights(const __nv_bfloat16* w, __nv_bfloat16* wt, __nv_bfloat16* wPrep,
+    __nv_bfloat16* wtPrep, const LayerTable& layers, cudaStream_t s);
 // Bricks to mark while the input is prepared from a world: active[b] = 1 for each
 // brick b holding a voxel whose material is not 0 (bricks of bx, by, bz voxels, cx and
 // cy of them along x and y, x fastest; the grid nx voxels along x, ny along y).  The

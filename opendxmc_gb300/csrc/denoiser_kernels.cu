@@ -612,18 +612,37 @@ namespace {
             pb[i] = __float2bfloat16_rn(p[i]);
     }
 
-    // dgrad weights of every layer: Wt[ci][t][co] = W[co][26 - t][ci]
-    __global__ void transposeWeightsKernel(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt,
-        const LayerTable layers)
+    // Copies of every layer's weights W[co][tap][ci]: for the input gradients
+    // Wt[ci][tap][co] = W[co][26 - tap][ci], and the prepared forms of both (conv3Tc's:
+    // [slice][in-plane tap][half][z-tap][output channel][8 input channels], z-taps from the
+    // last to the first).  A thread moves 8 input channels of a (co, tap) for W and 8 output
+    // channels of a (ci, tap) for Wt, lanes on neighbouring channels of the other kind.
+    __global__ void arrangeWeightsKernel(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt,
+        __nv_bfloat16* __restrict__ wPrep, __nv_bfloat16* __restrict__ wtPrep, const LayerTable layers)
     {
+        const auto prepared = [](int tap, int c8, int n, int N) { // in units of 8 channels
+            return (((c8 >> 1) * 9 + tap % 9) * 2 + (c8 & 1)) * 3 * N + (2 - tap / 9) * N + n;
+        };
         for (int k = static_cast<int>(blockIdx.y); k < layers.n; k += static_cast<int>(gridDim.y)) {
             const int Cout = layers.cout[k], Cin = layers.cin[k];
             const __nv_bfloat16* const src = w + layers.w[k];
-            __nv_bfloat16* const dst = wt + layers.wt[k];
-            const int n = Cout * 27 * Cin;
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-                const int co = i % Cout, t = (i / Cout) % 27, ci = i / (Cout * 27);
-                dst[i] = src[(co * 27 + (26 - t)) * Cin + ci];
+            const int n = Cout * 27 * Cin / 8;
+            for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < 2 * n; j += gridDim.x * blockDim.x) {
+                if (j < n) {
+                    const int co = j % Cout, tap = (j / Cout) % 27, c8 = j / (Cout * 27);
+                    reinterpret_cast<uint4*>(wPrep + layers.w[k])[prepared(tap, c8, co, Cout)]
+                        = *reinterpret_cast<const uint4*>(src + (co * 27 + tap) * Cin + c8 * 8);
+                } else {
+                    const int i = j - n;
+                    const int ci = i % Cin, tap = (i / Cin) % 27, c8 = i / (Cin * 27);
+                    __align__(16) __nv_bfloat16 v[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        v[e] = src[((c8 * 8 + e) * 27 + (26 - tap)) * Cin + ci];
+                    const uint4 u = *reinterpret_cast<const uint4*>(v);
+                    *reinterpret_cast<uint4*>(wt + layers.wt[k] + (ci * 27 + tap) * Cout + c8 * 8) = u;
+                    reinterpret_cast<uint4*>(wtPrep + layers.wt[k])[prepared(tap, c8, ci, Cin)] = u;
+                }
             }
         }
     }
@@ -836,10 +855,10 @@ cudaError_t launchToBf16(const float* p, __nv_bfloat16* pb, size_t n, cudaStream
     return cudaGetLastError();
 }
 
-cudaError_t launchTransposeWeights(const __nv_bfloat16* w, __nv_bfloat16* wt, const LayerTable& layers,
-    cudaStream_t s)
+cudaError_t launchArrangeWeights(const __nv_bfloat16* w, __nv_bfloat16* wt, __nv_bfloat16* wPrep,
+    __nv_bfloat16* wtPrep, const LayerTable& layers, cudaStream_t s)
 {
-    transposeWeightsKernel<<<dim3(smCount(), std::max(1, layers.n)), 256, 0, s>>>(w, wt, layers);
+    arrangeWeightsKernel<<<dim3(smCount(), std::max(1, layers.n)), 256, 0, s>>>(w, wt, wPrep, wtPrep, layers);
     return cudaGetLastError();
 }
 
