@@ -674,6 +674,39 @@ namespace {
         return B * ((D + zt - 1) / zt) * ((H + 15) / 16) * ((W + 7) / 8);
     }
 
+    struct TcShape {
+        int nt, zt;
+    };
+    // the brick shape of grids that fill the SMs
+    TcShape wholeShape(int Cout) { return Cout % 64 == 0 ? TcShape { 64, 4 } : TcShape { Cout % 32 == 0 ? 32 : 16, 8 }; }
+    // The brick shape of a grid: wholeShape where that has a CTA for every SM, else the thinner
+    // bricks or narrower tiles that need the least time: bricks a CTA times zt + 3 (ZT + 2
+    // planes of MMAs and about one more for the hand-over: a slice took 3.0, 1.8 and 1.4 us at
+    // 32 channels, 2.3, 1.5 and 1.15 us at 16).  Thin bricks re-read more halo, so they lose
+    // once the SMs are full: 8 x 64^3 voxels keep wholeShape.  Network, in wholeShape / this
+    // way: 32^3 voxels of level 1 (32 channels) 78 -> 43 us for its four convolutions (mma.sync
+    // with its pooling pass 107), 8 x 16^3 of level 2 (64 channels) 105 -> 74 us (180),
+    // 8 x 8^3 of level 3 51 -> 31 us (56).
+    TcShape shapeFor(int B, int D, int H, int W, int Cout)
+    {
+        const int sms = nn::smCount();
+        const TcShape whole = wholeShape(Cout);
+        if (tilesOf(B, D, H, W, whole.zt) * (Cout / whole.nt) >= sms)
+            return whole;
+        TcShape best { whole.nt == 16 ? 16 : 32, 8 };
+        long long least = -1;
+        for (int zt = 8; zt >= 2; zt /= 2) {
+            const int tiles = tilesOf(B, D, H, W, zt);
+            const int gx = std::max(1, std::min(tiles, sms / (Cout / best.nt)));
+            const long long cost = static_cast<long long>((tiles + gx - 1) / gx) * (zt + 3);
+            if (least < 0 || cost < least) {
+                least = cost;
+                best.zt = zt;
+            }
+        }
+        return best;
+    }
+
     // cuTensorMapEncodeTiled from the driver, looked up once through the runtime
     PFN_cuTensorMapEncodeTiled_v12000 tensorMapEncoder()
     {
@@ -703,15 +736,7 @@ namespace {
         if (tma && in.b)
             tma = nn::brickTensorMap(&mapB, in.b, B, D, H, W, in.cb, 10, 18, S::HZ);
         // one persistent CTA per SM and output-channel tile, never more than bricks
-        static const int sms = [] {
-            int dev = 0, n = 0;
-            if (cudaGetDevice(&dev) != cudaSuccess
-                || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-                return 0;
-            return n;
-        }();
-        if (sms <= 0)
-            return cudaErrorLaunchOutOfResources;
+        const int sms = nn::smCount();
         const int nSlices = Cin / 16;
         // resident weights where they fit and a CTA has several bricks; two stages then (a
         // third, where it fits, measured no faster on the 512 x 512 x 400 inference: the tensor
@@ -871,6 +896,10 @@ namespace nn {
             if (e == cudaSuccess)
                 e = configure(masked, smem);
         };
+        both(conv3TcKernel<16, 2, false>, conv3TcKernel<16, 2, true>, ConvTcShape<16, 2>::kMaxSmem);
+        both(conv3TcKernel<16, 4, false>, conv3TcKernel<16, 4, true>, ConvTcShape<16, 4>::kMaxSmem);
+        both(conv3TcKernel<32, 2, false>, conv3TcKernel<32, 2, true>, ConvTcShape<32, 2>::kMaxSmem);
+        both(conv3TcKernel<32, 4, false>, conv3TcKernel<32, 4, true>, ConvTcShape<32, 4>::kMaxSmem);
         both(conv3TcKernel<16, 8, false>, conv3TcKernel<16, 8, true>, ConvTcShape<16, 8>::kMaxSmem);
         both(conv3TcKernel<32, 8, false>, conv3TcKernel<32, 8, true>, ConvTcShape<32, 8>::kMaxSmem);
         both(conv3TcKernel<64, 4, false>, conv3TcKernel<64, 4, true>, ConvTcShape<64, 4>::kMaxSmem);
@@ -887,28 +916,29 @@ namespace nn {
         // the pooled output needs whole 2 x 2 x 2 windows; the head a 16-channel output
         if ((e.pooled && ((D | H | W) & 1)) || (e.head && Cout != 16))
             return cudaErrorInvalidValue;
-        if (Cout % 64 == 0)
-            return launchTc<64, 4>(in, B, D, H, W, Cin, w, bias, Cout, relu, out, s, e);
-        if (Cout % 32 == 0)
-            return launchTc<32, 8>(in, B, D, H, W, Cin, w, bias, Cout, relu, out, s, e);
-        return launchTc<16, 8>(in, B, D, H, W, Cin, w, bias, Cout, relu, out, s, e);
+        const TcShape t = e.list ? wholeShape(Cout) : shapeFor(B, D, H, W, Cout);
+        const auto go = [&](auto launch) { return launch(in, B, D, H, W, Cin, w, bias, Cout, relu, out, s, e); };
+        if (t.nt == 64)
+            return go(launchTc<64, 4>);
+        if (t.nt == 32)
+            return t.zt == 8 ? go(launchTc<32, 8>) : (t.zt == 4 ? go(launchTc<32, 4>) : go(launchTc<32, 2>));
+        return t.zt == 8 ? go(launchTc<16, 8>) : (t.zt == 4 ? go(launchTc<16, 4>) : go(launchTc<16, 2>));
     }
 
-    int conv3TcCtas(int B, int D, int H, int W, int Cout)
+    bool conv3TcFills(int B, int D, int H, int W, int Cout)
     {
-        const auto ctas = [&](int zt, int nt) {
-            return B * ((D + zt - 1) / zt) * ((H + 15) / 16) * ((W + 7) / 8) * (Cout / nt);
-        };
-        if (Cout % 64 == 0)
-            return ctas(4, 64);
-        if (Cout % 32 == 0)
-            return ctas(8, 32);
-        return ctas(8, 16);
+        const TcShape t = wholeShape(Cout);
+        return tilesOf(B, D, H, W, t.zt) * (Cout / t.nt) >= smCount();
+    }
+
+    bool conv3TcPays(int B, int D, int H, int W, int Cout)
+    {
+        return conv3TcFills(B, D, H, W, Cout) || conv3SmallCtas(B, D, H, W, Cout) > 2 * smCount();
     }
 
     void conv3TcBrickDims(int D, int H, int W, int Cout, int brick[3], int count[3])
     {
-        const int zt = Cout % 64 == 0 ? 4 : (Cout % 32 == 0 ? 8 : 8);
+        const int zt = wholeShape(Cout).zt;
         brick[0] = 8;
         brick[1] = 16;
         brick[2] = zt;

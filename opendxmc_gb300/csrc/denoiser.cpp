@@ -41,7 +41,6 @@ struct dxmcg_denoiser {
     bool configured = false;
     bool tensorCores = true;  // tcgen05 convolutions (else warp-level mma.sync)
     bool tcEverywhere = false; // tcgen05 even where the grid has fewer bricks than SMs
-    int sms = 1;              // streaming multiprocessors of the device
     uint32_t waitPolls = 0;   // hand-over wait limit of the tcgen05 convolution (0: default)
 
     // activations and gradients of the current shape, per level
@@ -127,11 +126,16 @@ int refreshWeights(dxmcg_denoiser* d, cudaStream_t s)
     return DXMCG_OK;
 }
 
-// tcgen05 for a convolution unless its grid would leave SMs without a CTA (or always,
-// when asked for with conv_path 1)
+// tcgen05 for a convolution unless its grid is too small for it (or always, when asked for
+// with conv_path 1)
 bool useTensorCores(const dxmcg_denoiser* d, int D, int H, int W, int Cout)
 {
-    return d->tensorCores && (d->tcEverywhere || nn::conv3TcCtas(d->B, D, H, W, Cout) >= d->sms);
+    return d->tensorCores && (d->tcEverywhere || nn::conv3TcPays(d->B, D, H, W, Cout));
+}
+// the convolution goes by a list of bricks where one is at hand
+bool useBrickList(const dxmcg_denoiser* d, int D, int H, int W, int Cout)
+{
+    return d->tensorCores && (d->tcEverywhere || nn::conv3TcFills(d->B, D, H, W, Cout));
 }
 
 // conv + bias + ReLU of layer k at level l; on the tcgen05 path the epilogue also does
@@ -510,7 +514,7 @@ namespace nn {
         // sets, which the readout does not use.
         // The input pass marks the tissue bricks; every brick list comes from one launch.
         Sparse sp;
-        const bool sparse = d->ch[0] == 16 && useTensorCores(d, nz, ny, nx, d->ch[0]);
+        const bool sparse = d->ch[0] == 16 && useBrickList(d, nz, ny, nx, d->ch[0]);
         int brick[3] = { 1, 1, 1 }, count[3] = { 1, 1, 1 };
         size_t nb = 0;
         BrickMarks marks;
@@ -557,7 +561,7 @@ namespace nn {
                 int bl[3], cl[3];
             };
             std::vector<SetSpec> specs;
-            const auto tc = [&](int l) { return useTensorCores(d, nz >> l, ny >> l, nx >> l, d->ch[l]); };
+            const auto tc = [&](int l) { return useBrickList(d, nz >> l, ny >> l, nx >> l, d->ch[l]); };
             for (int lt = 0; lt < 3 && lt <= d->L - 2 && tc(lt); ++lt)
                 specs.push_back({ { kEncoderPair, lt }, &d->maskEnc[lt], &d->listEnc[lt], 4 + lt, &sp.enc[lt],
                     &sp.encLen[lt], {}, {} });
@@ -645,8 +649,6 @@ DXMCG_API int dxmcg_denoiser_create(const dxmcg_denoiser_config* c, dxmcg_denois
     d->L = c->levels;
     d->tensorCores = c->conv_path != 2;
     d->tcEverywhere = c->conv_path == 1;
-    if (cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, d->device) != cudaSuccess || d->sms < 1)
-        d->sms = 1;
     for (int l = 0; l < d->L; ++l)
         d->ch[l] = c->channels[l];
     std::vector<std::pair<int, int>> shapes; // (cin, cout) in layer order

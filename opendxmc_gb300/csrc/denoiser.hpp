@@ -27,7 +27,7 @@ struct ConvIn {
 size_t conv3SmemBytes(int nt);
 cudaError_t conv3Configure(); // opt the kernels into their shared-memory size (once per device)
 cudaError_t wgradConfigure(); // the same for launchWgrad's (conv3Configure calls it)
-int smCount();                // of the current device
+int smCount();                // streaming multiprocessors of the device
 
 // Options of the tcgen05 convolution beyond launchConv3's:
 //   list:   device array of output-brick indices (conv3TcBrickDims, x fastest, then y,
@@ -63,9 +63,16 @@ cudaError_t launchConv3Tc(const ConvIn& in, int B, int D, int H, int W, int Cin,
     const float* bias, int Cout, bool relu, __nv_bfloat16* out, cudaStream_t s, const ConvOptions* ep = nullptr);
 cudaError_t conv3TcErrors(unsigned* flags);
 cudaError_t convErrorFlags(unsigned** flags); // where kernels set what conv3TcErrors reads
-// CTAs of the tcgen05 launch for this shape (a grid under one CTA per SM leaves the
-// tensor cores of the other SMs idle: the caller then takes launchConv3)
-int conv3TcCtas(int B, int D, int H, int W, int Cout);
+// whether the tcgen05 launch's own brick shape (conv3TcBrickDims, which a list goes by) has
+// a CTA for every SM
+bool conv3TcFills(int B, int D, int H, int W, int Cout);
+// whether launchConv3Tc, which takes thinner bricks for smaller grids, is the faster one:
+// below two CTAs an SM in launchConv3's smallest bricks that one is (16^3 voxels, 64
+// channels, 256 CTAs: 52 us for the four convolutions and the pooling of a level, tcgen05 52;
+// 16^3, 32 channels, 128 CTAs: 31 against 38; 8^3, 128 channels, 64 CTAs: 19 against 26; but
+// 8 x 8^3, 512 CTAs: 56 against 31)
+bool conv3TcPays(int B, int D, int H, int W, int Cout);
+int conv3SmallCtas(int B, int D, int H, int W, int Cout); // CTAs of launchConv3's smallest bricks
 // the output bricks of the tcgen05 launch for this shape: (x, y, z) voxels per brick
 // and the brick counts along x, y, z (per batch item)
 void conv3TcBrickDims(int D, int H, int W, int Cout, int brick[3], int count[3]);

@@ -758,10 +758,13 @@ namespace {
 
 int smCount()
 {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 1;
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n > 0 ? n : 1;
+    }();
+    return sms;
 }
 
 size_t conv3SmemBytes(int nt) { return 2 * static_cast<size_t>(kHaloBytes + 27 * nt * 32); }
@@ -781,6 +784,11 @@ cudaError_t conv3Configure()
     return e;
 }
 
+int conv3SmallCtas(int B, int D, int H, int W, int Cout)
+{
+    return B * ((D + 1) / 2) * ((H + 3) / 4) * ((W + 7) / 8) * (Cout / 16);
+}
+
 cudaError_t launchConv3(const ConvIn& in, int B, int D, int H, int W, int Cin, const __nv_bfloat16* w,
     const float* bias, int Cout, bool relu, __nv_bfloat16* out, cudaStream_t s, const __nv_bfloat16* mask)
 {
@@ -794,7 +802,7 @@ cudaError_t launchConv3(const ConvIn& in, int B, int D, int H, int W, int Cin, c
     // 64 to 64 (128 CTAs) 30 against 51 us.
     if (4 * bricks * (Cout / (Cout % 32 == 0 ? 32 : 16)) <= smCount()
         && static_cast<size_t>(B) * D * H * W < (1ull << 31)) {
-        const int small = B * ((D + 1) / 2) * ((H + 3) / 4) * ((W + 7) / 8);
+        const int small = conv3SmallCtas(B, D, H, W, Cout) / (Cout / 16);
         conv3SmallKernel<<<dim3(small, Cout / 16), 128, kSmallStages * kSmallStage, s>>>(in, D, H, W, Cin, w, bias,
             Cout, relu ? 1 : 0, out, mask);
     } else if (Cout % 32 == 0) {
