@@ -811,46 +811,34 @@ namespace {
             *jobs.len[j] = base;
     }
 
-    // grown[b] = 1 where brick b or one of its 26 neighbours is active
-    __global__ void brickGrowKernel(const uint8_t* __restrict__ active, int cx, int cy, int cz,
-        uint8_t* __restrict__ grown)
+    // mask_j[b] = 1 where a marked brick lies in the box of input bricks that output brick b of
+    // set j reads; grid: x over b, y: j.  A warp an output brick, its lanes over the rows
+    // of the box (up to about 12 x 8 x 12 bytes, from L1; a thread a brick took 25 us).  One launch of 22 us for
+    // the 8 sets of a four-level network in place of 22, a pass per axis and set, of 3 to 6.
+    __global__ void brickSetsKernel(const uint8_t* __restrict__ in, int nx, int ny, const nn::BrickSetJobs jobs)
     {
-        const int nb = cx * cy * cz;
-        for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-            const int ix = b % cx, iy = (b / cx) % cy, iz = b / (cx * cy);
-            uint8_t g = 0;
-            for (int dz = -1; dz <= 1; ++dz)
-                for (int dy = -1; dy <= 1; ++dy)
-                    for (int dx = -1; dx <= 1; ++dx) {
-                        const int x = ix + dx, y = iy + dy, z = iz + dz;
-                        if (x >= 0 && x < cx && y >= 0 && y < cy && z >= 0 && z < cz)
-                            g |= active[(static_cast<size_t>(z) * cy + y) * cx + x];
-                    }
-            grown[b] = g;
-        }
-    }
-
-    // One pass of a separable union of brick boxes: `out` has in's counts (nx, ny, nz)
-    // with the count along `axis` (0: x, 1: y, 2: z) replaced by nOut, and out[.., b, ..]
-    // = 1 where in[.., c, ..] is marked for some c in [range[2b], range[2b + 1]].
-    __global__ void brickMapAxisKernel(const uint8_t* __restrict__ in, int nx, int ny, int nz, int axis, int nOut,
-        const int* __restrict__ range, uint8_t* __restrict__ out)
-    {
-        const int ox = axis == 0 ? nOut : nx, oy = axis == 1 ? nOut : ny, oz = axis == 2 ? nOut : nz;
-        const int total = ox * oy * oz;
-        for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < total; o += gridDim.x * blockDim.x) {
-            const int x = o % ox, y = (o / ox) % oy, z = o / (ox * oy);
-            const int b = axis == 0 ? x : (axis == 1 ? y : z);
-            const int c1 = range[2 * b + 1];
-            uint8_t v = 0;
-            for (int c = range[2 * b]; c <= c1 && !v; ++c) {
-                const int ix = axis == 0 ? c : x, iy = axis == 1 ? c : y, iz = axis == 2 ? c : z;
-                v = in[(static_cast<size_t>(iz) * ny + iy) * nx + ix];
+        const int j = static_cast<int>(blockIdx.y);
+        const int ox = jobs.count[j][0], oy = jobs.count[j][1];
+        const int2* __restrict__ rx = reinterpret_cast<const int2*>(jobs.ranges[j]);
+        const int2* __restrict__ ry = rx + ox;
+        const int2* __restrict__ rz = ry + oy;
+        const int total = ox * oy * jobs.count[j][2];
+        const int lane = threadIdx.x & 31, warps = static_cast<int>(gridDim.x * blockDim.x) >> 5;
+        for (int o = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x) >> 5; o < total; o += warps) {
+            const int2 x = rx[o % ox], y = ry[(o / ox) % oy], z = rz[o / (ox * oy)];
+            const int ey = y.y - y.x + 1, rows = ey > 0 ? ey * (z.y - z.x + 1) : 0;
+            unsigned v = 0u;
+            for (int i = lane; i < rows; i += 32) {
+                const uint8_t* row = in + (static_cast<size_t>(z.x + i / ey) * ny + y.x + i % ey) * nx;
+#pragma unroll 4
+                for (int c = x.x; c <= x.y; ++c)
+                    v |= row[c];
             }
-            out[o] = v ? 1 : 0;
+            v = __any_sync(0xffffffffu, v != 0u);
+            if (lane == 0)
+                jobs.mask[j][o] = v ? 1 : 0;
         }
     }
-
 
 } // namespace
 
@@ -947,33 +935,17 @@ namespace nn {
         count[2] = (D + zt - 1) / zt;
     }
 
-    cudaError_t launchBrickGrow(const uint8_t* active, const int count[3], uint8_t* grown, cudaStream_t s)
+    cudaError_t launchBrickSets(const uint8_t* in, const int inCount[3], const BrickSetJobs& jobs, cudaStream_t s)
     {
-        const int nb = count[0] * count[1] * count[2];
-        brickGrowKernel<<<std::max(1, std::min((nb + 255) / 256, 4096)), 256, 0, s>>>(active, count[0], count[1],
-            count[2], grown);
-        return cudaGetLastError();
-    }
-
-    cudaError_t launchBrickMap(const uint8_t* in, const int inCount[3], const int outCount[3], const int* ranges,
-        uint8_t* out, uint8_t* tmp1, uint8_t* tmp2, cudaStream_t s)
-    {
-        for (int a = 0; a < 3; ++a)
-            if (inCount[a] < 1 || outCount[a] < 1)
-                return cudaErrorInvalidValue;
-        if (!in || !ranges || !out || !tmp1 || !tmp2 || in == out || in == tmp1 || in == tmp2 || out == tmp1
-            || out == tmp2 || tmp1 == tmp2)
+        if (jobs.n == 0)
+            return cudaSuccess;
+        if (!in || inCount[0] < 1 || inCount[1] < 1 || inCount[2] < 1 || jobs.n > kMaxBrickLists)
             return cudaErrorInvalidValue;
-        const auto grid = [](int items) { return std::max(1, std::min((items + 255) / 256, 4096)); };
-        const int* rx = ranges;
-        const int* ry = rx + 2 * outCount[0];
-        const int* rz = ry + 2 * outCount[1];
-        brickMapAxisKernel<<<grid(outCount[0] * inCount[1] * inCount[2]), 256, 0, s>>>(in, inCount[0], inCount[1],
-            inCount[2], 0, outCount[0], rx, tmp1);
-        brickMapAxisKernel<<<grid(outCount[0] * outCount[1] * inCount[2]), 256, 0, s>>>(tmp1, outCount[0],
-            inCount[1], inCount[2], 1, outCount[1], ry, tmp2);
-        brickMapAxisKernel<<<grid(outCount[0] * outCount[1] * outCount[2]), 256, 0, s>>>(tmp2, outCount[0],
-            outCount[1], inCount[2], 2, outCount[2], rz, out);
+        int most = 1;
+        for (int j = 0; j < jobs.n; ++j)
+            most = std::max(most, jobs.count[j][0] * jobs.count[j][1] * jobs.count[j][2]);
+        brickSetsKernel<<<dim3(std::min((most + 7) / 8, 1024), jobs.n), 256, 0, s>>>(in, inCount[0], inCount[1],
+            jobs);
         return cudaGetLastError();
     }
 

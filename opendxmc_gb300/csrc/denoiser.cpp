@@ -56,7 +56,7 @@ struct dxmcg_denoiser {
     // tissue grown by one; the decoders of levels 1-2 and the encoders of levels 0-2:
     // the bricks that the tissue bricks need), two scratch masks and the brick ranges
     // that map the tissue bricks onto those grids
-    DevBuf<uint8_t> mask0[2], mask1[2], mask2[2], maskEnc[3], maskTmp[2];
+    DevBuf<uint8_t> mask0[2], mask1[2], mask2[2], maskEnc[3];
     DevBuf<int> list0[2], list1[2], list2[2], listEnc[3], listLens, encRanges;
     std::vector<int> encRangesHost;
     DevBuf<unsigned long long> meanCount;
@@ -540,7 +540,6 @@ namespace nn {
                 NN_CUDA(l.reserve(nb));
             NN_CUDA(d->listLens.reserve(9));
             BrickListJobs lists;
-            NN_CUDA(launchBrickGrow(d->mask0[0].p, count, d->mask0[1].p, s));
             lists.add(d->mask0[0].p, static_cast<int>(nb), d->list0[0].p, d->listLens.p);
             lists.add(d->mask0[1].p, static_cast<int>(nb), d->list0[1].p, d->listLens.p + 1);
             NN_CUDA(cudaMemsetAsync(d->worldOut.p, 0, n * sizeof(double), s));
@@ -578,41 +577,47 @@ namespace nn {
                 }
             }
             const int dim0[3] = { nx, ny, nz };
-            size_t nRanges = 0, tmp1 = 1, tmp2 = 1;
+            // ranges of every set, the neighbours of the tissue bricks first
+            size_t nRanges = 2 * static_cast<size_t>(count[0] + count[1] + count[2]);
             for (auto& sc : specs) {
                 const int l = sc.t.level;
                 conv3TcBrickDims(nz >> l, ny >> l, nx >> l, d->ch[l], sc.bl, sc.cl);
                 nRanges += 2 * static_cast<size_t>(sc.cl[0] + sc.cl[1] + sc.cl[2]);
-                tmp1 = std::max(tmp1, static_cast<size_t>(sc.cl[0]) * count[1] * count[2]);
-                tmp2 = std::max(tmp2, static_cast<size_t>(sc.cl[0]) * sc.cl[1] * count[2]);
             }
-            if (!specs.empty()) {
-                d->encRangesHost.assign(nRanges, 0);
-                size_t off = 0;
-                for (auto& sc : specs)
-                    for (int a = 0; a < 3; ++a) {
-                        brickRanges(d->L, sc.t, dim0[a], brick[a], count[a], dim0[a] >> sc.t.level, sc.bl[a],
-                            sc.cl[a], d->encRangesHost.data() + off);
-                        off += 2 * static_cast<size_t>(sc.cl[a]);
-                    }
-                NN_CUDA(d->encRanges.reserve(nRanges));
-                NN_CUDA(cudaMemcpyAsync(d->encRanges.p, d->encRangesHost.data(), nRanges * sizeof(int),
-                    cudaMemcpyHostToDevice, s));
-                NN_CUDA(d->maskTmp[0].reserve(tmp1));
-                NN_CUDA(d->maskTmp[1].reserve(tmp2));
-                off = 0;
-                for (auto& sc : specs) {
-                    const size_t nbl = static_cast<size_t>(sc.cl[0]) * sc.cl[1] * sc.cl[2];
-                    NN_CUDA(sc.mask->reserve(nbl));
-                    NN_CUDA(sc.list->reserve(nbl));
-                    NN_CUDA(launchBrickMap(d->mask0[0].p, count, sc.cl, d->encRanges.p + off, sc.mask->p,
-                        d->maskTmp[0].p, d->maskTmp[1].p, s));
-                    off += 2 * static_cast<size_t>(sc.cl[0] + sc.cl[1] + sc.cl[2]);
-                    lists.add(sc.mask->p, static_cast<int>(nbl), sc.list->p, d->listLens.p + sc.lenIndex);
-                    *sc.spList = sc.list->p;
-                    *sc.spLen = d->listLens.p + sc.lenIndex;
+            d->encRangesHost.assign(nRanges, 0);
+            NN_CUDA(d->encRanges.reserve(nRanges));
+            BrickSetJobs sets;
+            size_t off = 0;
+            const auto addSet = [&](uint8_t* mask, const int n3[3]) {
+                sets.mask[sets.n] = mask;
+                sets.ranges[sets.n] = d->encRanges.p + off;
+                for (int a = 0; a < 3; ++a)
+                    sets.count[sets.n][a] = n3[a];
+                ++sets.n;
+            };
+            addSet(d->mask0[1].p, count);
+            for (int a = 0; a < 3; ++a)
+                for (int b = 0; b < count[a]; ++b) {
+                    d->encRangesHost[off++] = std::max(0, b - 1);
+                    d->encRangesHost[off++] = std::min(count[a] - 1, b + 1);
                 }
+            for (auto& sc : specs) {
+                const size_t nbl = static_cast<size_t>(sc.cl[0]) * sc.cl[1] * sc.cl[2];
+                NN_CUDA(sc.mask->reserve(nbl));
+                NN_CUDA(sc.list->reserve(nbl));
+                addSet(sc.mask->p, sc.cl);
+                for (int a = 0; a < 3; ++a) {
+                    brickRanges(d->L, sc.t, dim0[a], brick[a], count[a], dim0[a] >> sc.t.level, sc.bl[a], sc.cl[a],
+                        d->encRangesHost.data() + off);
+                    off += 2 * static_cast<size_t>(sc.cl[a]);
+                }
+                lists.add(sc.mask->p, static_cast<int>(nbl), sc.list->p, d->listLens.p + sc.lenIndex);
+                *sc.spList = sc.list->p;
+                *sc.spLen = d->listLens.p + sc.lenIndex;
             }
+            NN_CUDA(cudaMemcpyAsync(d->encRanges.p, d->encRangesHost.data(), nRanges * sizeof(int),
+                cudaMemcpyHostToDevice, s));
+            NN_CUDA(launchBrickSets(d->mask0[0].p, count, sets, s));
             NN_CUDA(launchBrickLists(lists, s));
         }
         if ((rc = forward(d, d->worldInput.p, s, nullptr, d->worldOut.p, scale, sparse ? &sp : nullptr)) != DXMCG_OK)

@@ -78,21 +78,22 @@ int conv3SmallCtas(int B, int D, int H, int W, int Cout); // CTAs of launchConv3
 void conv3TcBrickDims(int D, int H, int W, int Cout, int brick[3], int count[3]);
 // Brick sets of the world path (one byte per brick, bricks x fastest, all on the device;
 // the tissue set comes from launchPrepareInput's brick marks):
-//   grow:     the marked bricks and their 26 neighbours;
-//   map:      bricks of another brick grid (outCount per axis) that a marked brick
-//             needs: the union over marked bricks (cx, cy, cz) of the boxes
-//             X(cx) x Y(cy) x Z(cz), where `ranges` (device) holds for each output brick
-//             index b along x, then y, then z, the range [lo, hi] of input brick indices
-//             whose interval holds b; three one-axis passes (tmp1: outCount[0] x
-//             inCount[1] x inCount[2] bytes, tmp2: outCount[0] x outCount[1] x
-//             inCount[2]);
+//   sets:     bricks of other brick grids (count per axis) that a marked brick needs: the
+//             union over marked bricks (cx, cy, cz) of the boxes X(cx) x Y(cy) x Z(cz), where
+//             `ranges` (device) holds for each output brick index b along x, then y, then z,
+//             the range [lo, hi] of input brick indices whose interval holds b (lo > hi:
+//             none); up to kMaxBrickLists sets in one launch;
 //   list:     the marked indices in increasing order, and how many (*listLen);
 //             launchBrickLists compacts up to kMaxBrickLists masks in one launch.
-cudaError_t launchBrickGrow(const uint8_t* active, const int count[3], uint8_t* grown, cudaStream_t s);
-cudaError_t launchBrickMap(const uint8_t* in, const int inCount[3], const int outCount[3], const int* ranges,
-    uint8_t* out, uint8_t* tmp1, uint8_t* tmp2, cudaStream_t s);
-cudaError_t launchBrickList(const uint8_t* mask, int nb, int* list, int* listLen, cudaStream_t s);
 constexpr int kMaxBrickLists = 12;
+struct BrickSetJobs {
+    uint8_t* mask[kMaxBrickLists] = {};
+    const int* ranges[kMaxBrickLists] = {};
+    int count[kMaxBrickLists][3] = {};
+    int n = 0;
+};
+cudaError_t launchBrickSets(const uint8_t* in, const int inCount[3], const BrickSetJobs& jobs, cudaStream_t s);
+cudaError_t launchBrickList(const uint8_t* mask, int nb, int* list, int* listLen, cudaStream_t s);
 struct BrickListJobs {
     const uint8_t* mask[kMaxBrickLists] = {};
     int* list[kMaxBrickLists] = {};
