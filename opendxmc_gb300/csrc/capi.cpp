@@ -12,11 +12,16 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
+#include <thread>
 #include <vector>
+
+#include <unistd.h>
 
 #include <cuda_runtime.h>
 
@@ -526,6 +531,103 @@ int segLut(const SegTable& t, const double*& lutD, const uint8_t*& lutM)
     }
     lutD = cache.d.p;
     lutM = cache.m.p;
+    return DXMCG_OK;
+}
+
+// whether kernels can work on these arrays in host memory, through the host's page tables
+bool hostPagesOnDevice(std::initializer_list<const void*> arrays)
+{
+    for (const void* p : arrays) {
+        cudaPointerAttributes a {};
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        if (a.type != cudaMemoryTypeUnregistered && a.type != cudaMemoryTypeHost)
+            return false;
+    }
+    int dev = 0, access = 0, tables = 0;
+    return cudaGetDevice(&dev) == cudaSuccess
+        && cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess
+        && cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) == cudaSuccess
+        && access && tables;
+}
+
+// maps the pages of a buffer (of one that is to be written: by a write, as a read would map
+// the page of zeros that all fresh memory shares)
+template <bool WRITE, class T>
+void touchPages(const T* p, size_t n)
+{
+    static const uintptr_t kPage = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
+    const auto a = reinterpret_cast<uintptr_t>(p), b = a + n * sizeof(T);
+    for (uintptr_t q = a; q < b; q = (q / kPage + 1) * kPage) {
+        if constexpr (WRITE)
+            *reinterpret_cast<volatile unsigned char*>(q) = 0;
+        else
+            (void)*reinterpret_cast<const volatile unsigned char*>(q);
+    }
+}
+
+// Segmentation where the kernel reads and writes the caller's arrays themselves: no device
+// buffers, no copies.  What takes the time then are the pages of fresh output arrays, which the
+// host maps (and zeroes) at their first touch: a few threads touch them block by block (59 MB
+// by 1, 4 and 8 threads: 1730, 550 and 690 us), and the kernel works on the blocks whose pages
+// are there.  256 x 256 x 100 voxels into fresh arrays, their release included: 3200 us before
+// (the copy into untouched pages alone took 2800, the device buffers 500), 1150 this way; into
+// arrays in use 1040 and 580.
+int segmentInPlace(const SegTable& t, const double* lutD, const uint8_t* lutM, const double* hu, uint64_t n,
+    uint8_t* material, double* density)
+{
+    constexpr uint64_t kBlock = 1ull << 19;
+    constexpr unsigned kThreads = 4;
+    const uint64_t blocks = (n + kBlock - 1) / kBlock;
+    const std::unique_ptr<std::atomic<unsigned char>[]> there(new (std::nothrow) std::atomic<unsigned char>[blocks]());
+    if (!there)
+        return fail(DXMCG_ERR_CAPACITY, "ct_segment: out of host memory");
+    std::atomic<uint64_t> next { 0 };
+    const auto touchNext = [&] {
+        const uint64_t b = next.fetch_add(1);
+        if (b >= blocks)
+            return false;
+        const uint64_t a = b * kBlock;
+        const size_t m = std::min<uint64_t>(kBlock, n - a);
+        touchPages<false>(hu + a, m);
+        touchPages<true>(material + a, m);
+        touchPages<true>(density + a, m);
+        there[b].store(1, std::memory_order_release);
+        return true;
+    };
+    std::vector<std::thread> helpers;
+    try {
+        helpers.reserve(kThreads);
+        for (uint64_t k = 1; k < std::min<uint64_t>(kThreads, blocks); ++k)
+            helpers.emplace_back([&] {
+                while (touchNext()) { }
+            });
+    } catch (const std::exception&) {
+        // fewer helpers, or none: this thread touches what they do not
+    }
+    // what is there goes to the device whenever that has nothing to do, and the rest at the end
+    cudaError_t e = cudaSuccess;
+    for (uint64_t sent = 0, ready = 0; sent < blocks;) {
+        while (ready < blocks && there[ready].load(std::memory_order_acquire))
+            ++ready;
+        if (ready > sent && (ready == blocks || cudaStreamQuery(nullptr) != cudaErrorNotReady)) {
+            const uint64_t a = sent * kBlock;
+            if (e == cudaSuccess)
+                e = launchSegment(hu + a, std::min<uint64_t>(ready * kBlock, n) - a, t, lutD, lutM, material + a,
+                    density + a, nullptr);
+            sent = ready;
+        } else if (!touchNext()) {
+            std::this_thread::yield(); // the others are at the last blocks
+        }
+    }
+    for (auto& h : helpers)
+        h.join();
+    const cudaError_t done = cudaStreamSynchronize(nullptr);
+    if (e != cudaSuccess)
+        return cudaFail(e, "segmentation kernel launch");
+    DXMCG_CUDA(done);
     return DXMCG_OK;
 }
 
@@ -1521,6 +1623,8 @@ DXMCG_API int dxmcg_ct_segment(const dxmcg_segmentation* table, const double* hu
     const uint8_t* lutM = nullptr;
     if ((rc = segLut(t, lutD, lutM)) != DXMCG_OK)
         return rc;
+    if (hostPagesOnDevice({ hu, material, density }))
+        return segmentInPlace(t, lutD, lutM, hu, n, material, density);
     const size_t chunk = std::min<uint64_t>(n, kStreamChunk);
     DeviceBuffer<double> dh, dd;
     DeviceBuffer<uint8_t> dm;
