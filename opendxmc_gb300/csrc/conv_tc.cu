@@ -42,6 +42,7 @@
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
 
+#include "chain.cuh"
 #include "denoiser.hpp"
 #include "engine.hpp"
 #include "tensor_map.hpp"
@@ -242,13 +243,6 @@ namespace {
         const uint32_t sbase = (umma::smemAddr(smemRaw) + 255u) & ~255u;
         unsigned char* const smem = smemRaw + (sbase - umma::smemAddr(smemRaw));
         const uint32_t wbase = sbase + stages * S::kHalo;
-        // this CTA's bricks: blockIdx.x, blockIdx.x + gridDim.x, ... of the brick list
-        // (ep.list, ep.listLen entries) or of all `tiles` bricks
-        const int nBricks = ep.list ? __ldg(ep.listLen) : tiles;
-        const int myTiles = static_cast<int>(blockIdx.x) < nBricks
-            ? (nBricks - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1
-            : 0;
-        const int nItems = myTiles * nSlices;
         volatile int* abortp = &abortFlag;
         // limit of the hand-over waits between the roles (the drains keep kPolls)
         const uint32_t hp = ep.handoverPolls ? ep.handoverPolls : kPolls;
@@ -281,6 +275,15 @@ namespace {
             umma::storeWait();
         }
 
+        chain::afterPrevious();
+        chain::letNextStart();
+        // this CTA's bricks: blockIdx.x, blockIdx.x + gridDim.x, ... of the brick list
+        // (ep.list, ep.listLen entries) or of all `tiles` bricks
+        const int nBricks = ep.list ? __ldg(ep.listLen) : tiles;
+        const int myTiles = static_cast<int>(blockIdx.x) < nBricks
+            ? (nBricks - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1
+            : 0;
+        const int nItems = myTiles * nSlices;
         // a slice's weights for all taps, z-taps stacked per in-plane tap, from the prepared
         // weights: 54 blocks (in-plane tap, channel half, z-tap) of NT contiguous rows.  From
         // the weights as they are stored each 16 bytes were a sector of their own: a brick of
@@ -746,10 +749,9 @@ namespace {
         const bool resident = tiles > gx && S::smemFor(nSlices, true, 2) <= S::kMaxSmem;
         const int stages = tiles <= gx && S::smemFor(nSlices, resident, 3) <= S::kMaxSmem ? 3 : 2;
         // the mask's registers would spill in the forward pass
-        (ep.mask ? conv3TcKernel<NT, ZT, true> : conv3TcKernel<NT, ZT, false>)<<<dim3(gx, gy), kConvThreads,
-            S::smemFor(nSlices, resident, stages), s>>>(in, D, H, W, Cin, w, bias, Cout, relu ? 1 : 0, out, mapA,
-            mapB, tma ? 1 : 0, tiles, resident ? 1 : 0, stages, ep);
-        return cudaGetLastError();
+        return chain::launchChained(ep.mask ? conv3TcKernel<NT, ZT, true> : conv3TcKernel<NT, ZT, false>,
+            dim3(gx, gy), kConvThreads, S::smemFor(nSlices, resident, stages), s, in, D, H, W, Cin, w, bias, Cout,
+            relu ? 1 : 0, out, mapA, mapB, tma ? 1 : 0, tiles, resident ? 1 : 0, stages, ep);
     }
 
     // For each job j (one CTA of 1024 threads each): list_j[0 .. *len_j) = the indices b
@@ -762,6 +764,7 @@ namespace {
         const int j = static_cast<int>(blockIdx.x);
         const uint8_t* __restrict__ active = jobs.mask[j];
         int* __restrict__ list = jobs.list[j];
+        chain::letNextStart();
         const int nb = jobs.nb[j];
         const bool words = (reinterpret_cast<uintptr_t>(active) & 3u) == 0u;
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;

@@ -19,6 +19,7 @@
 
 #include <cuda_bf16.h>
 
+#include "chain.cuh"
 #include "denoiser.hpp"
 #include "device.cuh"
 
@@ -245,6 +246,8 @@ namespace {
         const __nv_bfloat16* __restrict__ wgt, const float* __restrict__ bias, int Cout, int relu,
         __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ mask)
     {
+        chain::afterPrevious();
+        chain::letNextStart();
         extern __shared__ __align__(128) unsigned char smem[];
         const int nbx = (W + 7) >> 3, nby = (H + 3) >> 2, nbz = (D + 1) >> 1;
         int brick = static_cast<int>(blockIdx.x);
@@ -403,6 +406,8 @@ namespace {
     __global__ void avgPoolKernel(const uint4* __restrict__ x, uint4* __restrict__ out, int B, int D, int H, int W,
         int groups)
     {
+        chain::afterPrevious();
+        chain::letNextStart();
         const int Dh = D >> 1, Hh = H >> 1, Wh = W >> 1;
         const size_t items = static_cast<size_t>(B) * Dh * Hh * Wh * groups;
         for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < items;
@@ -440,6 +445,8 @@ namespace {
         const uint4* __restrict__ dxNext, const uint4* __restrict__ yu, uint4* __restrict__ du,
         const uint4* __restrict__ ye, uint4* __restrict__ de, int B, int D, int H, int W)
     {
+        chain::afterPrevious();
+        chain::letNextStart();
         const int gc = gu + gs;
         const int Dh = D >> 1, Hh = H >> 1, Wh = W >> 1;
         const size_t nU = du ? static_cast<size_t>(B) * Dh * Hh * Wh * gu : 0;
@@ -499,6 +506,8 @@ namespace {
         double* __restrict__ predOut, __nv_bfloat16* __restrict__ dd, float* __restrict__ dhw,
         double* __restrict__ lossSum)
     {
+        chain::afterPrevious();
+        chain::letNextStart();
         float w[C0];
 #pragma unroll
         for (int c = 0; c < C0; ++c)
@@ -592,6 +601,8 @@ namespace {
         float* __restrict__ v, __nv_bfloat16* __restrict__ pb, size_t n, float lr, float b1, float b2, float eps,
         float c1, float c2)
     {
+        chain::afterPrevious();
+        chain::letNextStart();
         for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
              i += static_cast<size_t>(gridDim.x) * blockDim.x) {
             const float gi = g[i];
@@ -620,6 +631,8 @@ namespace {
     __global__ void arrangeWeightsKernel(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt,
         __nv_bfloat16* __restrict__ wPrep, __nv_bfloat16* __restrict__ wtPrep, const LayerTable layers)
     {
+        chain::afterPrevious();
+        chain::letNextStart();
         const auto prepared = [](int tap, int c8, int n, int N) { // in units of 8 channels
             return (((c8 >> 1) * 9 + tap % 9) * 2 + (c8 & 1)) * 3 * N + (2 - tap / 9) * N + n;
         };
@@ -803,8 +816,8 @@ cudaError_t launchConv3(const ConvIn& in, int B, int D, int H, int W, int Cin, c
     if (4 * bricks * (Cout / (Cout % 32 == 0 ? 32 : 16)) <= smCount()
         && static_cast<size_t>(B) * D * H * W < (1ull << 31)) {
         const int small = conv3SmallCtas(B, D, H, W, Cout) / (Cout / 16);
-        conv3SmallKernel<<<dim3(small, Cout / 16), 128, kSmallStages * kSmallStage, s>>>(in, D, H, W, Cin, w, bias,
-            Cout, relu ? 1 : 0, out, mask);
+        return chain::launchChained(conv3SmallKernel, dim3(small, Cout / 16), 128, kSmallStages * kSmallStage, s, in, D,
+            H, W, Cin, w, bias, Cout, relu ? 1 : 0, out, mask);
     } else if (Cout % 32 == 0) {
         conv3Kernel<32><<<dim3(bricks, Cout / 32), 256, conv3SmemBytes(32), s>>>(in, D, H, W, Cin, w, bias, Cout,
             relu ? 1 : 0, out, mask);
@@ -819,9 +832,8 @@ cudaError_t launchAvgPool(const __nv_bfloat16* x, __nv_bfloat16* out, int B, int
     cudaStream_t s)
 {
     const size_t items = static_cast<size_t>(B) * (D / 2) * (H / 2) * (W / 2) * (C / 8);
-    avgPoolKernel<<<grid1d(items), 256, 0, s>>>(reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(out), B,
-        D, H, W, C / 8);
-    return cudaGetLastError();
+    return chain::launchChained(avgPoolKernel, grid1d(items), 256, 0, s, reinterpret_cast<const uint4*>(x),
+        reinterpret_cast<uint4*>(out), B, D, H, W, C / 8);
 }
 
 cudaError_t launchSplitConcatGrad(const __nv_bfloat16* dcat, int cu, int cs, const __nv_bfloat16* dxNext,
@@ -830,10 +842,9 @@ cudaError_t launchSplitConcatGrad(const __nv_bfloat16* dcat, int cu, int cs, con
 {
     const size_t items = (du ? static_cast<size_t>(B) * (D / 2) * (H / 2) * (W / 2) * (cu / 8) : 0)
         + (de ? static_cast<size_t>(B) * D * H * W * (cs / 8) : 0);
-    splitConcatGradKernel<<<grid1d(items), 256, 0, s>>>(reinterpret_cast<const uint4*>(dcat), cu / 8, cs / 8,
-        reinterpret_cast<const uint4*>(dxNext), reinterpret_cast<const uint4*>(yu), reinterpret_cast<uint4*>(du),
-        reinterpret_cast<const uint4*>(ye), reinterpret_cast<uint4*>(de), B, D, H, W);
-    return cudaGetLastError();
+    return chain::launchChained(splitConcatGradKernel, grid1d(items), 256, 0, s, reinterpret_cast<const uint4*>(dcat),
+        cu / 8, cs / 8, reinterpret_cast<const uint4*>(dxNext), reinterpret_cast<const uint4*>(yu),
+        reinterpret_cast<uint4*>(du), reinterpret_cast<const uint4*>(ye), reinterpret_cast<uint4*>(de), B, D, H, W);
 }
 
 cudaError_t launchHead(const __nv_bfloat16* d, int C0, const float* hw, size_t nvox, const float* target,
@@ -841,20 +852,16 @@ cudaError_t launchHead(const __nv_bfloat16* d, int C0, const float* hw, size_t n
 {
     const float invN = nvox ? 1.0f / static_cast<float>(nvox) : 0.0f;
     const int g = grid1d(nvox);
-    if (C0 == 16)
-        headKernel<16><<<g, 256, 0, s>>>(d, hw, nvox, target, invN, pred, predScale, predOut, dd, dhw, lossSum);
-    else if (C0 == 32)
-        headKernel<32><<<g, 256, 0, s>>>(d, hw, nvox, target, invN, pred, predScale, predOut, dd, dhw, lossSum);
-    else
+    if (C0 != 16 && C0 != 32)
         return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    return chain::launchChained(C0 == 16 ? headKernel<16> : headKernel<32>, g, 256, 0, s, d, hw, nvox, target, invN, pred,
+        predScale, predOut, dd, dhw, lossSum);
 }
 
 cudaError_t launchAdam(float* p, const float* g, float* m, float* v, __nv_bfloat16* pb, size_t n, float lr, float b1,
     float b2, float eps, float c1, float c2, cudaStream_t s)
 {
-    adamKernel<<<grid1d(n), 256, 0, s>>>(p, g, m, v, pb, n, lr, b1, b2, eps, c1, c2);
-    return cudaGetLastError();
+    return chain::launchChained(adamKernel, grid1d(n), 256, 0, s, p, g, m, v, pb, n, lr, b1, b2, eps, c1, c2);
 }
 
 cudaError_t launchToBf16(const float* p, __nv_bfloat16* pb, size_t n, cudaStream_t s)
@@ -866,8 +873,8 @@ cudaError_t launchToBf16(const float* p, __nv_bfloat16* pb, size_t n, cudaStream
 cudaError_t launchArrangeWeights(const __nv_bfloat16* w, __nv_bfloat16* wt, __nv_bfloat16* wPrep,
     __nv_bfloat16* wtPrep, const LayerTable& layers, cudaStream_t s)
 {
-    arrangeWeightsKernel<<<dim3(smCount(), std::max(1, layers.n)), 256, 0, s>>>(w, wt, wPrep, wtPrep, layers);
-    return cudaGetLastError();
+    return chain::launchChained(arrangeWeightsKernel, dim3(smCount(), std::max(1, layers.n)), 256, 0, s, w, wt, wPrep,
+        wtPrep, layers);
 }
 
 cudaError_t launchPrepareInput(const float* dose, const float* dens, const uint8_t* mat, const Tally* tally,

@@ -30,6 +30,7 @@
 
 #include <cuda_bf16.h>
 
+#include "chain.cuh"
 #include "denoiser.hpp"
 #include "tensor_map.hpp"
 #include "umma.cuh"
@@ -165,6 +166,8 @@ namespace {
         }
         umma::fenceProxyAsync();
         __syncthreads();
+        chain::afterPrevious();
+        chain::letNextStart();
 
         const int first = static_cast<int>(blockIdx.x), hop = static_cast<int>(gridDim.x);
         const int mine = first < nBricks ? (nBricks - 1 - first) / hop + 1 : 0;
@@ -312,9 +315,8 @@ cudaError_t launchWgrad(const ConvIn& in, const __nv_bfloat16* dz, int B, int D,
     const int tiles = (Cout / 16) * (Cin / 16);
     // one CTA an SM: as many per tile as fill the SMs once
     const int gx = std::max(1, std::min(bricks, smCount() / tiles));
-    wgradKernel<<<dim3(gx, Cout / 16, Cin / 16), kThreads, kSmem, s>>>(mapA, mapB, mapZ, in.ca, in.halfA ? 1 : 0, D, H,
-        W, Cin, bricks, dW, db, errors);
-    return cudaGetLastError();
+    return chain::launchChained(wgradKernel, dim3(gx, Cout / 16, Cin / 16), kThreads, kSmem, s, mapA, mapB, mapZ, in.ca,
+        in.halfA ? 1 : 0, D, H, W, Cin, bricks, dW, db, errors);
 }
 
 } // namespace nn
