@@ -684,8 +684,8 @@ namespace {
     TcShape wholeShape(int Cout) { return Cout % 64 == 0 ? TcShape { 64, 4 } : TcShape { Cout % 32 == 0 ? 32 : 16, 8 }; }
     // The brick shape of a grid: wholeShape where that has a CTA for every SM, else the thinner
     // bricks or narrower tiles that need the least time: bricks a CTA times zt + 3 (ZT + 2
-    // planes of MMAs and about one more for the hand-over: a slice took 3.0, 1.8 and 1.4 us at
-    // 32 channels, 2.3, 1.5 and 1.15 us at 16).  Thin bricks re-read more halo, so they lose
+    // planes of MMAs and about one more for the hand-over), times 6 at 32 channels and 5 at 16
+    // (a slice took 3.0, 1.8 and 1.4 us at 32 channels, 2.3, 1.5 and 1.15 us at 16).  Thin bricks re-read more halo, so they lose
     // once the SMs are full: 8 x 64^3 voxels keep wholeShape.  Network, in wholeShape / this
     // way: 32^3 voxels of level 1 (32 channels) 78 -> 43 us for its four convolutions (mma.sync
     // with its pooling pass 107), 8 x 16^3 of level 2 (64 channels) 105 -> 74 us (180),
@@ -696,17 +696,19 @@ namespace {
         const TcShape whole = wholeShape(Cout);
         if (tilesOf(B, D, H, W, whole.zt) * (Cout / whole.nt) >= sms)
             return whole;
-        TcShape best { whole.nt == 16 ? 16 : 32, 8 };
+        TcShape best = whole;
         long long least = -1;
-        for (int zt = 8; zt >= 2; zt /= 2) {
-            const int tiles = tilesOf(B, D, H, W, zt);
-            const int gx = std::max(1, std::min(tiles, sms / (Cout / best.nt)));
-            const long long cost = static_cast<long long>((tiles + gx - 1) / gx) * (zt + 3);
-            if (least < 0 || cost < least) {
-                least = cost;
-                best.zt = zt;
+        for (int nt = whole.nt == 16 ? 16 : 32; nt >= 16; nt -= 16)
+            for (int zt = 8; zt >= 2; zt /= 2) {
+                const int tiles = tilesOf(B, D, H, W, zt);
+                const int gx = std::max(1, std::min(tiles, sms / (Cout / nt)));
+                const long long cost
+                    = static_cast<long long>((tiles + gx - 1) / gx) * (zt + 3) * (nt == 32 ? 6 : 5);
+                if (least < 0 || cost < least) {
+                    least = cost;
+                    best = { nt, zt };
+                }
             }
-        }
         return best;
     }
 
@@ -924,7 +926,7 @@ namespace nn {
 
     bool conv3TcPays(int B, int D, int H, int W, int Cout)
     {
-        return conv3TcFills(B, D, H, W, Cout) || conv3SmallCtas(B, D, H, W, Cout) > 2 * smCount();
+        return conv3TcFills(B, D, H, W, Cout) || conv3SmallCtas(B, D, H, W, Cout) > smCount();
     }
 
     void conv3TcBrickDims(int D, int H, int W, int Cout, int brick[3], int count[3])

@@ -66,11 +66,10 @@ cudaError_t convErrorFlags(unsigned** flags); // where kernels set what conv3TcE
 // whether the tcgen05 launch's own brick shape (conv3TcBrickDims, which a list goes by) has
 // a CTA for every SM
 bool conv3TcFills(int B, int D, int H, int W, int Cout);
-// whether launchConv3Tc, which takes thinner bricks for smaller grids, is the faster one:
-// below two CTAs an SM in launchConv3's smallest bricks that one is (16^3 voxels, 64
-// channels, 256 CTAs: 52 us for the four convolutions and the pooling of a level, tcgen05 52;
-// 16^3, 32 channels, 128 CTAs: 31 against 38; 8^3, 128 channels, 64 CTAs: 19 against 26; but
-// 8 x 8^3, 512 CTAs: 56 against 31)
+// whether launchConv3Tc, which takes thinner bricks for smaller grids, is the faster one: not
+// where launchConv3's smallest bricks leave SMs idle.  The network on 64^3, 32^3, 2 x 48^3 and
+// 8 x 32^3 voxels: 153, 99, 155 and 156 us with the line at one such brick an SM; at two 168,
+// 99, 171 and 162; tcgen05 everywhere 160, 122, 158 and 158.
 bool conv3TcPays(int B, int D, int H, int W, int Cout);
 int conv3SmallCtas(int B, int D, int H, int W, int Cout); // CTAs of launchConv3's smallest bricks
 // the output bricks of the tcgen05 launch for this shape: (x, y, z) voxels per brick

@@ -11,7 +11,7 @@ SHAPES = [
     (1, 32, 32, 32),   # level 0: (16, 2)
     (2, 32, 32, 32),   # level 0: (16, 4)
     (1, 40, 24, 56),   # level 0: (16, 4), partial bricks along y and z
-    (1, 64, 64, 64),   # level 1: (32, 2), levels 2 and 3 on mma.sync
+    (1, 64, 64, 64),   # level 1: (32, 2), level 2: (16, 2), level 3 on mma.sync
     (12, 32, 32, 32),  # level 1: (32, 4), level 2: (32, 2), level 3 4^3 voxels
     (3, 8, 8, 8),      # every level smaller than its bricks
 ]
