@@ -377,9 +377,9 @@ int deviceErrors(const DevCounters& c, const char* what)
 // the SMs another job's tail frees; one world at a time keeps its voxels and tally in L2.
 // Smaller jobs would mostly be tails: they run side by side on up to kSmallStreams
 // streams, each with twice its share of the resident blocks, so that blocks of the jobs
-// still running replace those of jobs that are done.  Eight jobs of 1e5 to 2e6 histories:
-// 0.74 ms in one launch over a shared queue (whose lanes read their job's descriptor
-// from memory), 0.48 ms side by side, 0.80 ms one after another.
+// still running replace those of jobs that are done.  Eight jobs of 1e5 to 2e6 histories,
+// dose read back: 1.19 ms in one launch over a shared queue (whose lanes read their job's
+// descriptor from memory), 1.07 ms side by side.
 constexpr uint64_t kLargeJob = 1ull << 21;
 constexpr int kLargeStreams = 4, kSmallStreams = 32;
 
