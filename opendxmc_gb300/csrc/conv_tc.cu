@@ -816,11 +816,28 @@ namespace {
             *jobs.len[j] = base;
     }
 
+    // bits[row][w]: bit i set where brick 32 w + i of the row (nx bricks) is marked
+    __global__ void brickBitsKernel(const uint8_t* __restrict__ in, int nx, int rows, uint32_t* __restrict__ bits)
+    {
+        const int words = (nx + 31) >> 5;
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < rows * words; t += gridDim.x * blockDim.x) {
+            const int row = t / words, x0 = 32 * (t % words);
+            uint32_t v = 0u;
+#pragma unroll 8
+            for (int i = 0; i < 32; ++i)
+                if (x0 + i < nx && in[static_cast<size_t>(row) * nx + x0 + i])
+                    v |= 1u << i;
+            bits[t] = v;
+        }
+    }
+
     // mask_j[b] = 1 where a marked brick lies in the box of input bricks that output brick b of
-    // set j reads; grid: x over b, y: j.  A warp an output brick, its lanes over the rows
-    // of the box (up to about 12 x 8 x 12 bytes, from L1; a thread a brick took 25 us).  One launch of 22 us for
-    // the 8 sets of a four-level network in place of 22, a pass per axis and set, of 3 to 6.
-    __global__ void brickSetsKernel(const uint8_t* __restrict__ in, int nx, int ny, const nn::BrickSetJobs jobs)
+    // set j reads; grid: x over b, y: j.  A warp an output brick, its lanes over the rows of
+    // the box (up to about 12 x 8 x 12 bricks; a row is one or two words of bits).  The 8 sets
+    // of a four-level network took 22 launches of 3 to 6 us, a pass per axis and set, on
+    // 256 x 256 x 200 voxels and 103 us on 512 x 512 x 400; with the box read byte by byte one
+    // launch of 22 and 264 us, with the bits 17 and 78 us in two.
+    __global__ void brickSetsKernel(const uint32_t* __restrict__ bits, int words, int ny, const nn::BrickSetJobs jobs)
     {
         const int j = static_cast<int>(blockIdx.y);
         const int ox = jobs.count[j][0], oy = jobs.count[j][1];
@@ -831,13 +848,18 @@ namespace {
         const int lane = threadIdx.x & 31, warps = static_cast<int>(gridDim.x * blockDim.x) >> 5;
         for (int o = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x) >> 5; o < total; o += warps) {
             const int2 x = rx[o % ox], y = ry[(o / ox) % oy], z = rz[o / (ox * oy)];
-            const int ey = y.y - y.x + 1, rows = ey > 0 ? ey * (z.y - z.x + 1) : 0;
-            unsigned v = 0u;
+            const int ey = y.y - y.x + 1, rows = ey > 0 && x.y >= x.x ? ey * (z.y - z.x + 1) : 0;
+            uint32_t v = 0u;
             for (int i = lane; i < rows; i += 32) {
-                const uint8_t* row = in + (static_cast<size_t>(z.x + i / ey) * ny + y.x + i % ey) * nx;
-#pragma unroll 4
-                for (int c = x.x; c <= x.y; ++c)
-                    v |= row[c];
+                const uint32_t* row = bits + (static_cast<size_t>(z.x + i / ey) * ny + y.x + i % ey) * words;
+                for (int w = x.x >> 5; w <= x.y >> 5; ++w) {
+                    uint32_t m = 0xffffffffu;
+                    if (w == x.x >> 5)
+                        m &= 0xffffffffu << (x.x & 31);
+                    if (w == x.y >> 5)
+                        m &= 0xffffffffu >> (31 - (x.y & 31));
+                    v |= row[w] & m;
+                }
             }
             v = __any_sync(0xffffffffu, v != 0u);
             if (lane == 0)
@@ -940,17 +962,26 @@ namespace nn {
         count[2] = (D + zt - 1) / zt;
     }
 
-    cudaError_t launchBrickSets(const uint8_t* in, const int inCount[3], const BrickSetJobs& jobs, cudaStream_t s)
+    size_t brickBitWords(const int count[3])
+    {
+        return static_cast<size_t>((count[0] + 31) / 32) * count[1] * count[2];
+    }
+
+    cudaError_t launchBrickSets(const uint8_t* in, const int inCount[3], uint32_t* bits, const BrickSetJobs& jobs,
+        cudaStream_t s)
     {
         if (jobs.n == 0)
             return cudaSuccess;
-        if (!in || inCount[0] < 1 || inCount[1] < 1 || inCount[2] < 1 || jobs.n > kMaxBrickLists)
+        if (!in || !bits || inCount[0] < 1 || inCount[1] < 1 || inCount[2] < 1 || jobs.n > kMaxBrickLists)
             return cudaErrorInvalidValue;
+        const int words = static_cast<int>(brickBitWords(inCount));
+        brickBitsKernel<<<std::min((words + 127) / 128, 4096), 128, 0, s>>>(in, inCount[0], inCount[1] * inCount[2],
+            bits);
         int most = 1;
         for (int j = 0; j < jobs.n; ++j)
             most = std::max(most, jobs.count[j][0] * jobs.count[j][1] * jobs.count[j][2]);
-        brickSetsKernel<<<dim3(std::min((most + 7) / 8, 1024), jobs.n), 256, 0, s>>>(in, inCount[0], inCount[1],
-            jobs);
+        brickSetsKernel<<<dim3(std::min((most + 7) / 8, 1024), jobs.n), 256, 0, s>>>(bits, (inCount[0] + 31) / 32,
+            inCount[1], jobs);
         return cudaGetLastError();
     }
 

@@ -57,6 +57,7 @@ struct dxmcg_denoiser {
     // the bricks that the tissue bricks need), two scratch masks and the brick ranges
     // that map the tissue bricks onto those grids
     DevBuf<uint8_t> mask0[2], mask1[2], mask2[2], maskEnc[3];
+    DevBuf<uint32_t> maskBits;
     DevBuf<int> list0[2], list1[2], list2[2], listEnc[3], listLens, encRanges;
     std::vector<int> encRangesHost;
     cudaStream_t side = nullptr; // the zeros of a dose that lies in host memory
@@ -677,7 +678,8 @@ namespace nn {
             }
             NN_CUDA(cudaMemcpyAsync(d->encRanges.p, d->encRangesHost.data(), nRanges * sizeof(int),
                 cudaMemcpyHostToDevice, s));
-            NN_CUDA(launchBrickSets(d->mask0[0].p, count, sets, s));
+            NN_CUDA(d->maskBits.reserve(brickBitWords(count)));
+            NN_CUDA(launchBrickSets(d->mask0[0].p, count, d->maskBits.p, sets, s));
             NN_CUDA(launchBrickLists(lists, s));
         }
         if ((rc = forward(d, d->worldInput.p, s, nullptr, direct ? direct : d->worldOut.p, scale, sparse ? &sp : nullptr)) != DXMCG_OK)

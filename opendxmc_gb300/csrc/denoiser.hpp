@@ -81,7 +81,8 @@ void conv3TcBrickDims(int D, int H, int W, int Cout, int brick[3], int count[3])
 //             union over marked bricks (cx, cy, cz) of the boxes X(cx) x Y(cy) x Z(cz), where
 //             `ranges` (device) holds for each output brick index b along x, then y, then z,
 //             the range [lo, hi] of input brick indices whose interval holds b (lo > hi:
-//             none); up to kMaxBrickLists sets in one launch;
+//             none); up to kMaxBrickLists sets at once (bits: brickBitWords(inCount) words
+//             of scratch);
 //   list:     the marked indices in increasing order, and how many (*listLen);
 //             launchBrickLists compacts up to kMaxBrickLists masks in one launch.
 constexpr int kMaxBrickLists = 12;
@@ -91,7 +92,9 @@ struct BrickSetJobs {
     int count[kMaxBrickLists][3] = {};
     int n = 0;
 };
-cudaError_t launchBrickSets(const uint8_t* in, const int inCount[3], const BrickSetJobs& jobs, cudaStream_t s);
+size_t brickBitWords(const int count[3]);
+cudaError_t launchBrickSets(const uint8_t* in, const int inCount[3], uint32_t* bits, const BrickSetJobs& jobs,
+    cudaStream_t s);
 cudaError_t launchBrickList(const uint8_t* mask, int nb, int* list, int* listLen, cudaStream_t s);
 struct BrickListJobs {
     const uint8_t* mask[kMaxBrickLists] = {};
