@@ -166,7 +166,7 @@ typedef struct {
     uint64_t hist_begin;  /* history range [begin, end) of the beam; end 0 = all */
     uint64_t hist_end;
     int32_t interact_batch; /* parked scatterings a warp gathers before sampling them, 0 = default */
-    int32_t refill_batch;   /* dead lanes a warp gathers before starting new histories, 0 = default */
+    int32_t refill_batch;   /* free photon slots a warp gathers before starting new histories, 0 = default */
     int32_t macro_cell;     /* MACRO tracking: cell edge in voxels, 0 = default (16) */
     int32_t woodcock_steps; /* WOODCOCK tracking: steps a lane takes between regroupings, 0 = default:
                              * 1.4 / p clamped to 4..16, p = stops per step of the world's
@@ -277,10 +277,11 @@ DXMCG_API int dxmcg_world_packed_density(dxmcg_world* w, float* density, uint8_t
 DXMCG_API int dxmcg_transport_run(dxmcg_world* w, const dxmcg_beam* beam, const dxmcg_run_options* opts,
     dxmcg_progress* progress, dxmcg_stats* stats);
 
-/* ---- batches: many (world, beam) jobs in one persistent launch --------------
+/* ---- batches: many (world, beam) jobs in one graph --------------------------
  * No counterpart in the reference, which runs one beam per Transport call
- * (simulationpipeline.cpp:165).  All jobs draw from one shared history queue, so
- * a batch of small or uneven jobs keeps every SM busy until the last history.
+ * (simulationpipeline.cpp:165).  Every job is a launch of its own, large jobs on a
+ * few streams and small ones side by side, so that a batch of small or uneven jobs
+ * keeps the SMs busy until the last history.
  * Job j runs histories 0..N_j-1 of beams[j] with opts[j].seed and opts[j].stream
  * and deposits into worlds[j]'s tally: the same histories, hence the same tallies
  * up to the summation order, as dxmcg_transport_run(worlds[j], beams + j,
@@ -289,7 +290,7 @@ DXMCG_API int dxmcg_transport_run(dxmcg_world* w, const dxmcg_beam* beam, const 
  * jobs (launch shape from opts[0]), hist_begin = hist_end = 0, one macro_cell
  * per world.  Exposures, spectra and calibrations are fixed at create time; the
  * worlds must outlive the batch and must not run other transports meanwhile.
- * The first dxmcg_batch_run captures a CUDA graph (counter reset + the launch)
+ * The first dxmcg_batch_run captures a CUDA graph (counter resets + the launches)
  * that every later run replays; each run adds N_j histories to world j's dose
  * normalisation.  stats are summed over all jobs (calibration: job 0's). */
 typedef struct dxmcg_batch dxmcg_batch;
@@ -409,8 +410,8 @@ typedef struct {
     int32_t channels[5]; /* per level, multiples of 16; channels[0] 16 or 32 */
     uint64_t seed;       /* He-normal initialisation */
     int32_t conv_path;   /* 3x3x3 convolutions: 0 = default: tcgen05 tensor cores with
-                            accumulators in tensor memory, except a launch whose grid would
-                            leave SMs idle (fewer output bricks than SMs), which takes mma.sync;
+                            accumulators in tensor memory, except a launch whose grid leaves
+                            SMs idle even in mma.sync's smallest bricks, which takes mma.sync;
                             1 = tcgen05 for every convolution; 2 = warp-level mma.sync */
 } dxmcg_denoiser_config;
 DXMCG_API int dxmcg_denoiser_create(const dxmcg_denoiser_config* config, dxmcg_denoiser** out);

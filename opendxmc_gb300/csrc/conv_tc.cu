@@ -685,11 +685,11 @@ namespace {
     // The brick shape of a grid: wholeShape where that has a CTA for every SM, else the thinner
     // bricks or narrower tiles that need the least time: bricks a CTA times zt + 3 (ZT + 2
     // planes of MMAs and about one more for the hand-over), times 6 at 32 channels and 5 at 16
-    // (a slice took 3.0, 1.8 and 1.4 us at 32 channels, 2.3, 1.5 and 1.15 us at 16).  Thin bricks re-read more halo, so they lose
-    // once the SMs are full: 8 x 64^3 voxels keep wholeShape.  Network, in wholeShape / this
-    // way: 32^3 voxels of level 1 (32 channels) 78 -> 43 us for its four convolutions (mma.sync
-    // with its pooling pass 107), 8 x 16^3 of level 2 (64 channels) 105 -> 74 us (180),
-    // 8 x 8^3 of level 3 51 -> 31 us (56).
+    // (a slice took 3.0, 1.8 and 1.4 us at 32 channels, 2.3, 1.5 and 1.15 us at 16).  Thin
+    // bricks re-read more halo, so they lose once the SMs are full: 8 x 64^3 voxels keep wholeShape.  The convolutions of a level, in
+    // bricks of 8 slices -> this way: 32^3 voxels of level 1 (32 channels) 70 -> 43 us (mma.sync
+    // with its pooling pass 107), 8 x 16^3 of level 2 (64 channels) 105 -> 74 us (180), 8 x 8^3
+    // of level 3 51 -> 31 us (56).
     TcShape shapeFor(int B, int D, int H, int W, int Cout)
     {
         const int sms = nn::smCount();
