@@ -428,13 +428,14 @@ namespace {
 
 namespace {
     // kernel instance for a tracking mode on the packed (world) or unpacked
-    // (caller-owned arrays) voxel layout with n_mats materials; nullptr where no instance
+    // (caller-owned arrays) voxel layout with n_mats materials, with or without the gather
+    // skip's cell bounds, at correction level 2 (bound) or below; nullptr where no instance
     // exists
-    TransportFn kernelFor(int tracking, bool packed, int n_mats)
+    TransportFn kernelFor(int tracking, bool packed, int n_mats, bool skip, bool bound)
     {
         switch (tracking) {
-        case DXMCG_TRACK_WOODCOCK: return woodcockKernelFor(packed, false, n_mats);
-        case kTrackWoodcockBox: return woodcockKernelFor(packed, true, n_mats);
+        case DXMCG_TRACK_WOODCOCK: return woodcockKernelFor(packed, false, n_mats, skip, bound);
+        case kTrackWoodcockBox: return woodcockKernelFor(packed, true, n_mats, skip, bound);
         case DXMCG_TRACK_SIDDON:
             return packed ? transportKernel<DXMCG_TRACK_SIDDON, true> : transportKernel<DXMCG_TRACK_SIDDON, false>;
         case DXMCG_TRACK_MACRO: return packed ? transportKernel<DXMCG_TRACK_MACRO, true> : nullptr;
@@ -447,7 +448,8 @@ namespace {
     {
         const int tracking = kernelTracking(job);
         const bool woodcock = tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox;
-        const TransportFn fn = kernelFor(tracking, packed, job.n_mats);
+        const TransportFn fn = kernelFor(tracking, packed, job.n_mats, job.cbound != nullptr,
+            job.correction >= 2);
         if (!fn)
             return cudaErrorInvalidValue;
         const int refill = shape.refill_batch > 0 ? shape.refill_batch : (woodcock ? kWoodcockRefillBatch : 8);
@@ -464,7 +466,7 @@ namespace {
     {
         int n = 0;
         const bool woodcock = tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox;
-        const TransportFn fn = kernelFor(tracking, packed, kSharedTableMaterials);
+        const TransportFn fn = kernelFor(tracking, packed, kSharedTableMaterials, false, true);
         const size_t smem = woodcock ? woodcockSharedBytes(block, kSharedTableMaterials) : 0;
         if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) != cudaSuccess)
             return 1;
@@ -491,7 +493,7 @@ int transportMaxBlocksPerSM(int block, int tracking) { return residentBlocks(tra
 int transportRegistersPerThread(int tracking)
 {
     cudaFuncAttributes a {};
-    const TransportFn fn = kernelFor(tracking, true, kSharedTableMaterials);
+    const TransportFn fn = kernelFor(tracking, true, kSharedTableMaterials, false, true);
     return fn && cudaFuncGetAttributes(&a, fn) == cudaSuccess ? a.numRegs : -1;
 }
 

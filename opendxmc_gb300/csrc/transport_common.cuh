@@ -93,7 +93,7 @@ using TransportFn = void (*)(const DevJob, unsigned long long, DevCounters*, int
 
 // woodcock.cu: the Woodcock kernel's instance for a voxel layout, one region or two and
 // n_mats materials; its dynamic shared memory at a block size; its default batch sizes
-TransportFn woodcockKernelFor(bool packed, bool box, int n_mats);
+TransportFn woodcockKernelFor(bool packed, bool box, int n_mats, bool skip, bool bound);
 size_t woodcockSharedBytes(int block, int n_mats);
 extern const int kWoodcockRefillBatch, kWoodcockInteractBatch;
 // materials whose attenuation tables a block holds in shared memory: with the photon

@@ -90,7 +90,7 @@ namespace {
     // collision in voxel v / material m, kFree outside the grid, kOuter when a virtual
     // collision lies outside the two-region box (BOX), else kFly.
     //
-    // Gather skip (J.cbound set): the tentative collision is real when u mu_max(E) <
+    // Gather skip (SKIP, J.cbound set): the tentative collision is real when u mu_max(E) <
     // rho mu_m(E).  The cell's bound b_c satisfies rho mu_m(E) <= b_c mu_max(E) for each
     // of its voxels, with a margin larger than the FP32 roundings of both sides, so
     // u mu_max >= b_c mu_max settles the step as virtual without reading the voxel.
@@ -102,7 +102,7 @@ namespace {
     // BOX: a flight that ends outside the box decides its tentative collision as usual
     // (maj bounds every voxel); the flights after it are outerFlight's, and `packed` is
     // marked.
-    template <bool PACKED, bool BOX, bool TAB>
+    template <bool PACKED, bool BOX, bool TAB, bool SKIP>
     __device__ __forceinline__ int woodcockStep(const DevJob& J, const float* sTot, Photon& ph, Rng& rng,
         const EnergyCache& ec, unsigned& packed, uint32_t& v, int& m, unsigned& visits, unsigned& skipped)
     {
@@ -112,12 +112,12 @@ namespace {
             return kFree;
         ++visits;
         v = static_cast<uint32_t>(ix + J.nx * (iy + J.ny * iz));
-        const bool left = BOX && J.boxOn && outsideBox(J, ix, iy, iz);
+        const bool left = BOX && outsideBox(J, ix, iy, iz);
         if (left)
             packed |= kPackOuter;
         const int on = left ? kOuter : kFly;
         float t = -1.0f;
-        if (J.cbound) {
+        if (SKIP) {
             const float b = __ldg(J.cbound
                 + ((ix >> kCellShift) + J.cb[0] * ((iy >> kCellShift) + J.cb[1] * (iz >> kCellShift))));
             if (b <= FLT_MAX) {
@@ -132,7 +132,7 @@ namespace {
         if (m == DXMCG_TRANSPARENT_MATERIAL)
             return on;
         const float mu = rho * attenuation<TAB>(J, sTot, m, ec);
-        if (!(t >= 0.0f))
+        if (!SKIP || !(t >= 0.0f))
             t = rng.u() * ec.mmax;
         return t < mu ? kPark : on;
     }
@@ -204,7 +204,12 @@ namespace {
     constexpr size_t kPoolBytes = kSlots * 64 + 6 * 32 * sizeof(float) + 10 * sizeof(unsigned long long);
 
     // TAB: the block keeps the job's attenuation tables in shared memory, behind the pools.
-    template <bool PACKED, bool BOX, bool TAB>
+    // SKIP: with cell bounds (J.cbound).  BOUND: correction level 2 (Doppler-broadened
+    // Compton, fluorescence).  An instance each: asked at run time, the cell bounds and the
+    // level-2 samplers held registers (the steps spilled) and issue slots where they are off.
+    // 1e7 histories of the DX cylinder 1.26 -> 1.18 ms, 2e8 of the torso 24.9 -> 23.2, 3e8 of
+    // the 512 x 512 x 400 torso 53.3 -> 51.2, 1e7 of a level-2 CBCT 3.65 -> 3.32.
+    template <bool PACKED, bool BOX, bool TAB, bool SKIP, bool BOUND>
     __global__ void __launch_bounds__(256, 4) woodcockKernel(const DevJob J, unsigned long long h_end,
         DevCounters* __restrict__ ctr, int refillBatch, int interactBatch, int woodcockSteps)
     {
@@ -298,7 +303,7 @@ namespace {
                     if (entered) {
                         gridPos(ph.E, ec.ie, ec.fe);
                         packed |= static_cast<unsigned>(ec.ie);
-                        if (BOX && J.boxOn
+                        if (BOX
                             && outsideBox(J, __float2int_rd(ph.px * J.isp[0]), __float2int_rd(ph.py * J.isp[1]),
                                 __float2int_rd(ph.pz * J.isp[2])))
                             packed |= kPackOuter;
@@ -350,7 +355,7 @@ namespace {
                     photo = rt < pe;
                     compton = !photo && rt < pe + ic;
                     rayleigh = !photo && !compton;
-                    const bool atomic = photo && J.correction >= 2; // may emit fluorescence
+                    const bool atomic = BOUND && photo; // may emit fluorescence
                     error = (!photo || atomic) && (packed >> kPackSteps) > J.maxSteps;
                     if (error) {
                         err |= kErrStepLimit;
@@ -358,9 +363,9 @@ namespace {
                         float Ep = ph.E;
                         if (!photo) {
                             float cost;
-                            if (J.correction >= 2 && compton) {
+                            if (BOUND && compton) {
                                 Ep = sampleCompton(ph.E, J.mats + pm, J.ctab + pm * (kTableNE * kCTabK), ec.ie, ec.fe,
-                                    J.correction, rng, cost, err);
+                                    2, rng, cost, err);
                             } else {
                                 // one path for both: the angle from the kind's quantile table
                                 const float omu = oneMinusCos((compton ? J.ctab : J.rtab) + pm * (kTableNE * kCTabK),
@@ -460,7 +465,7 @@ namespace {
                 }
                 for (int k = 0;;) {
                     if (to == kFly) {
-                        to = woodcockStep<PACKED, BOX, TAB>(J, sTot, ph, rng, ec, packed, v, m, visits, skipped);
+                        to = woodcockStep<PACKED, BOX, TAB, SKIP>(J, sTot, ph, rng, ec, packed, v, m, visits, skipped);
                         packed += 1u << kPackSteps;
                     }
                     if (++k >= woodcockSteps || __popc(__ballot_sync(kFull, to == kFly)) <= (n >> 1))
@@ -513,22 +518,30 @@ namespace {
         }
     }
 
-    template <bool PACKED, bool BOX>
-    TransportFn instance(bool tab)
+    template <bool PACKED, bool BOX, bool TAB, bool SKIP>
+    TransportFn byLevel(bool bound)
     {
-        return tab ? woodcockKernel<PACKED, BOX, true> : woodcockKernel<PACKED, BOX, false>;
+        return bound ? woodcockKernel<PACKED, BOX, TAB, SKIP, true> : woodcockKernel<PACKED, BOX, TAB, SKIP, false>;
+    }
+    template <bool PACKED, bool BOX>
+    TransportFn instance(bool tab, bool skip, bool bound)
+    {
+        if constexpr (PACKED) // the unpacked layout has no cell bounds
+            if (skip)
+                return tab ? byLevel<true, BOX, true, true>(bound) : byLevel<true, BOX, false, true>(bound);
+        return tab ? byLevel<PACKED, BOX, true, false>(bound) : byLevel<PACKED, BOX, false, false>(bound);
     }
 } // namespace
 
 // lanes a warp wants of a kind before it runs that kind's phase
 extern const int kWoodcockRefillBatch = 28, kWoodcockInteractBatch = 28;
 
-TransportFn woodcockKernelFor(bool packed, bool box, int n_mats)
+TransportFn woodcockKernelFor(bool packed, bool box, int n_mats, bool skip, bool bound)
 {
     const bool tab = n_mats <= kSharedTableMaterials;
     if (packed)
-        return box ? instance<true, true>(tab) : instance<true, false>(tab);
-    return box ? instance<false, true>(tab) : instance<false, false>(tab);
+        return box ? instance<true, true>(tab, skip, bound) : instance<true, false>(tab, skip, bound);
+    return box ? instance<false, true>(tab, false, bound) : instance<false, false>(tab, false, bound);
 }
 
 size_t woodcockSharedBytes(int block, int n_mats)
