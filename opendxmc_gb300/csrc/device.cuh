@@ -92,6 +92,26 @@ namespace dev {
         return fmaf(f, ab.y - ab.x, ab.x);
     }
 
+    // Correctly rounded 1 / x and sqrt(x) for 2^-112 <= x < 2^107 (and sqrt(0) = 0): the
+    // hardware's approximation and one Newton step in fused arithmetic (Markstein, IBM J.
+    // Res. Dev. 34, 111, 1990).  Without the library forms' range tests and slow paths; the
+    // same bits as those for every float of that range.  In the interactions and majorants: 1e7
+    // histories of the DX cylinder 1.18 -> 1.15 ms, 2e8 of the torso 23.2 -> 22.5 ms.
+    __device__ __forceinline__ float reciprocal(float x)
+    {
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+        return __fmaf_rn(__fmaf_rn(-x, r, 1.0f), r, r);
+    }
+    __device__ __forceinline__ float squareRoot(float x)
+    {
+        float y;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        const float g = __fmul_rn(x, y);
+        const float s = __fmaf_rn(__fmaf_rn(-g, g, x), __fmul_rn(0.5f, y), g);
+        return x > 0.0f ? s : 0.0f;
+    }
+
     // ---------------------------------------------------------------- samplers
     constexpr float kCutoffKeV = 1.0f; // photons below this energy are absorbed on the spot
     constexpr int kPzTries = 32;       // electron-momentum draws per accepted scattering angle
@@ -232,7 +252,7 @@ namespace dev {
                     continue;
                 return Ep;
             }
-            return E * __frcp_rn(ratio);
+            return E * reciprocal(ratio);
         }
         err |= kErrRejectLimit;
         cost = 1.0f;
@@ -304,7 +324,7 @@ namespace dev {
     __device__ __forceinline__ void isotropicDirection(float& dx, float& dy, float& dz, float u1, float u2)
     {
         const float ct = 2.0f * u1 - 1.0f;
-        const float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
+        const float st = squareRoot(fmaxf(0.0f, 1.0f - ct * ct));
         float sp, cp;
         sincospif(2.0f * u2, &sp, &cp);
         dx = st * cp;
@@ -314,7 +334,7 @@ namespace dev {
 
     __device__ __forceinline__ void scatterDirection(float& dx, float& dy, float& dz, float cost, float phiU)
     {
-        const float sint = sqrtf(fmaxf(0.0f, 1.0f - cost * cost));
+        const float sint = squareRoot(fmaxf(0.0f, 1.0f - cost * cost));
         float sp, cp;
         sincospif(2.0f * phiU, &sp, &cp);
         float nx, ny, nz;
@@ -323,13 +343,14 @@ namespace dev {
             ny = sint * sp;
             nz = (dz > 0.0f ? 1.0f : -1.0f) * cost;
         } else {
-            const float tmp = sqrtf(1.0f - dz * dz);
-            const float it = 1.0f / tmp;
+            const float tmp = squareRoot(1.0f - dz * dz);
+            const float it = reciprocal(tmp);
             nx = sint * (dx * dz * cp - dy * sp) * it + dx * cost;
             ny = sint * (dy * dz * cp + dx * sp) * it + dy * cost;
             nz = -sint * cp * tmp + dz * cost;
         }
-        const float inv = rsqrtf(nx * nx + ny * ny + nz * nz);
+        float inv; // of about 1, not subnormal
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(nx * nx + ny * ny + nz * nz));
         dx = nx * inv;
         dy = ny * inv;
         dz = nz * inv;
@@ -523,7 +544,7 @@ namespace dev {
         const float ay = (2.0f * r.u() - 1.0f) * q3.y;
         // |angle| < pi/2: the hardware sine is within 2^-21.4
         const float sx = __sinf(ax), sy = __sinf(ay);
-        const float sz = sqrtf(fmaxf(0.0f, 1.0f - sx * sx - sy * sy));
+        const float sz = squareRoot(fmaxf(0.0f, 1.0f - sx * sx - sy * sy));
         const float4 q0 = __ldg(ex4), q1 = __ldg(ex4 + 1), q2 = __ldg(ex4 + 2);
         ph.dx = q0.w * sx + q1.z * sy + q2.y * sz;
         ph.dy = q1.x * sx + q1.w * sy + q2.z * sz;

@@ -42,8 +42,8 @@ namespace {
     constexpr int kSumSource = 0, kSumEscaped = 1, kSumDeposited = 2; // per-lane energy sums
 
     // The photon's energy-grid position and the majorant its next flight steps against.
-    // __frcp_rn is the correctly rounded 1 / mmax, as a division gives, in fewer
-    // instructions.
+    // reciprocal is the correctly rounded 1 / mmax, as a division gives (tables hold 1e-30 or
+    // more).
     struct EnergyCache {
         int ie;
         float fe, mmax, invMmax;
@@ -55,7 +55,7 @@ namespace {
         __device__ __forceinline__ void setMajorant(const float2* maj)
         {
             mmax = lerp1(maj, ie, fe);
-            invMmax = __frcp_rn(mmax);
+            invMmax = reciprocal(mmax);
         }
     };
 

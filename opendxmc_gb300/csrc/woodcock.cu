@@ -372,7 +372,7 @@ namespace {
                                     ec.ie, ec.fe, rng.u());
                                 cost = 1.0f - omu;
                                 if (compton)
-                                    Ep = ph.E * __frcp_rn(comptonRatio(ph.E, omu));
+                                    Ep = ph.E * reciprocal(comptonRatio(ph.E, omu));
                             }
                             scatterDirection(ph.dx, ph.dy, ph.dz, cost, rng.u());
                             alive = true;
