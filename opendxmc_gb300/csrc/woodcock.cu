@@ -186,12 +186,13 @@ namespace {
     // order from its own stream, so its result does not depend on when, or in which lane,
     // its phases run.
     //
-    // Issue bounds the kernel (about 85 % of the issue slots in steady state, 116 to 131
-    // warp instructions a history), with the L1/shared pipe next (28 to 30 wavefronts a
-    // history).  Against one photon per lane, parked in registers until enough lanes of a
+    // Issue bounds the kernel (about 85 % of the issue slots in steady state, 117 warp
+    // instructions a history of the torso), with the L1/shared pipe next (28 to 30
+    // wavefronts a history).  Against one photon per lane, parked in registers until enough lanes of a
     // warp waited: 13 -> 23 active lanes an instruction; 2e8 histories of the 256x256x200
     // torso 34.9 -> 26.0 ms, 3e8 of the 512x512x400 torso 67.7 -> 54.7 ms, 1e7 of the DX
-    // cylinder 1.48 -> 1.26 ms.  Measured beside it: stacks of slot numbers in place of
+    // cylinder 1.48 -> 1.26 ms (with the instances below and shorter arithmetic since: 22.5,
+    // 50.1 and 1.15).  Measured beside it at that time: stacks of slot numbers in place of
     // moved photons (random slots conflict 2.5-fold: 25.9 / 53.5 / 1.33 ms), slots bound to
     // lanes by residue (no conflicts, fuller warps lost: 27.4 / 56.8 / 1.37 ms), 48
     // registers for 40 warps (spills: 33.5 ms), three blocks an SM (27.8 / 60.9 / 1.33 ms).
