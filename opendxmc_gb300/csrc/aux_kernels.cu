@@ -205,6 +205,7 @@ namespace {
     // voxels a thread, 16-byte stores.  Eight worlds of 0.7-1.4 million voxels into device
     // memory: 594 -> 168 us in all; 105 million voxels: 7.2 -> 1.53 ms (0.94 at the
     // copy rate).  Into pinned host memory the link bounds it, 193 GB/s, as a copy measures.
+    // A thread does its V voxels and no more: the grid grows with the world.
     template <bool VEC>
     __global__ void finalizeKernel(const Tally* __restrict__ t, const uint32_t* __restrict__ vox, size_t n,
         DoseScale scale, double nh, double invNh, double* __restrict__ dose, double* __restrict__ var,
@@ -429,12 +430,16 @@ cudaError_t launchFinalize(const Tally* tally, const uint32_t* vox, size_t n, Do
                           | reinterpret_cast<uintptr_t>(count))
                          & 15u)
         == 0u;
+    // fewer than 2^32 voxels: at most 2^24 blocks
+    const size_t blocks = std::max<size_t>(((vec ? (n + 1) / 2 : n) + 255) / 256, 1);
+    if (blocks > INT_MAX)
+        return cudaErrorInvalidValue;
     if (vec)
-        finalizeKernel<true><<<gridFor((n + 1) / 2, 256), 256, 0, s>>>(tally, vox, n, scale, n_histories, inv, dose,
-            var, count);
+        finalizeKernel<true><<<static_cast<unsigned>(blocks), 256, 0, s>>>(tally, vox, n, scale, n_histories, inv,
+            dose, var, count);
     else
-        finalizeKernel<false><<<gridFor(n, 256), 256, 0, s>>>(tally, vox, n, scale, n_histories, inv, dose, var,
-            count);
+        finalizeKernel<false><<<static_cast<unsigned>(blocks), 256, 0, s>>>(tally, vox, n, scale, n_histories, inv,
+            dose, var, count);
     return cudaGetLastError();
 }
 
