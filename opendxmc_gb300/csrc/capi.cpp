@@ -553,6 +553,12 @@ bool hostPagesOnDevice(std::initializer_list<const void*> arrays)
         && access && tables;
 }
 
+bool overlap(const void* a, size_t na, const void* b, size_t nb)
+{
+    const auto x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + nb && y < x + na;
+}
+
 // maps the pages of a buffer (of one that is to be written: by a write, as a read would map
 // the page of zeros that all fresh memory shares)
 template <bool WRITE, class T>
@@ -1623,7 +1629,13 @@ DXMCG_API int dxmcg_ct_segment(const dxmcg_segmentation* table, const double* hu
     const uint8_t* lutM = nullptr;
     if ((rc = segLut(t, lutD, lutM)) != DXMCG_OK)
         return rc;
-    if (hostPagesOnDevice({ hu, material, density }))
+    // touching an output's pages writes to them, and the kernel takes its arrays as distinct:
+    // arrays that share memory (a segmentation in place) go by the copies, a chunk's input
+    // taken before its outputs are written
+    const size_t wide = n * sizeof(double);
+    const bool shared = overlap(hu, wide, density, wide) || overlap(hu, wide, material, n)
+        || overlap(density, wide, material, n);
+    if (!shared && hostPagesOnDevice({ hu, material, density }))
         return segmentInPlace(t, lutD, lutM, hu, n, material, density);
     const size_t chunk = std::min<uint64_t>(n, kStreamChunk);
     DeviceBuffer<double> dh, dd;
