@@ -1635,7 +1635,10 @@ DXMCG_API int dxmcg_ct_segment(const dxmcg_segmentation* table, const double* hu
     const size_t wide = n * sizeof(double);
     const bool shared = overlap(hu, wide, density, wide) || overlap(hu, wide, material, n)
         || overlap(density, wide, material, n);
-    if (!shared && hostPagesOnDevice({ hu, material, density }))
+    // the kernel reads and writes doubles whole; a copy takes them from any address
+    const bool aligned
+        = (reinterpret_cast<uintptr_t>(hu) | reinterpret_cast<uintptr_t>(density)) % alignof(double) == 0;
+    if (!shared && aligned && hostPagesOnDevice({ hu, material, density }))
         return segmentInPlace(t, lutD, lutM, hu, n, material, density);
     const size_t chunk = std::min<uint64_t>(n, kStreamChunk);
     DeviceBuffer<double> dh, dd;
