@@ -330,6 +330,9 @@ namespace {
                 if (ok && sl == 0 && k >= 2)
                     ok = umma::mbarWaitOrAbort(&accEmpty[set], static_cast<uint32_t>((k >> 1) - 1) & 1u, hp,
                         abortp);
+                // every lane waited for itself: the warp stays or leaves as one, as the lanes
+                // that stay meet in the barrier below
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok)
                     break;
                 umma::fenceAfterSync();
@@ -535,7 +538,9 @@ namespace {
                         }
                     }
                 }
-                if (!umma::mbarWaitOrAbort(&accFull[set], static_cast<uint32_t>(k >> 1) & 1u, hp, abortp)) {
+                const bool there
+                    = umma::mbarWaitOrAbort(&accFull[set], static_cast<uint32_t>(k >> 1) & 1u, hp, abortp);
+                if (!__all_sync(0xffffffffu, there)) { // the whole warp takes part in the loads below
                     *abortp = 1;
                     break;
                 }
