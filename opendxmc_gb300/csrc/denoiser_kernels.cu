@@ -584,14 +584,16 @@ namespace {
             atomicAdd(dhw + C0, gb);
         }
         __syncthreads();
-        if (threadIdx.x < C0 + 1) {
+        if (threadIdx.x < C0) {
             float v = 0.0f;
             for (int w = 0; w < 8; ++w)
                 v += part[w][threadIdx.x];
-            if (threadIdx.x < C0)
-                atomicAdd(dhw + threadIdx.x, v);
-            else
-                atomicAdd(lossSum, static_cast<double>(v));
+            atomicAdd(dhw + threadIdx.x, v);
+        } else if (threadIdx.x == C0) { // the loss: in FP64 from the warps' sums on
+            double v = 0.0;
+            for (int w = 0; w < 8; ++w)
+                v += static_cast<double>(part[w][C0]);
+            atomicAdd(lossSum, v);
         }
     }
 
