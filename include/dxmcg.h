@@ -279,9 +279,9 @@ DXMCG_API int dxmcg_transport_run(dxmcg_world* w, const dxmcg_beam* beam, const 
 
 /* ---- batches: many (world, beam) jobs in one graph --------------------------
  * No counterpart in the reference, which runs one beam per Transport call
- * (simulationpipeline.cpp:165).  Every job is a launch of its own, large jobs on a
- * few streams and small ones side by side, so that a batch of small or uneven jobs
- * keeps the SMs busy until the last history.
+ * (simulationpipeline.cpp:165).  Large jobs are a launch each on a few streams, small
+ * ones share launches, so that a batch of many, small or uneven jobs keeps the SMs
+ * busy until the last history.
  * Job j runs histories 0..N_j-1 of beams[j] with opts[j].seed and opts[j].stream
  * and deposits into worlds[j]'s tally: the same histories, hence the same tallies
  * up to the summation order, as dxmcg_transport_run(worlds[j], beams + j,

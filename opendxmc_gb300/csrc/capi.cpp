@@ -19,6 +19,7 @@
 #include <new>
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include <unistd.h>
@@ -371,23 +372,35 @@ int deviceErrors(const DevCounters& c, const char* what)
 
 } // namespace
 
-// Several (world, beam) jobs, each one launch of the single-job kernel, captured once as a
-// CUDA graph and replayed by each run.  Jobs that average kLargeJob histories or more
-// fill the GPU one after another, on kLargeStreams streams so that one job's blocks take
-// the SMs another job's tail frees; one world at a time keeps its voxels and tally in L2.
-// Smaller jobs would mostly be tails: they run side by side on up to kSmallStreams
-// streams, each with twice its share of the resident blocks, so that blocks of the jobs
-// still running replace those of jobs that are done.  Eight jobs of 1e5 to 2e6 histories,
-// dose read back: 1.19 ms in one launch over a shared queue (whose lanes read their job's
-// descriptor from memory), 1.07 ms side by side.
+// Several (world, beam) jobs, captured once as a CUDA graph and replayed by each run.  Jobs
+// that average kLargeJob histories or more are a launch each and fill the GPU one after
+// another, on kLargeStreams streams so that one job's blocks take the SMs another job's tail
+// frees; one world at a time keeps its voxels and tally in L2.  Smaller jobs would mostly be
+// tails: they share launches (launchTransportPack), each with kSmallShare times its share of
+// the resident blocks, so that blocks of the jobs still to come replace those of jobs that
+// are done.  With a launch a job, on 32 streams, a batch of many jobs was as long as the
+// jobs' longest histories one after another: 512 Woodcock jobs of 1000 histories on 64^3
+// voxels 1.09 ms, this way 0.29; 1024 of 1e4 4.6 and 1.8 ms; eight of 1e5 to 2e6 histories
+// the same.  (Once the share, 64 jobs of 1e5 take 1.51 ms in place of 1.08.)
+// Where Siddon and macro tracking, whose lanes own a photon each, have more than
+// kQueueHistories histories a resident lane, their lanes take the histories of all jobs from
+// one queue (launchTransportQueue): shared launches hold a block until its job's last
+// history.  Siddon, shared launches and the queue: 512 jobs of 1000 (3.3 a lane) 1.25 and
+// 1.41 ms, 1024 of 1000 (6.6) 2.16 and 1.64, 1024 of 1e4 11.5 and 10.3; macro 0.59 and 0.67,
+// 1.00 and 0.77, 5.8 and 4.9.
 constexpr uint64_t kLargeJob = 1ull << 21;
 constexpr int kLargeStreams = 4, kSmallStreams = 32;
+constexpr double kSmallShare = 2.0, kQueueHistories = 5.0;
 
 struct dxmcg_batch {
     int device = 0;
     int tracking = DXMCG_TRACK_WOODCOCK;
     std::vector<DevJob> hostJobs;
     std::vector<LaunchShape> jobShapes;
+    std::vector<std::vector<int>> launches; // jobs of each launch
+    bool queue = false; // one launch over all jobs' histories in one queue
+    DeviceBuffer<DevJob> queueJobs;
+    DeviceBuffer<unsigned long long> queueOffsets;
     DeviceBuffer<DevCounters> jobCounters;
     std::vector<cudaStream_t> side;
     std::vector<cudaEvent_t> join;
@@ -1341,21 +1354,51 @@ DXMCG_API int dxmcg_batch_create(int n_jobs, dxmcg_world* const* worlds, const d
     for (int j = 0; j < n_jobs; ++j)
         if (kernelTracking(J[j]) == kTrackWoodcockBox)
             b->tracking = kTrackWoodcockBox;
-    // the occupancy query also loads the kernel, so the later graph capture loads nothing
     const bool large = b->total >= kLargeJob * static_cast<uint64_t>(n_jobs);
-    const int streams = std::min(n_jobs, large ? kLargeStreams : kSmallStreams);
+    const LaunchShape first = chooseShape(worlds[0], opts[0], kernelTracking(J[0]));
+    b->queue = !large && tracking != DXMCG_TRACK_WOODCOCK
+        && static_cast<double>(b->total) > kQueueHistories * first.grid * first.block;
+    if (b->queue) {
+        std::vector<unsigned long long> off(n_jobs + 1, 0ull);
+        for (int j = 0; j < n_jobs; ++j)
+            off[j + 1] = off[j] + b->nHist[j];
+        DXMCG_CUDA(b->queueJobs.alloc(n_jobs));
+        DXMCG_CUDA(b->queueOffsets.alloc(off.size()));
+        DXMCG_CUDA(cudaMemcpy(b->queueJobs.p, J.data(), n_jobs * sizeof(DevJob), cudaMemcpyHostToDevice));
+        DXMCG_CUDA(cudaMemcpy(b->queueOffsets.p, off.data(), off.size() * sizeof(unsigned long long),
+            cudaMemcpyHostToDevice));
+    }
+    std::map<std::pair<int, int>, std::vector<int>> open; // by kernel instance and block size
     for (int j = 0; j < n_jobs; ++j) {
         LaunchShape sh = chooseShape(worlds[j], opts[j], kernelTracking(J[j]));
-        if (!large) {
-            // twice the job's share of the blocks that run at a time, 128 histories a block
-            // at least
-            const double share = 2.0 * n_jobs / streams * static_cast<double>(b->nHist[j])
+        if (b->queue) {
+            sh = first;
+        } else if (!large) {
+            // 128 histories a block at least
+            const double share = kSmallShare * static_cast<double>(b->nHist[j])
                 / static_cast<double>(std::max<uint64_t>(b->total, 1));
             const double blocks = std::min(std::ceil(sh.grid * share), std::ceil(b->nHist[j] / 128.0));
             sh.grid = static_cast<int>(std::max(1.0, std::min<double>(sh.grid, blocks)));
+            std::vector<int>& o = open[{ transportInstance(J[j]), sh.block }];
+            o.push_back(j);
+            if (static_cast<int>(o.size()) == kMaxPackedJobs) {
+                b->launches.push_back(o);
+                o.clear();
+            }
+        } else {
+            b->launches.push_back({ j });
         }
         b->jobShapes.push_back(sh);
     }
+    for (const auto& o : open)
+        if (!o.second.empty())
+            b->launches.push_back(o.second);
+    // loaded here, so that the later graph capture loads nothing
+    if (b->queue)
+        DXMCG_CUDA(loadTransport(J[0], LaunchKind::kQueue));
+    for (const auto& jobs : b->launches)
+        DXMCG_CUDA(loadTransport(J[jobs[0]], jobs.size() > 1 ? LaunchKind::kPack : LaunchKind::kAlone));
+    const int streams = std::min(static_cast<int>(b->launches.size()), large ? kLargeStreams : kSmallStreams);
     DXMCG_CUDA(b->jobCounters.alloc(n_jobs));
     DXMCG_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
     for (int k = 0; k < streams; ++k) {
@@ -1395,16 +1438,29 @@ DXMCG_API int dxmcg_batch_run(dxmcg_batch* b, dxmcg_stats* stats)
     const int nJobs = static_cast<int>(b->worlds.size());
     if (!b->exec) {
         DXMCG_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        // fork to the side streams, one launch per job round-robin, join
+        // fork to the side streams, the launches round-robin, join
         const int streams = static_cast<int>(b->side.size());
         cudaError_t e = cudaMemsetAsync(b->jobCounters.p, 0, nJobs * sizeof(DevCounters), b->stream);
         if (e == cudaSuccess)
             e = cudaEventRecord(b->fork, b->stream);
         for (int k = 0; k < streams && e == cudaSuccess; ++k)
             e = cudaStreamWaitEvent(b->side[k], b->fork, 0);
-        for (int j = 0; j < nJobs && e == cudaSuccess; ++j)
-            e = launchTransport(b->hostJobs[j], b->nHist[j], b->jobCounters.p + j, b->jobShapes[j],
-                b->side[j % streams]);
+        if (e == cudaSuccess && b->queue)
+            e = launchTransportQueue(b->tracking, b->queueJobs.p, b->queueOffsets.p, nJobs, b->total,
+                b->jobCounters.p, b->jobShapes[0], b->stream);
+        for (size_t k = 0; k < b->launches.size() && e == cudaSuccess; ++k) {
+            const std::vector<int>& jobs = b->launches[k];
+            const cudaStream_t t = b->side[k % streams];
+            if (jobs.size() == 1) {
+                const int j = jobs[0];
+                e = launchTransport(b->hostJobs[j], b->nHist[j], b->jobCounters.p + j, b->jobShapes[j], t);
+                continue;
+            }
+            std::vector<PackedJob> pack;
+            for (int j : jobs)
+                pack.push_back({ &b->hostJobs[j], b->nHist[j], b->jobCounters.p + j, b->jobShapes[j] });
+            e = launchTransportPack(pack.data(), static_cast<int>(pack.size()), t);
+        }
         for (int k = 0; k < streams && e == cudaSuccess; ++k) {
             e = cudaEventRecord(b->join[k], b->side[k]);
             if (e == cudaSuccess)

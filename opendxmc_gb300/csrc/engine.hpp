@@ -256,6 +256,25 @@ cudaError_t launchSampleRayleigh(int n, const float* E, const DevMaterial* m, co
 cudaError_t launchSampleSource(const DevJob& job, unsigned long long h0, int n, float* out8, cudaStream_t s);
 cudaError_t launchHistoryStream(unsigned long long key, unsigned long long h0, int n_hist, int n_draws,
     uint32_t* out, cudaStream_t s);
+// One launch of up to kMaxPackedJobs jobs on packed worlds, whose kernel instance
+// (transportInstance) and block size are one; each with the blocks of its shape's grid.
+struct PackedJob {
+    const DevJob* job;
+    unsigned long long h_end;
+    DevCounters* ctr;
+    LaunchShape shape;
+};
+constexpr int kMaxPackedJobs = 64;
+int transportInstance(const DevJob& job);
+// loads the kernel that launches `job`, alone or with others (packed) or from a queue, so that
+// a later graph capture loads nothing
+enum class LaunchKind { kAlone, kPack, kQueue };
+cudaError_t loadTransport(const DevJob& job, LaunchKind kind);
+cudaError_t launchTransportPack(const PackedJob* jobs, int n, cudaStream_t s);
+// Siddon and macro tracking: one launch over several jobs' histories in one queue, their
+// descriptors and offsets (nJobs + 1: the first history of each, then the total) on the device
+cudaError_t launchTransportQueue(int tracking, const DevJob* jobs, const unsigned long long* offsets, int nJobs,
+    unsigned long long h_end, DevCounters* ctr, LaunchShape shape, cudaStream_t s);
 int transportRegistersPerThread(int tracking);
 int transportMaxBlocksPerSM(int block, int tracking);
 // the same kernel reading caller-owned float density / uint8 material arrays

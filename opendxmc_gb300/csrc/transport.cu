@@ -25,8 +25,10 @@
 // depend on when, or in which lane, each phase runs.
 #include <algorithm>
 #include <cfloat>
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <memory>
 
 #include "transport_common.cuh"
 
@@ -179,10 +181,15 @@ namespace {
         return rng.u() * muc < mu;
     }
 
-    template <int TRACKING, bool PACKED>
-    __global__ void __launch_bounds__(256) transportKernel(const DevJob J, unsigned long long h_end,
-        DevCounters* __restrict__ ctr, int refillBatch, int interactBatch, int)
+    // MULTI: one queue over the concatenated history ranges of nJobs jobs (offsets[j] is the
+    // first global history of job j, offsets[nJobs] the total); each lane reads its job's
+    // descriptor from `jobs`.  Otherwise J0 is the only job.
+    template <int TRACKING, bool PACKED, bool MULTI>
+    __device__ __forceinline__ void transportRun(const DevJob& J0, const DevJob* __restrict__ jobs,
+        const unsigned long long* __restrict__ offsets, int nJobs, unsigned long long h_end,
+        DevCounters* __restrict__ ctr, int refillBatch, int interactBatch)
     {
+        int jid = 0;
         // event counters per warp (no block-wide barrier: warps finish independently)
         __shared__ unsigned long long sCountAll[256 / 32][cNum];
         const unsigned lane = threadIdx.x & 31u;
@@ -231,7 +238,20 @@ namespace {
                 const bool start = st == kDead && rank < avail;
                 bool entered = false;
                 if (start) {
-                    const unsigned long long h = poolNext + rank;
+                    unsigned long long h = poolNext + rank;
+                    if (MULTI) { // the queue spans all jobs: find this history's
+                        int lo = 0, hi = nJobs;
+                        while (hi - lo > 1) {
+                            const int mid = (lo + hi) >> 1;
+                            if (__ldg(offsets + mid) <= h)
+                                lo = mid;
+                            else
+                                hi = mid;
+                        }
+                        jid = lo;
+                        h -= __ldg(offsets + lo);
+                    }
+                    const DevJob& J = MULTI ? jobs[jid] : J0;
                     rng.init(J.key, h);
                     sampleSource(J, h, ph, rng);
                     sum[kSumSource].add(ph.w * ph.E);
@@ -261,6 +281,9 @@ namespace {
                     atomicAdd(&sCount[cMissed], static_cast<unsigned long long>(__popc(mStart & ~mIn)));
                 }
             }
+
+            // the lane's job, after the refill may have changed it
+            const DevJob& J = MULTI ? jobs[jid] : J0;
 
             // ---- interact
             const int nPark = __popc(parked);
@@ -424,6 +447,26 @@ namespace {
         }
     }
 
+    template <int TRACKING, bool PACKED>
+    __global__ void __launch_bounds__(256) transportKernel(const DevJob J, unsigned long long h_end,
+        DevCounters* __restrict__ ctr, int refillBatch, int interactBatch, int)
+    {
+        transportRun<TRACKING, PACKED, false>(J, nullptr, nullptr, 1, h_end, ctr, refillBatch, interactBatch);
+    }
+    template <int TRACKING>
+    __global__ void __launch_bounds__(256) transportPackKernel(const __grid_constant__ JobPack pack)
+    {
+        const JobPack::Entry& e = pack.e[packJob(pack)];
+        transportRun<TRACKING, true, false>(e.job, nullptr, nullptr, 1, e.h_end, e.ctr, e.refill, e.interact);
+    }
+    template <int TRACKING>
+    __global__ void __launch_bounds__(256) transportQueueKernel(const DevJob* __restrict__ jobs,
+        const unsigned long long* __restrict__ offsets, int nJobs, unsigned long long h_end,
+        DevCounters* __restrict__ ctr, int refillBatch, int interactBatch)
+    {
+        transportRun<TRACKING, true, true>(jobs[0], jobs, offsets, nJobs, h_end, ctr, refillBatch, interactBatch);
+    }
+
 } // namespace
 
 namespace {
@@ -443,19 +486,39 @@ namespace {
         }
     }
 
+    // the same for a launch of several jobs, all of one instance
+    PackFn packFor(int tracking, int n_mats, bool skip, bool bound)
+    {
+        switch (tracking) {
+        case DXMCG_TRACK_WOODCOCK: return woodcockPackFor(false, n_mats, skip, bound);
+        case kTrackWoodcockBox: return woodcockPackFor(true, n_mats, skip, bound);
+        case DXMCG_TRACK_SIDDON: return transportPackKernel<DXMCG_TRACK_SIDDON>;
+        case DXMCG_TRACK_MACRO: return transportPackKernel<DXMCG_TRACK_MACRO>;
+        default: return nullptr;
+        }
+    }
+
+    bool isWoodcock(int tracking) { return tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox; }
+
+    // the batch sizes and steps of a shape, defaults filled in
+    void phaseSizes(const LaunchShape& shape, bool woodcock, int& refill, int& interact, int& steps)
+    {
+        refill = shape.refill_batch > 0 ? shape.refill_batch : (woodcock ? kWoodcockRefillBatch : 8);
+        interact = shape.interact_batch > 0 ? shape.interact_batch : (woodcock ? kWoodcockInteractBatch : 8);
+        steps = shape.woodcock_steps > 0 ? shape.woodcock_steps : 8;
+    }
+
     cudaError_t launch(bool packed, const DevJob& job, unsigned long long h_end, DevCounters* ctr, LaunchShape shape,
         cudaStream_t s)
     {
         const int tracking = kernelTracking(job);
-        const bool woodcock = tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox;
+        const bool woodcock = isWoodcock(tracking);
         const TransportFn fn = kernelFor(tracking, packed, job.n_mats, job.cbound != nullptr,
             job.correction >= 2);
         if (!fn)
             return cudaErrorInvalidValue;
-        const int refill = shape.refill_batch > 0 ? shape.refill_batch : (woodcock ? kWoodcockRefillBatch : 8);
-        const int interact
-            = shape.interact_batch > 0 ? shape.interact_batch : (woodcock ? kWoodcockInteractBatch : 8);
-        const int wsteps = shape.woodcock_steps > 0 ? shape.woodcock_steps : 8;
+        int refill = 0, interact = 0, wsteps = 0;
+        phaseSizes(shape, woodcock, refill, interact, wsteps);
         const size_t smem = woodcock ? woodcockSharedBytes(shape.block, job.n_mats) : 0;
         fn<<<shape.grid, shape.block, smem, s>>>(job, h_end, ctr, refill, interact, wsteps);
         return cudaGetLastError();
@@ -465,7 +528,7 @@ namespace {
     int residentBlocks(int tracking, bool packed, int block)
     {
         int n = 0;
-        const bool woodcock = tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox;
+        const bool woodcock = isWoodcock(tracking);
         const TransportFn fn = kernelFor(tracking, packed, kSharedTableMaterials, false, true);
         const size_t smem = woodcock ? woodcockSharedBytes(block, kSharedTableMaterials) : 0;
         if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) != cudaSuccess)
@@ -478,6 +541,75 @@ cudaError_t launchTransport(const DevJob& job, unsigned long long h_end, DevCoun
     cudaStream_t s)
 {
     return launch(true, job, h_end, ctr, shape, s);
+}
+
+int transportInstance(const DevJob& job)
+{
+    const int tracking = kernelTracking(job);
+    if (!isWoodcock(tracking))
+        return tracking;
+    return tracking | (job.n_mats <= kSharedTableMaterials ? 8 : 0) | (job.cbound ? 16 : 0)
+        | (job.correction >= 2 ? 32 : 0);
+}
+
+cudaError_t launchTransportPack(const PackedJob* jobs, int n, cudaStream_t s)
+{
+    if (n < 1 || n > kPackJobs)
+        return cudaErrorInvalidValue;
+    const DevJob& J = *jobs[0].job;
+    const int tracking = kernelTracking(J);
+    const bool woodcock = isWoodcock(tracking);
+    const PackFn fn = packFor(tracking, J.n_mats, J.cbound != nullptr, J.correction >= 2);
+    if (!fn)
+        return cudaErrorInvalidValue;
+    const auto pack = std::make_unique<JobPack>();
+    pack->n = n;
+    int mats = 0;
+    unsigned blocks = 0;
+    for (int k = 0; k < n; ++k) {
+        const PackedJob& p = jobs[k];
+        if (transportInstance(*p.job) != transportInstance(J) || p.shape.block != jobs[0].shape.block
+            || p.shape.grid < 1)
+            return cudaErrorInvalidValue;
+        JobPack::Entry& e = pack->e[k];
+        e.job = *p.job;
+        e.h_end = p.h_end;
+        e.ctr = p.ctr;
+        phaseSizes(p.shape, woodcock, e.refill, e.interact, e.steps);
+        pack->first[k] = blocks;
+        blocks += static_cast<unsigned>(p.shape.grid);
+        mats = std::max(mats, p.job->n_mats);
+    }
+    pack->first[n] = blocks;
+    const size_t smem = woodcock ? woodcockSharedBytes(jobs[0].shape.block, mats) : 0;
+    fn<<<blocks, jobs[0].shape.block, smem, s>>>(*pack);
+    return cudaGetLastError();
+}
+
+cudaError_t launchTransportQueue(int tracking, const DevJob* jobs, const unsigned long long* offsets, int nJobs,
+    unsigned long long h_end, DevCounters* ctr, LaunchShape shape, cudaStream_t s)
+{
+    if (!jobs || !offsets || nJobs < 1 || (tracking != DXMCG_TRACK_SIDDON && tracking != DXMCG_TRACK_MACRO))
+        return cudaErrorInvalidValue;
+    int refill = 0, interact = 0, wsteps = 0;
+    phaseSizes(shape, false, refill, interact, wsteps);
+    const auto fn = tracking == DXMCG_TRACK_SIDDON ? transportQueueKernel<DXMCG_TRACK_SIDDON>
+                                                   : transportQueueKernel<DXMCG_TRACK_MACRO>;
+    fn<<<shape.grid, shape.block, 0, s>>>(jobs, offsets, nJobs, h_end, ctr, refill, interact);
+    return cudaGetLastError();
+}
+
+cudaError_t loadTransport(const DevJob& J, LaunchKind kind)
+{
+    const int tracking = kernelTracking(J);
+    const bool skip = J.cbound != nullptr, bound = J.correction >= 2;
+    cudaFuncAttributes a {};
+    if (kind == LaunchKind::kPack)
+        return cudaFuncGetAttributes(&a, packFor(tracking, J.n_mats, skip, bound));
+    if (kind == LaunchKind::kQueue)
+        return tracking == DXMCG_TRACK_SIDDON ? cudaFuncGetAttributes(&a, transportQueueKernel<DXMCG_TRACK_SIDDON>)
+                                              : cudaFuncGetAttributes(&a, transportQueueKernel<DXMCG_TRACK_MACRO>);
+    return cudaFuncGetAttributes(&a, kernelFor(tracking, true, J.n_mats, skip, bound));
 }
 
 cudaError_t launchTransportUnpacked(const DevJob& job, unsigned long long h_end, DevCounters* ctr,

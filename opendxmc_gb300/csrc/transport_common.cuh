@@ -89,11 +89,48 @@ namespace {
 
 } // namespace
 
+// Jobs that share a launch: block b works on job k with first[k] <= b < first[k + 1].  They
+// are kernel parameters, so that a block reads its job from the constant bank, as it does
+// where the launch has only one; kPackJobs of them stay below the 32,764 bytes a launch
+// can pass.
+constexpr int kPackJobs = kMaxPackedJobs;
+struct JobPack {
+    struct Entry {
+        DevJob job;
+        unsigned long long h_end;
+        DevCounters* ctr;
+        int refill, interact, steps;
+    };
+    int n;
+    unsigned first[kPackJobs + 1];
+    Entry e[kPackJobs];
+};
+static_assert(sizeof(JobPack) <= 32764, "kernel parameters");
+
+namespace {
+    // the job of this block (first[0] = 0, every job has a block)
+    __device__ __forceinline__ int packJob(const JobPack& p)
+    {
+        int lo = 0, hi = p.n;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (p.first[mid] <= blockIdx.x)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        return lo;
+    }
+} // namespace
+
 using TransportFn = void (*)(const DevJob, unsigned long long, DevCounters*, int, int, int);
+using PackFn = void (*)(const JobPack);
 
 // woodcock.cu: the Woodcock kernel's instance for a voxel layout, one region or two and
-// n_mats materials; its dynamic shared memory at a block size; its default batch sizes
+// n_mats materials (for several jobs: in the packed layout); its dynamic shared memory at a
+// block size; its default batch sizes
 TransportFn woodcockKernelFor(bool packed, bool box, int n_mats, bool skip, bool bound);
+PackFn woodcockPackFor(bool box, int n_mats, bool skip, bool bound);
 size_t woodcockSharedBytes(int block, int n_mats);
 extern const int kWoodcockRefillBatch, kWoodcockInteractBatch;
 // materials whose attenuation tables a block holds in shared memory: with the photon

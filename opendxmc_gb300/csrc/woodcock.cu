@@ -210,9 +210,10 @@ namespace {
     // level-2 samplers held registers (the steps spilled) and issue slots where they are off.
     // 1e7 histories of the DX cylinder 1.26 -> 1.18 ms, 2e8 of the torso 24.9 -> 23.2, 3e8 of
     // the 512 x 512 x 400 torso 53.3 -> 51.2, 1e7 of a level-2 CBCT 3.65 -> 3.32.
+    // blocks: the blocks that work on this job.
     template <bool PACKED, bool BOX, bool TAB, bool SKIP, bool BOUND>
-    __global__ void __launch_bounds__(256, 4) woodcockKernel(const DevJob J, unsigned long long h_end,
-        DevCounters* __restrict__ ctr, int refillBatch, int interactBatch, int woodcockSteps)
+    __device__ __forceinline__ void woodcockRun(const DevJob& J, unsigned long long h_end,
+        DevCounters* __restrict__ ctr, int refillBatch, int interactBatch, int woodcockSteps, unsigned blocks)
     {
         extern __shared__ __align__(16) unsigned char sRaw[];
         const int lane = static_cast<int>(threadIdx.x & 31u);
@@ -242,7 +243,7 @@ namespace {
         bool exhausted = false;
         unsigned visits = 0, skipped = 0, outerVisits = 0, err = 0;
         // half the warps' share of the histories left
-        const float halfShare = 0.5f / static_cast<float>(gridDim.x * static_cast<unsigned>(warps));
+        const float halfShare = 0.5f / static_cast<float>(blocks * static_cast<unsigned>(warps));
 
         const auto addSum = [&](int K, float x) { // Kahan step of the lane's sum K
             const float c = sums[32 * (2 * K + 1)], s0 = sums[32 * (2 * K)];
@@ -519,6 +520,35 @@ namespace {
         }
     }
 
+    template <bool PACKED, bool BOX, bool TAB, bool SKIP, bool BOUND>
+    __global__ void __launch_bounds__(256, 4) woodcockKernel(const DevJob J, unsigned long long h_end,
+        DevCounters* __restrict__ ctr, int refillBatch, int interactBatch, int woodcockSteps)
+    {
+        woodcockRun<PACKED, BOX, TAB, SKIP, BOUND>(J, h_end, ctr, refillBatch, interactBatch, woodcockSteps,
+            gridDim.x);
+    }
+    template <bool BOX, bool TAB, bool SKIP, bool BOUND>
+    __global__ void __launch_bounds__(256, 4) woodcockPackKernel(const __grid_constant__ JobPack pack)
+    {
+        const int k = packJob(pack);
+        const JobPack::Entry& e = pack.e[k];
+        woodcockRun<true, BOX, TAB, SKIP, BOUND>(e.job, e.h_end, e.ctr, e.refill, e.interact, e.steps,
+            pack.first[k + 1] - pack.first[k]);
+    }
+
+    template <bool BOX, bool TAB, bool SKIP>
+    PackFn packByLevel(bool bound)
+    {
+        return bound ? woodcockPackKernel<BOX, TAB, SKIP, true> : woodcockPackKernel<BOX, TAB, SKIP, false>;
+    }
+    template <bool BOX>
+    PackFn packInstance(bool tab, bool skip, bool bound)
+    {
+        if (skip)
+            return tab ? packByLevel<BOX, true, true>(bound) : packByLevel<BOX, false, true>(bound);
+        return tab ? packByLevel<BOX, true, false>(bound) : packByLevel<BOX, false, false>(bound);
+    }
+
     template <bool PACKED, bool BOX, bool TAB, bool SKIP>
     TransportFn byLevel(bool bound)
     {
@@ -543,6 +573,12 @@ TransportFn woodcockKernelFor(bool packed, bool box, int n_mats, bool skip, bool
     if (packed)
         return box ? instance<true, true>(tab, skip, bound) : instance<true, false>(tab, skip, bound);
     return box ? instance<false, true>(tab, false, bound) : instance<false, false>(tab, false, bound);
+}
+
+PackFn woodcockPackFor(bool box, int n_mats, bool skip, bool bound)
+{
+    const bool tab = n_mats <= kSharedTableMaterials;
+    return box ? packInstance<true>(tab, skip, bound) : packInstance<false>(tab, skip, bound);
 }
 
 size_t woodcockSharedBytes(int block, int n_mats)

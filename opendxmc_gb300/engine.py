@@ -331,8 +331,8 @@ class GpuWorld:
 
 
 class Batch:
-    """Several (world, beam, options) jobs in one persistent launch over a shared
-    history queue, replayed as a CUDA graph by run().  The worlds must outlive it."""
+    """Several (world, beam, options) jobs as one CUDA graph replayed by run(): large jobs a
+    launch each, small ones in shared launches.  The worlds must outlive it."""
 
     def __init__(self, jobs: list[tuple[GpuWorld, dict, N.RunOptions | None]]):
         n = len(jobs)
