@@ -165,8 +165,11 @@ typedef struct {
     int32_t chunk_histories_log2; /* histories per launch (progress/cancel granularity), 0 = default */
     uint64_t hist_begin;  /* history range [begin, end) of the beam; end 0 = all */
     uint64_t hist_end;
-    int32_t interact_batch; /* parked scatterings a warp gathers before sampling them, 0 = default */
-    int32_t refill_batch;   /* free photon slots a warp gathers before starting new histories, 0 = default */
+    /* lanes whose photons wait for a scattering that a warp gathers before sampling them,
+     * and lanes free for a new history before it starts some; 0 = default.  1..32; the
+     * Woodcock kernel, with two photons a lane, gathers twice as many (32 at most) */
+    int32_t interact_batch;
+    int32_t refill_batch;
     int32_t macro_cell;     /* MACRO tracking: cell edge in voxels, 0 = default (16) */
     int32_t woodcock_steps; /* WOODCOCK tracking: steps a lane takes between regroupings, 0 = default:
                              * 1.4 / p clamped to 4..16, p = stops per step of the world's
@@ -305,7 +308,7 @@ DXMCG_API void dxmcg_batch_destroy(dxmcg_batch* b);
  * No counterpart in the reference.  Times the transport kernel on
  * sample_histories (0: 2^24) histories from the middle of the beam for each
  * block size {128, 256} x interact batch {8, 12, 16, 24} x refill batch
- * {4, 8, 16} x Woodcock steps per phase {8, 16} (Woodcock tracking only),
+ * {4, 8, 16} x Woodcock steps per phase {4, 8, 12} (Woodcock tracking only),
  * depositing into a scratch tally (the world's dose is untouched), and writes the
  * fastest block_size / interact_batch / refill_batch / woodcock_steps into *opts
  * (blocks_per_sm = 0: all resident blocks).  histories_per_second may be NULL. */

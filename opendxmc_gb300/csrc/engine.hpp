@@ -190,8 +190,10 @@ enum ErrorFlag : unsigned {
 struct LaunchShape {
     int grid = 0;
     int block = 256;
-    int refill_batch = 0;   // dead lanes a warp gathers before starting new histories (0: default)
-    int interact_batch = 0; // parked lanes a warp gathers before running scatterings (0: default)
+    // lanes free for new histories, or parked at a scattering, that a warp gathers before it
+    // runs them (0: default; two photon slots a lane in the Woodcock kernel, see phaseSizes)
+    int refill_batch = 0;
+    int interact_batch = 0;
     int woodcock_steps = 0; // Woodcock steps per lane and step phase (0: default)
 };
 

@@ -500,11 +500,18 @@ namespace {
 
     bool isWoodcock(int tracking) { return tracking == DXMCG_TRACK_WOODCOCK || tracking == kTrackWoodcockBox; }
 
-    // the batch sizes and steps of a shape, defaults filled in
+    // The batch sizes and steps of a shape, defaults filled in.  Batches are counted in lanes:
+    // of the Woodcock kernel's two photon slots a lane, twice as many (32 at most, a phase's
+    // lanes).
     void phaseSizes(const LaunchShape& shape, bool woodcock, int& refill, int& interact, int& steps)
     {
-        refill = shape.refill_batch > 0 ? shape.refill_batch : (woodcock ? kWoodcockRefillBatch : 8);
-        interact = shape.interact_batch > 0 ? shape.interact_batch : (woodcock ? kWoodcockInteractBatch : 8);
+        const auto size = [&](int batch, int woodcockDefault) {
+            if (batch <= 0)
+                return woodcock ? woodcockDefault : 8;
+            return woodcock ? std::min(32, 2 * batch) : batch;
+        };
+        refill = size(shape.refill_batch, kWoodcockRefillBatch);
+        interact = size(shape.interact_batch, kWoodcockInteractBatch);
         steps = shape.woodcock_steps > 0 ? shape.woodcock_steps : 8;
     }
 

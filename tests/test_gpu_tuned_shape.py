@@ -1,0 +1,31 @@
+"""Batch sizes that a caller sets, or the autotuner finds among the documented ones, run as
+fast as the defaults on the Woodcock kernel."""
+import pytest
+
+from opendxmc_gb300 import phantoms as P
+
+pytestmark = pytest.mark.gpu
+
+
+def kernel_ms(w, beam, options):
+    times = []
+    for _ in range(9):
+        w.clear()
+        times.append(w.run(beam, options)["kernel_ms"])
+    return min(times)
+
+
+def test_tuned_and_given_shapes_against_the_default(gpu):
+    """Measured: the tuned shape 1.003 times the default's time (1.05 when batches were counted
+    in photon slots), batches of 8 lanes 1.10 times (1.43)."""
+    ph = P.torso_phantom()
+    w = gpu.GpuWorld(ph.dims, ph.spacing, ph.materials)
+    w.set_data(ph.density, ph.material)
+    w.build()
+    beam = P.ct_spiral_params(particles=1)
+    beam["particles_per_exposure"] = 20_000_000 // len(gpu.beam_exposures(beam))
+    w.run(beam, gpu.run_options(seed=1))
+    default = kernel_ms(w, beam, gpu.run_options(seed=3))
+    tuned, _ = w.autotune(beam, gpu.run_options(seed=3))
+    assert kernel_ms(w, beam, tuned) < 1.03 * default
+    assert kernel_ms(w, beam, gpu.run_options(seed=3, interact_batch=8, refill_batch=8)) < 1.25 * default
