@@ -290,12 +290,13 @@ DXMCG_API int dxmcg_transport_run(dxmcg_world* w, const dxmcg_beam* beam, const 
  * up to the summation order, as dxmcg_transport_run(worlds[j], beams + j,
  * opts + j, ...).  A world may appear in several jobs (their doses add).
  * Requirements: every world built and on one device, one tracking mode for all
- * jobs (launch shape from opts[0]), hist_begin = hist_end = 0, one macro_cell
- * per world.  Exposures, spectra and calibrations are fixed at create time; the
+ * jobs, hist_begin = hist_end = 0, one macro_cell per world.  The launch shape is
+ * opts[0]'s for all jobs, or each job's own where they average 2^21 histories or more.  Exposures, spectra and calibrations are fixed at create time; the
  * worlds must outlive the batch and must not run other transports meanwhile.
  * The first dxmcg_batch_run captures a CUDA graph (counter resets + the launches)
  * that every later run replays; each run adds N_j histories to world j's dose
- * normalisation.  stats are summed over all jobs (calibration: job 0's). */
+ * normalisation.  stats are summed over all jobs (calibration and woodcock_steps:
+ * job 0's). */
 typedef struct dxmcg_batch dxmcg_batch;
 DXMCG_API int dxmcg_batch_create(int n_jobs, dxmcg_world* const* worlds, const dxmcg_beam* beams,
     const dxmcg_run_options* opts, dxmcg_batch** out);

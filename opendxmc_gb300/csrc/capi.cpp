@@ -1370,7 +1370,8 @@ DXMCG_API int dxmcg_batch_create(int n_jobs, dxmcg_world* const* worlds, const d
     }
     std::map<std::pair<int, int>, std::vector<int>> open; // by kernel instance and block size
     for (int j = 0; j < n_jobs; ++j) {
-        LaunchShape sh = chooseShape(worlds[j], opts[j], kernelTracking(J[j]));
+        // jobs that share launches take their shape from the first job's options
+        LaunchShape sh = chooseShape(worlds[j], opts[large ? j : 0], kernelTracking(J[j]));
         if (b->queue) {
             sh = first;
         } else if (!large) {

@@ -29,3 +29,20 @@ def test_tuned_and_given_shapes_against_the_default(gpu):
     tuned, _ = w.autotune(beam, gpu.run_options(seed=3))
     assert kernel_ms(w, beam, tuned) < 1.03 * default
     assert kernel_ms(w, beam, gpu.run_options(seed=3, interact_batch=8, refill_batch=8)) < 1.25 * default
+
+
+def test_small_batches_take_the_first_jobs_shape(gpu):
+    """Shapes in the other jobs' options, here ones that take 4.8 times the time, are not used
+    where jobs share launches."""
+    ph = P.ellipsoid_phantom((64, 64, 64), (0.3, 0.3, 0.3), seed=3)
+    w = gpu.GpuWorld(ph.dims, ph.spacing, ph.materials)
+    w.set_data(ph.density, ph.material)
+    w.build()
+    beam = P.dx_beam_params(particles=1_000_000, exposures=1)
+    poor = dict(interact_batch=1, refill_batch=1, woodcock_steps=1, block_size=32)
+    ms = []
+    for rest in ({}, poor):
+        batch = gpu.Batch([(w, beam, gpu.run_options(seed=j, **(rest if j else {}))) for j in range(8)])
+        ms.append(min(batch.run()["kernel_ms"] for _ in range(9)))
+        batch.close()
+    assert ms[1] < 1.1 * ms[0], ms
