@@ -1020,8 +1020,10 @@ DXMCG_API int dxmcg_world_build(dxmcg_world* w)
     if (!w->doseFactors.p && toDose > 1e-200 && toDose < 1e200) {
         DXMCG_CUDA(w->doseFactors.alloc(kDoseFactors));
         e = launchDoseFactors(toDose, w->doseFactors.p, w->stream);
-        if (e != cudaSuccess)
+        if (e != cudaSuccess) {
+            w->doseFactors.reset(); // never kept unfilled: the next build makes it anew
             return cudaFail(e, "dose-factor kernel");
+        }
     }
     // gather-skip bounds of the Woodcock step
     {
