@@ -92,10 +92,13 @@ namespace dev {
         return fmaf(f, ab.y - ab.x, ab.x);
     }
 
-    // Correctly rounded 1 / x and sqrt(x) for 2^-112 <= x < 2^107 (and sqrt(0) = 0): the
-    // hardware's approximation and one Newton step in fused arithmetic (Markstein, IBM J.
-    // Res. Dev. 34, 111, 1990).  Without the library forms' range tests and slow paths; the
-    // same bits as those for every float of that range.  In the interactions and majorants: 1e7
+    // Correctly rounded 1 / x for 2^-112 <= x < 2^107 and sqrt(x) for 0 and 2^-102 <= x <
+    // 2^107: the hardware's approximation and one Newton step in fused arithmetic (Markstein,
+    // IBM J. Res. Dev. 34, 111, 1990).  Below 2^-102 the root's residual is no multiple of the
+    // least subnormal, and for 1 / x the theorem leaves out the significand of all ones; every
+    // float of these ranges is checked against __frcp_rn and __fsqrt_rn
+    // (tests/cpp/arithmetic.cu).  Majorants are 1e-30 and more, the roots' arguments 0 or
+    // 2^-72 and more (of 1 - s^2 - t^2 with floats s, t).  In place of those functions: 1e7
     // histories of the DX cylinder 1.18 -> 1.15 ms, 2e8 of the torso 23.2 -> 22.5 ms.
     __device__ __forceinline__ float reciprocal(float x)
     {
@@ -110,6 +113,24 @@ namespace dev {
         const float g = __fmul_rn(x, y);
         const float s = __fmaf_rn(__fmaf_rn(-g, g, x), __fmul_rn(0.5f, y), g);
         return x > 0.0f ? s : 0.0f;
+    }
+    // 1 / sqrt(x) of a squared length near 1, by the hardware's approximation; rsqrtf's bits
+    // there (checked between 1/4 and 4, as above).
+    __device__ __forceinline__ float unitRsqrt(float x)
+    {
+        float y;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    }
+    // -ln u = -ln 2 log2 u of a uniform (toUniform), by the hardware's log2: |error| <=
+    // 2^-21.4 near u = 1.  __logf's bits for each of the 2^23 uniforms (checked, as above).
+    // 1e7 histories of the DX cylinder 1518 -> 1502 us in its place, 2e8 of the torso 27.10
+    // -> 26.88 ms.
+    __device__ __forceinline__ float negLog(float u)
+    {
+        float l;
+        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(u));
+        return __fmul_rn(l, -0.693147180559945309f);
     }
 
     // ---------------------------------------------------------------- samplers
@@ -351,8 +372,7 @@ namespace dev {
             ny = sint * (dy * dz * cp + dx * sp) * it + dy * cost;
             nz = -sint * cp * tmp + dz * cost;
         }
-        float inv; // of about 1, not subnormal
-        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(nx * nx + ny * ny + nz * nz));
+        const float inv = unitRsqrt(nx * nx + ny * ny + nz * nz);
         dx = nx * inv;
         dy = ny * inv;
         dz = nz * inv;

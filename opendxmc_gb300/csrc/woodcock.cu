@@ -51,14 +51,11 @@ namespace {
             & (static_cast<unsigned>(iz) < static_cast<unsigned>(J.nz));
     }
 
-    // Free path to the next tentative collision.  Hardware log2: |error| <= 2^-21.4 near
-    // u = 1, where the step is < 1e-6 mean free paths.  No uniform is subnormal, so the form
-    // that need not scale those gives what __logf does, in fewer instructions.
+    // Free path to the next tentative collision (an error of negLog near u = 1 is one of less
+    // than 1e-6 mean free paths).
     __device__ __forceinline__ float freePath(Rng& rng, float invMmax)
     {
-        float l;
-        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(rng.u()));
-        return fmaxf(__fmul_rn(l, -0.693147182464599609375f), 0.0f) * invMmax; // ln 2
+        return fmaxf(negLog(rng.u()), 0.0f) * invMmax;
     }
 
     __device__ __forceinline__ void fly(Photon& ph, float s)
