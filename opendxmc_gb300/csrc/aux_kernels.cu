@@ -303,7 +303,7 @@ namespace {
         int ie;
         float fe;
         gridPos(E[i], ie, fe);
-        eo[i] = sampleCompton(E[i], M, ctab, ie, fe, correction, r, cost, err);
+        eo[i] = sampleCompton<true>(E[i], M, ctab, ie, fe, correction, r, cost, err);
         co[i] = cost;
         used[i] = r.used;
     }

@@ -294,7 +294,7 @@ namespace {
                 // the samplers diverge; the direction update they share runs once
                 float cost = 1.0f, Ep = ph.E;
                 if (compton)
-                    Ep = sampleCompton(ph.E, J.mats + pm, J.ctab + pm * (kTableNE * kCTabK), ec.ie, ec.fe,
+                    Ep = sampleCompton<false>(ph.E, J.mats + pm, J.ctab + pm * (kTableNE * kCTabK), ec.ie, ec.fe,
                         J.correction, rng, cost, err);
                 else if (rayleigh)
                     cost = sampleRayleigh(J.rtab + pm * (kTableNE * kCTabK), ec.ie, ec.fe, rng);

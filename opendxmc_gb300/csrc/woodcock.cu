@@ -363,7 +363,7 @@ namespace {
                         if (!photo) {
                             float cost;
                             if (BOUND && compton) {
-                                Ep = sampleCompton(ph.E, J.mats + pm, J.ctab + pm * (kTableNE * kCTabK), ec.ie, ec.fe,
+                                Ep = sampleCompton<true>(ph.E, J.mats + pm, J.ctab + pm * (kTableNE * kCTabK), ec.ie, ec.fe,
                                     2, rng, cost, err);
                             } else {
                                 // one path for both: the angle from the kind's quantile table

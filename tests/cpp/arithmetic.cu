@@ -42,7 +42,7 @@ __global__ void compareForms(uint32_t first, unsigned long long n, unsigned long
 }
 
 // dopplerEnergy as a plain loop: the shell by two passes over the shells, every draw tried
-template <class U>
+template <bool FUSED, class U>
 __device__ bool plainDoppler(float E, float A, float omu, const DevMaterial* M, U& r, float& Ep)
 {
     float tot = 0.0f;
@@ -70,8 +70,10 @@ __device__ bool plainDoppler(float E, float A, float omu, const DevMaterial* M, 
             continue;
         const float rho = M->shellMomentum[sh] * a * sqrtf((powf(w, -0.4f) - 1.0f) / w);
         const float rho2 = __fmul_rn(rho, rho);
-        const float den = __fmaf_rn(A, A, -rho2);
-        const float disc = __fmaf_rn(am, am, __fmul_rn(sin2, __fsub_rn(1.0f, rho2)));
+        const float den = FUSED ? __fmaf_rn(A, A, -rho2) : __fsub_rn(__fmul_rn(A, A), rho2);
+        const float rest = __fsub_rn(1.0f, rho2);
+        const float disc
+            = FUSED ? __fmaf_rn(am, am, __fmul_rn(sin2, rest)) : __fmaf_rn(sin2, rest, __fmul_rn(am, am));
         if (!(den > 0.0f) || !(disc >= 0.0f))
             continue;
         const float e1 = E * (__fmaf_rn(rho, sqrtf(disc), __fmaf_rn(-rho2, c, A)) / den);
@@ -84,6 +86,7 @@ __device__ bool plainDoppler(float E, float A, float omu, const DevMaterial* M, 
 }
 
 // per draw: energy 1 to 150 keV and an angle; the same uniforms to both forms
+template <bool FUSED>
 __global__ void compareSamplers(const DevMaterial* mats, int nMats, int n, unsigned long long* badDoppler,
     unsigned long long* badFluorescence, unsigned long long* taken)
 {
@@ -95,7 +98,7 @@ __global__ void compareSamplers(const DevMaterial* mats, int nMats, int n, unsig
         Rng a = seed, b = seed;
         float ea = 0.0f, eb = 0.0f;
         const float A = comptonRatio(E, omu);
-        const bool ta = dopplerEnergy(E, A, omu, M, a, ea), tb = plainDoppler(E, A, omu, M, b, eb);
+        const bool ta = dopplerEnergy<FUSED>(E, A, omu, M, a, ea), tb = plainDoppler<FUSED>(E, A, omu, M, b, eb);
         // taken or not, the energy, and the uniforms used (the generators' states)
         if (ta != tb || __float_as_uint(ea) != __float_as_uint(eb) || a.s0 != b.s0 || a.s3 != b.s3)
             atomicAdd(badDoppler, 1ull);
@@ -200,9 +203,13 @@ int main()
     if (cudaMalloc(&m, mats.size() * sizeof *m) != cudaSuccess
         || cudaMemcpy(m, mats.data(), mats.size() * sizeof *m, cudaMemcpyHostToDevice) != cudaSuccess)
         return 2;
-    compareSamplers<<<2048, 128>>>(m, kMats, kDraws, c, c + 1, c + 2);
-    std::printf("dopplerEnergy %llu of %d\n", take(c), kDraws);
-    std::printf("samplePhotoFluorescence %llu of %d\n", take(c + 1), kDraws);
-    std::printf("taken %llu of %d\n", take(c + 2), kDraws);
+    const auto samplers = [&](auto kernel, const char* which) {
+        kernel<<<2048, 128>>>(m, kMats, kDraws, c, c + 1, c + 2);
+        std::printf("dopplerEnergy%s %llu of %d\n", which, take(c), kDraws);
+        std::printf("samplePhotoFluorescence%s %llu of %d\n", which, take(c + 1), kDraws);
+        std::printf("taken%s %llu of %d\n", which, take(c + 2), kDraws);
+    };
+    samplers(compareSamplers<true>, "Fused");
+    samplers(compareSamplers<false>, "Plain");
     return cudaDeviceSynchronize() == cudaSuccess ? 0 : 2;
 }

@@ -25,11 +25,12 @@ def checks(gpu, tmp_path_factory):
 
 @pytest.mark.parametrize("name,total", [
     ("reciprocal", 219 << 23), ("squareRoot", 209 << 23), ("squareRootOfZero", 1), ("unitRsqrt", 4 << 23),
-    ("negLog", 1 << 23), ("dopplerEnergy", 1 << 23), ("samplePhotoFluorescence", 1 << 23)])
+    ("negLog", 1 << 23), ("dopplerEnergyFused", 1 << 23), ("dopplerEnergyPlain", 1 << 23),
+    ("samplePhotoFluorescenceFused", 1 << 23), ("samplePhotoFluorescencePlain", 1 << 23)])
 def test_same_bits(checks, name, total):
     assert checks[name] == (0, total)
 
 
 def test_bound_electron_draws_are_taken_and_refused(checks):
-    taken, total = checks["taken"]
+    taken, total = checks["takenFused"]
     assert 0.2 * total < taken < 0.98 * total
