@@ -31,6 +31,7 @@ def test_every_voxel_of_a_large_world_is_written(gpu):
     for shift in (0, 1):  # on a 16-byte boundary: two voxels a thread; off it: one
         for x in out:
             x.fill_(-7)
+        torch.cuda.synchronize()  # the library reads out on a stream of the world's own
         at = [x.data_ptr() + 8 * shift for x in out]
         N.check(N.lib().dxmcg_world_read_dose(w._h, C.cast(at[0], C.POINTER(C.c_double)),
                                               C.cast(at[1], C.POINTER(C.c_double)),
