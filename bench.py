@@ -98,7 +98,7 @@ def parse():
                    default="torso",
                    help="torso: the spiral-CT torso job (256x256x200); torso512: the 512x512x400 spiral-CT torso; "
                         "c1: the DX water cylinder (1e7 histories per step unless --histories); "
-                        "batch: 64 uneven DX/CBCT jobs in one persistent launch; "
+                        "batch: 64 uneven DX/CBCT jobs in one captured graph; "
                         "pipelines: segmentation and organ dose table passes; denoiser: training step and "
                         "inference throughput; world-denoise: the world-path denoiser call on the 512x512x400 "
                         "torso after a 3e7-history run; c4-training: the denoiser trained on 200 seeded 128^3 "
@@ -583,7 +583,7 @@ def run_batch(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "peak_source": peak_kind, "traffic": None, "kernel_ms_per_launch": kernel_ms / args.steps},
         # jobs averaging 2^21 histories or more run one single-job launch each in the
-        # graph; smaller ones one shared-queue launch (the library's rule)
+        # graph; smaller ones share launches, one at least (the library's rule)
         "setup_s": t_setup, "gpu_launches": args.steps * (len(specs) if total >= (1 << 21) * len(specs) else 1),
         "clocks": clk,
     }

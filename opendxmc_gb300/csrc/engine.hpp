@@ -231,13 +231,13 @@ cudaError_t launchTransport(const DevJob& job, unsigned long long h_end, DevCoun
 // per-macro-cell majorant scale: max over the cell's voxels of rho * ratio[m]
 cudaError_t launchMacroScale(const uint32_t* vox, int nx, int ny, int nz, int mb, int mcx, int mcy,
     const float* ratio, unsigned* scaleBits, cudaStream_t s);
-// gather-skip bounds: per cell of kCellEdge^3 voxels (cells x fastest, ncx x ncy x ncz)
-// max over its voxels of rho * ratio[m] times (1 + 2^-12), +inf if one is transparent
 // bounding box of the voxels whose material is neither 0 nor transparent:
 // box = {min x, min y, min z, max x, max y, max z}, initialised by the caller to
 // {INT_MAX x3, -1 x3} (max x = -1 after the launch: no such voxel)
 cudaError_t launchMaterialBox(const uint32_t* vox, int nx, int ny, int nz, int* box, cudaStream_t s);
 cudaError_t launchMaterialBox(const uint8_t* mat, int nx, int ny, int nz, int* box, cudaStream_t s);
+// gather-skip bounds: per cell of kCellEdge^3 voxels (cells x fastest, ncx x ncy x ncz)
+// max over its voxels of rho * ratio[m] times (1 + 2^-12), +inf if one is transparent
 cudaError_t launchCellBound(const uint32_t* vox, int nx, int ny, int nz, int ncx, int ncy, int ncz, const float* ratio,
     float* bound, cudaStream_t s);
 cudaError_t launchDoseFactors(double toDose, double* factors, cudaStream_t s);
