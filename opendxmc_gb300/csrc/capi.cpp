@@ -376,12 +376,14 @@ int deviceErrors(const DevCounters& c, const char* what)
 // that average kLargeJob histories or more are a launch each and fill the GPU one after
 // another, on kLargeStreams streams so that one job's blocks take the SMs another job's tail
 // frees; one world at a time keeps its voxels and tally in L2.  Smaller jobs would mostly be
-// tails: they share launches (launchTransportPack), each with kSmallShare times its share of
-// the resident blocks, so that blocks of the jobs still to come replace those of jobs that
-// are done.  With a launch a job, on 32 streams, a batch of many jobs was as long as the
-// jobs' longest histories one after another: 512 Woodcock jobs of 1000 histories on 64^3
-// voxels 1.09 ms, this way 0.29; 1024 of 1e4 4.6 and 1.8 ms; eight of 1e5 to 2e6 histories
-// the same.  (Once the share, 64 jobs of 1e5 take 1.51 ms in place of 1.08.)
+// tails: they share launches (launchTransportPack) of two waves of blocks in all, more where a
+// block would get more than kSmallBlock histories, so that blocks of the jobs still to come
+// replace those of jobs that are done.  With a launch a job, on 32 streams, a batch of many
+// jobs was as long as the jobs' longest histories one after another: 512 Woodcock jobs of
+// 1000 histories on 64^3 voxels 1.09 ms, this way 0.29; 1024 of 1e4 4.6 and 1.8 ms; eight of
+// 1e5 to 2e6 histories the same.  (One wave: 64 jobs of 1e5 take 1.51 ms in place of 1.08.
+// Two at any size: 32 jobs of 1.5e6 on 160^3 voxels 12.2 ms in place of 11.0, 100 uneven ones
+// 15.1 in place of 12.1; blocks of 4096 histories 11.4 and 12.4, of 2048 12.3 and 13.2.)
 // Where Siddon and macro tracking, whose lanes own a photon each, have more than
 // kQueueHistories histories a resident lane, their lanes take the histories of all jobs from
 // one queue (launchTransportQueue): shared launches hold a block until its job's last
@@ -390,7 +392,7 @@ int deviceErrors(const DevCounters& c, const char* what)
 // 1.00 and 0.77, 5.8 and 4.9.
 constexpr uint64_t kLargeJob = 1ull << 21;
 constexpr int kLargeStreams = 4, kSmallStreams = 32;
-constexpr double kSmallShare = 2.0, kQueueHistories = 5.0;
+constexpr double kSmallWaves = 2.0, kSmallBlock = 8192.0, kQueueHistories = 5.0;
 
 struct dxmcg_batch {
     int device = 0;
@@ -1377,10 +1379,11 @@ DXMCG_API int dxmcg_batch_create(int n_jobs, dxmcg_world* const* worlds, const d
         if (b->queue) {
             sh = first;
         } else if (!large) {
-            // 128 histories a block at least
-            const double share = kSmallShare * static_cast<double>(b->nHist[j])
-                / static_cast<double>(std::max<uint64_t>(b->total, 1));
-            const double blocks = std::min(std::ceil(sh.grid * share), std::ceil(b->nHist[j] / 128.0));
+            // to a block of the job the fair share of a resident block over the waves, 128
+            // histories at least
+            const double fair = static_cast<double>(b->total) / sh.grid;
+            const double waves = std::max(kSmallWaves, std::round(fair / kSmallBlock));
+            const double blocks = std::ceil(b->nHist[j] / std::max(128.0, fair / waves));
             sh.grid = static_cast<int>(std::max(1.0, std::min<double>(sh.grid, blocks)));
             std::vector<int>& o = open[{ transportInstance(J[j]), sh.block }];
             o.push_back(j);
