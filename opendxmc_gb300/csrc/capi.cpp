@@ -1368,9 +1368,11 @@ DXMCG_API int dxmcg_batch_create(int n_jobs, dxmcg_world* const* worlds, const d
             off[j + 1] = off[j] + b->nHist[j];
         DXMCG_CUDA(b->queueJobs.alloc(n_jobs));
         DXMCG_CUDA(b->queueOffsets.alloc(off.size()));
-        DXMCG_CUDA(cudaMemcpy(b->queueJobs.p, J.data(), n_jobs * sizeof(DevJob), cudaMemcpyHostToDevice));
-        DXMCG_CUDA(cudaMemcpy(b->queueOffsets.p, off.data(), off.size() * sizeof(unsigned long long),
-            cudaMemcpyHostToDevice));
+        DXMCG_CUDA(cudaMemcpyAsync(b->queueJobs.p, J.data(), n_jobs * sizeof(DevJob), cudaMemcpyHostToDevice,
+            b->stream));
+        DXMCG_CUDA(cudaMemcpyAsync(b->queueOffsets.p, off.data(), off.size() * sizeof(unsigned long long),
+            cudaMemcpyHostToDevice, b->stream));
+        DXMCG_CUDA(cudaStreamSynchronize(b->stream));
     }
     std::map<std::pair<int, int>, std::vector<int>> open; // by kernel instance and block size
     for (int j = 0; j < n_jobs; ++j) {
@@ -1462,10 +1464,11 @@ DXMCG_API int dxmcg_batch_run(dxmcg_batch* b, dxmcg_stats* stats)
                 e = launchTransport(b->hostJobs[j], b->nHist[j], b->jobCounters.p + j, b->jobShapes[j], t);
                 continue;
             }
-            std::vector<PackedJob> pack;
+            PackedJob pack[kMaxPackedJobs];
+            int n = 0;
             for (int j : jobs)
-                pack.push_back({ &b->hostJobs[j], b->nHist[j], b->jobCounters.p + j, b->jobShapes[j] });
-            e = launchTransportPack(pack.data(), static_cast<int>(pack.size()), t);
+                pack[n++] = { &b->hostJobs[j], b->nHist[j], b->jobCounters.p + j, b->jobShapes[j] };
+            e = launchTransportPack(pack, n, t);
         }
         for (int k = 0; k < streams && e == cudaSuccess; ++k) {
             e = cudaEventRecord(b->join[k], b->side[k]);

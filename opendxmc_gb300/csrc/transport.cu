@@ -28,7 +28,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <memory>
 
 #include "transport_common.cuh"
 
@@ -569,8 +568,8 @@ cudaError_t launchTransportPack(const PackedJob* jobs, int n, cudaStream_t s)
     const PackFn fn = packFor(tracking, J.n_mats, J.cbound != nullptr, J.correction >= 2);
     if (!fn)
         return cudaErrorInvalidValue;
-    const auto pack = std::make_unique<JobPack>();
-    pack->n = n;
+    JobPack pack;
+    pack.n = n;
     int mats = 0;
     unsigned blocks = 0;
     for (int k = 0; k < n; ++k) {
@@ -578,18 +577,18 @@ cudaError_t launchTransportPack(const PackedJob* jobs, int n, cudaStream_t s)
         if (transportInstance(*p.job) != transportInstance(J) || p.shape.block != jobs[0].shape.block
             || p.shape.grid < 1)
             return cudaErrorInvalidValue;
-        JobPack::Entry& e = pack->e[k];
+        JobPack::Entry& e = pack.e[k];
         e.job = *p.job;
         e.h_end = p.h_end;
         e.ctr = p.ctr;
         phaseSizes(p.shape, woodcock, e.refill, e.interact, e.steps);
-        pack->first[k] = blocks;
+        pack.first[k] = blocks;
         blocks += static_cast<unsigned>(p.shape.grid);
         mats = std::max(mats, p.job->n_mats);
     }
-    pack->first[n] = blocks;
+    pack.first[n] = blocks;
     const size_t smem = woodcock ? woodcockSharedBytes(jobs[0].shape.block, mats) : 0;
-    fn<<<blocks, jobs[0].shape.block, smem, s>>>(*pack);
+    fn<<<blocks, jobs[0].shape.block, smem, s>>>(pack);
     return cudaGetLastError();
 }
 
